@@ -38,7 +38,7 @@ def build(ref: bool = False) -> None:
     """Compile liboracle.so (and, if ``ref`` and the reference tree exists, oracle/_ref)."""
     subprocess.run(["make", "-s", "-C", _HERE, "liboracle.so"], check=True)
     root = reference_root()
-    if ref and os.path.isdir(root):
+    if ref and os.path.isdir(os.path.join(root, "optix_raycasting")):   # an empty mount has nothing to compile
         subprocess.run(["make", "-s", "-C", _HERE, "ref", f"REF={root}"], check=True)
 
 
