@@ -340,17 +340,6 @@ __device__ __forceinline__ void slab_range(const RayState& r, int K, int nv, flo
 __device__ __forceinline__ int nwords(int count) { return (count + 31) >> 5; }
 
 // Union occupancy of the chunk's slabs (256 bits): bit k set when some lane has a hit in slab k.
-__device__ __forceinline__ void occ_set(unsigned long long* occ, int lo, int hi) {
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-        int a0 = max(lo, 64 * w), b0 = min(hi, 64 * w + 63);
-        if (a0 <= b0) {
-            int n = b0 - a0 + 1;
-            unsigned long long m = (n == 64) ? ~0ull : (((1ull << n) - 1ull) << (a0 - 64 * w));
-            occ[w] |= m;
-        }
-    }
-}
 __device__ __forceinline__ bool occ_test(const unsigned long long* occ, int k) {
     return (occ[k >> 6] >> (k & 63)) & 1ull;
 }
@@ -362,14 +351,6 @@ __device__ __forceinline__ int occ_next(const unsigned long long* occ, int k, in
         if (m) return min(K, 64 * w + __ffsll((long long)m) - 1);
     }
     return K;
-}
-
-template <bool FAST, int CAP>
-__device__ __forceinline__ void clear_occ(WarpSmem<FAST, CAP>& sm, int lane) {
-    if (lane == 0) {
-#pragma unroll
-        for (int w = 0; w < 4; ++w) sm.occ[w] = 0ull;
-    }
 }
 
 // Adds the tile's counters to the warp's totals and resets them.
@@ -433,53 +414,106 @@ __device__ __forceinline__ bool leaf_entry(WarpSmem<FAST, CAP>& sm, const Render
     if (lane == 0) {
         sm.ids[count] = leaf;
         sm.urng[count] = (unsigned)ulo | ((unsigned)uhi << 16);
-        occ_set(sm.occ, ulo, uhi);
     }
     ++count;
     return true;
 }
 
-// Publishes the chunk list: occupancy bits and the entry masks per block of MB slabs.
+// Bits lo..hi of 64-slab word w (none where the range does not meet it).
+__device__ __forceinline__ unsigned long long range_bits(int lo, int hi, int w) {
+    const int a0 = max(lo - 64 * w, 0), b0 = min(hi - 64 * w, 63);
+    return a0 <= b0 ? ((~0ull) >> (63 - (b0 - a0))) << a0 : 0ull;
+}
+
+// Publishes the chunk list: occupancy bits and the entry masks per block of MB slabs.  One lane per
+// entry: a word of 32 entries costs a ballot per block and an OR-reduction per 32 slabs, against a
+// serial walk of all entries per block and, for the occupancy, by lane 0 as entries were appended.
 template <bool FAST, int CAP, bool DIAG>
 __device__ __forceinline__ void finish_list(WarpSmem<FAST, CAP>& sm, int count, int K, int lane, WarpStats& ws) {
     __syncwarp();
     if (DIAG) ws.entries += count;
-    // lane l fills blocks l, l+32
     constexpr int MB = WarpSmem<FAST, CAP>::MB;
-    const int nblk = (K + MB - 1) / MB;
+    const int nblk = (K + MB - 1) / MB, nocc = (K + 63) >> 6;
     const int nw = nwords(count);
-    for (int bk = lane; bk < nblk; bk += 32) {
-        const int k0 = bk * MB, k1 = k0 + MB - 1;
+    if (lane < 4) sm.occ[lane] = 0ull;
+    __syncwarp();
 #pragma unroll 1
-        for (int w = 0; w < nw; ++w) {
-            unsigned mw = 0u;
-            const int e0 = 32 * w, e1 = min(count, e0 + 32);
+    for (int w = 0; w < nw; ++w) {
+        const int e = 32 * w + lane;
+        const unsigned u = e < count ? sm.urng[e] : 0xffffu;   // no entry: lo 65535 > hi 0
+        const int lo = (int)(u & 0xffffu), hi = (int)(u >> 16);
+        // entry e meets block bk iff b0 <= bk <= b1
+        const int b0 = lo / MB, b1 = hi / MB;
 #pragma unroll 1
-            for (int e = e0; e < e1; ++e) {
-                unsigned u = sm.urng[e];
-                if (k1 >= (int)(u & 0xffff) && k0 <= (int)(u >> 16)) mw |= 1u << (e - e0);
+        for (int bk = 0; bk < nblk; bk += 32) {
+            const int m = min(32, nblk - bk);
+            unsigned mine = 0u;
+#pragma unroll 4
+            for (int j = 0; j < m; ++j) {
+                const unsigned mw = __ballot_sync(kFull, b0 <= bk + j && bk + j <= b1);
+                if (lane == j) mine = mw;
             }
-            sm.smask[bk][w] = mw;
+            if (lane < m) sm.smask[bk + lane][w] = mine;
+        }
+#pragma unroll 1
+        for (int o = 0; o < nocc; ++o) {
+            const unsigned long long v = range_bits(lo, hi, o);
+            const unsigned vl = __reduce_or_sync(kFull, (unsigned)v), vh = __reduce_or_sync(kFull, (unsigned)(v >> 32));
+            if (lane == 0) sm.occ[o] |= ((unsigned long long)vh << 32) | vl;
         }
     }
     __syncwarp();
 }
 
+// Slabs of the chunk a lane marches (nv: slab k is marched iff tb_k < texit, tb_k by repeated
+// addition) and the end of its searched segment.
+__device__ __forceinline__ void chunk_extent(const RayState& r, bool on, int K, float t_end, int& nv, float& seg_hi) {
+    nv = 0;
+    seg_hi = r.tb;
+    if (!on) return;
+    if (K <= kExactChunk) {
+        float t = r.tb;
+        for (int kk = 0; kk < K; ++kk) {
+            if (t < r.texit) { nv = kk + 1; t = t + kSlab; } else break;
+        }
+        seg_hi = fminf(t_end, t);
+    } else {
+        nv = K;
+        seg_hi = fminf(t_end, r.tb + (float)(K + 1) * kSlab);
+    }
+}
+
 // Warp-cooperative traversal for the chunk [tb, seg_hi] of every active lane (the packet set by
-// set_packet).  At a wide node lane k tests child slot k against the packet; the first hit child is
-// visited next and the others wait on the stack, the lowest index on top, so leaves are reached in
-// increasing index (the multi-pass cursor relies on it).  Appends hit leaves with index > cursor to
-// the warp list; returns the entry count.  `ovf` is set when the list filled up before the
-// traversal finished.
+// set_packet).  At a wide node lane k tests child slot k against the packet.  Hit leaves go to a
+// candidate buffer (the leading ones of a node all at once); the first hit child that is a node is
+// visited next and the children after it wait on the stack, the lowest index on top, so leaves are
+// reached in increasing index (the multi-pass cursor relies on it).  Candidates are taken 32 at a
+// time: the leaves with index > cursor get the exact test per ray, and those that any ray hits
+// are appended to the warp list, whose entry count is returned.
+//
+// A list that fills up shortens the chunk (K, nv and seg_hi) in place: K is halved until an entry drops
+// out (one starting at slab K or later holds no slab of the shorter chunk), the entries that stay get
+// the exact test again for the shorter chunk, and the traversal goes on from its stack with the
+// smaller packet.  The list is the one that a traversal started with the shorter chunk builds, and
+// nothing is visited twice.  (Starting over, a tile that came on dense space with a long chunk filled
+// and dropped the list once per halving: 1M Gaussians x 16 views, 13M rays, appended 300M entries for
+// 122M used.  With this, and with the list published a ballot at a time, that forward went from
+// 272.6 to 234.4 ms and its backward, which publishes replayed lists, from 273.6 to 260.9 ms.)
+// `ovf` is set when the list filled up for a single slab before the traversal finished.
 template <bool FAST, int CAP, bool DIAG>
-__device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float seg_hi,
-                        int K, int nv, int cursor, bool& ovf, int lane, WarpStats& ws, bool infer) {
+__device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float t_end,
+                        float& seg_hi, int& K, int& nv, int cursor, bool& ovf, int lane, WarpStats& ws, bool infer) {
     int count = 0;
     ++ws.traversals;
     ovf = false;
-    clear_occ(sm, lane);
+    // candidates: the entry masks' space, which finish_list writes only afterwards
+    int* const cand = reinterpret_cast<int*>(&sm.smask[0][0]);
+    static_assert(sizeof(sm.smask) >= 96 * sizeof(int), "up to 63 candidates, read 32 at a time from any of the first 32");
+    int np = 0;              // candidates waiting
+    int rt = 0, rn = 0;      // entries of the shortened chunk's old list still to test again: [rt, rn)
     int sp = 0;
-    int cur = ~0;   // one Gaussian: the root is a leaf
+    int cur = ~0;            // one Gaussian: the root is a leaf
+    bool walk = true;        // cur is still to be visited
     if (a.n_leaves > 1) {
         const int2 root = __ldg(a.wide_tab);
         cur = wide_pack(root.x, root.y);
@@ -487,47 +521,108 @@ __device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayS
     unsigned guard = 0, visits = 0;
     const unsigned guard_max = 2u * (unsigned)a.n_leaves + 64u;
     while (true) {
-        if (++guard > guard_max) {
-            if (lane == 0) atomicAdd(&a.st->watchdog_trips, 1ull);
-            break;
-        }
-        if (cur >= 0) {
-            if (DIAG) ++visits;
-            const int first = cur & ((1 << kWideCountShift) - 1), count = (cur >> kWideCountShift) + 1;
-            bool hit = false;
-            int cid = 0;
-            if (lane < count) {
-                float3 lo, hi;
-                int range_hi;
-                load_slot(a.slots + first + lane, lo, hi, cid, range_hi);
-                hit = (range_hi > cursor) && packet_hit(sm.packet, lo, hi);
-            }
-            const unsigned hm = __ballot_sync(kFull, hit);
-            if (hm) {
-                // continue with the first hit child; the later ones go on the stack in reverse order
-                // (the hit child k at the position of the hit children above it), lowest on top
-                const int f = __ffs(hm) - 1;
-                const unsigned rest = hm & (hm - 1u);
-                const int np = __popc(rest);
-                if (sp + np <= kStack) {
-                    if ((rest >> lane) & 1u) sm.stack[sp + __popc(rest >> lane) - 1] = cid;
-                    sp += np;
-                } else if (lane == 0) {
-                    atomicAdd(&a.st->stack_overflows, 1ull);
-                }
-                cur = __shfl_sync(kFull, cid, f);
-                __syncwarp();
+        const bool again = rt < rn;
+        int mine = -1, m = 0;
+        unsigned todo;
+        if (again) {
+            // in registers before its places are written again (an entry never moves up)
+            const bool in = rt + lane < rn;
+            if (in) mine = sm.ids[rt + lane];
+            todo = __ballot_sync(kFull, in && (int)(sm.urng[rt + lane] & 0xffffu) < K);
+            rt += 32;
+        } else if (np >= 32 || (np > 0 && !walk)) {
+            m = min(np, 32);
+            if (lane < m) mine = cand[lane];
+            todo = __ballot_sync(kFull, mine > cursor);
+        } else if (walk) {
+            if (++guard > guard_max) {
+                if (lane == 0) atomicAdd(&a.st->watchdog_trips, 1ull);
+                walk = false;
                 continue;
             }
+            unsigned rest = 0u;
+            if (cur >= 0) {
+                if (DIAG) ++visits;
+                const int first = cur & ((1 << kWideCountShift) - 1), n = (cur >> kWideCountShift) + 1;
+                bool hit = false;
+                int cid = 0;
+                if (lane < n) {
+                    float3 lo, hi;
+                    int range_hi;
+                    load_slot(a.slots + first + lane, lo, hi, cid, range_hi);
+                    hit = (range_hi > cursor) && packet_hit(sm.packet, lo, hi);
+                }
+                const unsigned hm = __ballot_sync(kFull, hit), im = __ballot_sync(kFull, hit && cid >= 0);
+                const unsigned lead = hm & ((im & (0u - im)) - 1u);   // leaves before the first node (all: no node)
+                if ((lead >> lane) & 1u) cand[np + __popc(lead & ((1u << lane) - 1u))] = ~cid;
+                np += __popc(lead);
+                rest = hm & ~lead;
+                if (rest) {
+                    // a hit lane's place on the stack is the number of hit children above it
+                    const int f = __ffs(rest) - 1;
+                    rest &= rest - 1u;
+                    const int more = __popc(rest);
+                    if (sp + more <= kStack) {
+                        if ((rest >> lane) & 1u) sm.stack[sp + __popc(rest >> lane) - 1] = cid;
+                        sp += more;
+                    } else if (lane == 0) {
+                        atomicAdd(&a.st->stack_overflows, 1ull);
+                    }
+                    cur = __shfl_sync(kFull, cid, f);
+                    __syncwarp();
+                    continue;
+                }
+            } else {
+                if (lane == 0) cand[np] = ~cur;
+                ++np;
+            }
+            __syncwarp();
+            if (sp == 0) walk = false;
+            else cur = sm.stack[--sp];
+            continue;
         } else {
-            int leaf = ~cur;
-            if (leaf > cursor && !leaf_entry<FAST, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, leaf, count, lane, ws, infer)) {
+            break;
+        }
+        // the exact test of the batch's leaves, in order
+        while (todo) {
+            const int leaf = __shfl_sync(kFull, mine, __ffs(todo) - 1);
+            if (!leaf_entry<FAST, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, leaf, count, lane, ws, infer)) break;
+            todo &= todo - 1u;
+        }
+        if (todo) {
+            if (K == 1) {
                 ovf = true;
                 break;
             }
+            // the list is full: shorten the chunk, then come back to this leaf
+            __syncwarp();
+            unsigned halvings = 0;
+            int kept;
+            do {
+                K >>= 1;
+                ++halvings;
+                kept = 0;
+                for (int e = lane; e < CAP; e += 32)
+                    kept += __popc(__ballot_sync(kFull, (int)(sm.urng[e] & 0xffffu) < K));
+            } while (K > 1 && kept >= CAP);
+            if (lane == 0) atomicAdd(&a.st->chunk_splits, (unsigned long long)halvings);
+            chunk_extent(r, on, K, t_end, nv, seg_hi);
+            set_packet<FAST, CAP>(sm, r, on, seg_hi, lane);
+            rt = 0;
+            rn = count;
+            count = 0;
         }
-        if (sp == 0) break;
-        cur = sm.stack[--sp];
+        __syncwarp();
+        if (!again) {
+            // the candidates after the last one tested move to the front
+            const int done = todo ? __ffs(todo) - 1 : m;
+            const int c0 = cand[done + lane], c1 = cand[done + 32 + lane];
+            __syncwarp();
+            cand[lane] = c0;
+            cand[32 + lane] = c1;
+            np -= done;
+            __syncwarp();
+        }
     }
     if (DIAG) ws.node_visits += visits;
     finish_list<FAST, CAP, DIAG>(sm, count, K, lane, ws);
@@ -540,7 +635,6 @@ template <bool FAST, int CAP, bool DIAG>
 __device__ int replay_list(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float seg_hi,
                            int K, int nv, const unsigned* ids, int n, int lane, WarpStats& ws) {
     int count = 0;
-    clear_occ(sm, lane);
     n = min(n, CAP);
     for (int base = 0; base < n; base += 32) {
         const int m = min(32, n - base);
@@ -1110,23 +1204,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                     K = max(1, min(kmax, (int)((rec_hdr >> 16) & 0xffu)));
                 }
             }
-            // slabs of this chunk: slab k is marched iff tb_k < texit (tb_k by repeated addition)
-            int nv = 0;
-            float seg_hi = r.tb;
-            if (on) {
-                if (K <= kExactChunk) {
-                    float t = r.tb;
-                    for (int kk = 0; kk < K; ++kk) {
-                        if (t < r.texit) { nv = kk + 1; t = t + kSlab; } else break;
-                    }
-                    seg_hi = fminf(t_end, t);
-                } else {
-                    nv = K;
-                    seg_hi = fminf(t_end, r.tb + (float)(K + 1) * kSlab);
-                }
-                // a slab step that no longer changes tb (|t| beyond ~2^19) would march forever
-                if (!(r.tb < r.texit) || r.tb + kSlab == r.tb) { r.alive = false; on = false; nv = 0; }
-            }
+            int nv;
+            float seg_hi;
+            // a slab step that no longer changes tb (|t| beyond ~2^19) would march forever
+            if (on && (!(r.tb < r.texit) || r.tb + kSlab == r.tb)) r.alive = on = false;
+            chunk_extent(r, on, K, t_end, nv, seg_hi);
             bool ovf = false;
             int count;
             const bool replayed = BWD && rec_cur != kNoRecord && !(rec_hdr & kRecordMulti);
@@ -1137,14 +1219,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                                                lane, ws);
                 ++ws.replays;
             } else {
-                count = traverse<FAST, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, -1, ovf, lane, ws, infer);
+                count = traverse<FAST, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, -1, ovf, lane, ws, infer);
             }
             const unsigned long long* occ = sm.occ;
-            if (ovf && K > 1) {
-                K = max(1, K >> 1);
-                if (lane == 0) atomicAdd(&a.st->chunk_splits, 1ull);
-                continue;
-            }
             if (!BWD && rec_here && sm.rec_first != kRecordFailed) {
                 // chunk record: header (multi-pass flag | K << 16 | id count), next record, ids
                 const unsigned n_ids = ovf ? 0u : (unsigned)count;
@@ -1249,7 +1326,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                     int cursor = sm.ids[count - 1];
                     __syncwarp();
                     if (lane == 0) atomicAdd(&a.st->list_passes, 1ull);
-                    count = traverse<FAST, CAP, DIAG>(sm, a, r, on, seg_hi, 1, nv, cursor, more, lane, ws, infer);
+                    count = traverse<FAST, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, more, lane, ws, infer);
                     nh += slab_buffers<FAST, CAP, BWD, DIAG>(sm, 0, 1, has, r, a, rgb_base, roff, sig, Cb, gC,
                                                        nwords(count), lane, ws);
                 }
@@ -1270,7 +1347,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                     int cursor = -1;
                     bool more2 = true;
                     while (more2) {
-                        count = traverse<FAST, CAP, DIAG>(sm, a, r, on, seg_hi, 1, nv, cursor, more2, lane, ws, infer);
+                        count = traverse<FAST, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, more2, lane, ws, infer);
                         slab_adjoint<FAST, CAP, DIAG>(sm, 0, 1, act, r, a, rgb_base, roff, H, F, nwords(count), lane, ws,
                                                       view);
                         if (more2) cursor = sm.ids[count - 1];
