@@ -20,7 +20,7 @@ constexpr int kWarp = 32;
 constexpr int kTileW = 8;               // a warp renders an 8x4 pixel tile
 constexpr int kTileH = 4;
 constexpr int kMaxChunk = 255;          // slabs per traversal chunk (slab ranges are bytes)
-constexpr int kStack = 192;             // warp traversal stack depth (up to 31 pushes per wide node)
+constexpr int kStack = 256;             // warp traversal stack depth (up to 31 pushes per wide node on the path)
 
 // Device status block (mirrors rg_status) + work counters.
 struct DevStatus {
@@ -141,14 +141,13 @@ struct __align__(16) GaussRec {
     LeafIS is;
 };
 
-// Wide traversal nodes.  Every binary node at a depth that is a multiple of kWideLevels owns the
-// frontier of its subtree kWideLevels levels down (binary nodes there, or leaves reached earlier):
-// at most kWideSlots children, stored as consecutive slots in leaf order.  A slot holds the child's
-// box, its id and the last leaf of its subtree (the multi-pass cursor test).  The id of a leaf
-// child is ~leaf (< 0); that of a wide child holds the child's own slots, first slot | (count - 1)
-// << kWideCountShift (>= 0), so a visit needs no other load.  32 bytes, one 256-bit load per lane.
-constexpr int kWideLevels = 5;
-constexpr int kWideSlots = 1 << kWideLevels;
+// Wide traversal nodes of up to kWideSlots children (one per lane), collapsed from the binary tree
+// (k_refit decides which binary nodes they are), stored as consecutive slots in leaf order.  A slot
+// holds the child's box, its id and the last leaf of its subtree (the multi-pass cursor test).  The id
+// of a leaf child is ~leaf (< 0); that of a wide child holds the child's own slots, first slot |
+// (count - 1) << kWideCountShift (>= 0), so a visit needs no other load.  32 bytes, one 256-bit load
+// per lane.  A leaf or a wide node but the root is one slot: at most 2n.
+constexpr int kWideSlots = 32;
 constexpr int kWideCountShift = 26;                       // first slot < 2^26: at most 2^25 Gaussians
 constexpr long long kMaxGaussians = 1ll << 25;
 __host__ __device__ __forceinline__ int wide_pack(int first, int count) {

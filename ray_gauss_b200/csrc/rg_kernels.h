@@ -17,9 +17,9 @@ struct BvhBuffers {
     float4* leaf_lo = nullptr;
     float4* leaf_hi = nullptr;
     Node* nodes = nullptr;
-    int* depth = nullptr;         // per binary node: depth below the root
-    int* wide_cnt = nullptr;      // per binary node: wide children (0 unless a wide node)
-    int2* wide_tab = nullptr;     // per binary node: {first slot, slot count} of its wide node
+    int* depth = nullptr;         // per binary node: its units while building, then the first slot
+    int* wide_cnt = nullptr;      // per binary node: slots (0 unless a wide node)
+    int2* wide_tab = nullptr;     // per binary node: .y its units, > 0 for a wide node; entry 0: {0, slots} of the root
     WideSlot* slots = nullptr;    // wide-node children (at most 2n slots)
     int* leaf_parent = nullptr;
     int* node_parent = nullptr;
@@ -36,7 +36,7 @@ struct RenderArgs {
     const LeafIS* is_rec;
     const float4* ext;
     const float4* rgb;            // (n_views, n_leaves) leaf order
-    const int2* wide_tab;         // wide node of binary node i: {first slot, slot count} (root: entry 0)
+    const int2* wide_tab;         // entry 0: {first slot, slot count} of the root
     const WideSlot* slots;        // wide-node children
     int n_leaves;
     const int* scene_ord;
