@@ -75,6 +75,7 @@ struct WarpSmem {
     unsigned smask[NB][CAP / 32];                    // entries whose union range meets block k / MB
     unsigned long long occ[4];                       // slabs holding any entry (union occupancy)
     __align__(16) float packet[24];                  // the chunk's ray packet (set_packet), read as float4
+    __align__(16) float cone[12];                    // the tile's ray directions (set_cone), read as float4
     int stack[kStack];
     // hit-list record of the warp's current tile (written by lane 0)
     unsigned rec_first, rec_prev;                    // forward: first / last chunk record
@@ -197,6 +198,73 @@ __device__ __forceinline__ bool packet_hit(const float* F, float3 lo, float3 hi)
     return in_box && fmaxf(max3f(ix, iy, iz), qt.x) <= fminf(min3f(ox, oy, oz), qt.y);
 }
 
+// The tile's ray directions before normalisation, w + u dx + v dy, as centre + s * cone_u + t * cone_v
+// with s and t in [-1, 1]: {centre.xyz, cone_u.x}, {cone_u.yz, cone_v.xy}, {cone_v.z,
+// smallest and largest length, -}.
+template <bool FAST, int CAP>
+__device__ __forceinline__ void set_cone(WarpSmem<FAST, CAP>& sm, const rg_camera& cam, float dx, float dy, bool valid,
+                                         int lane) {
+    const float x0 = ord2f(__reduce_min_sync(kFull, valid ? f2ord(dx) : 0x7fffffff));
+    const float x1 = ord2f(__reduce_max_sync(kFull, valid ? f2ord(dx) : (int)0x80000000));
+    const float y0 = ord2f(__reduce_min_sync(kFull, valid ? f2ord(dy) : 0x7fffffff));
+    const float y1 = ord2f(__reduce_max_sync(kFull, valid ? f2ord(dy) : (int)0x80000000));
+    if (lane == 0) {
+        const float xc = 0.5f * (x0 + x1), yc = 0.5f * (y0 + y1), hx = 0.5f * (x1 - x0), hy = 0.5f * (y1 - y0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            sm.cone[c] = fmaf(cam.u[c], xc, fmaf(cam.v[c], yc, cam.w[c]));
+            sm.cone[3 + c] = cam.u[c] * hx;
+            sm.cone[6 + c] = cam.v[c] * hy;
+        }
+        // bounds of |D| over the tile
+        const float dc = sqrtf(dot3(f3(sm.cone[0], sm.cone[1], sm.cone[2]), f3(sm.cone[0], sm.cone[1], sm.cone[2])));
+        const float dh = sqrtf(dot3(f3(sm.cone[3], sm.cone[4], sm.cone[5]), f3(sm.cone[3], sm.cone[4], sm.cone[5]))) +
+                         sqrtf(dot3(f3(sm.cone[6], sm.cone[7], sm.cone[8]), f3(sm.cone[6], sm.cone[7], sm.cone[8])));
+        sm.cone[9] = fmaxf(dc - dh, 0.f);
+        sm.cone[10] = dc + dh;
+    }
+}
+
+// Whether a ray of the tile may meet the leaf's threshold ellipsoid at ray parameters in [t0, t1] (one
+// leaf per lane), and a lower bound of the parameter where it does.  In the space of m = M (x - mu) the
+// ellipsoid is a sphere of radius R = 1 / k around 0 and the rays leave O = M (o - mu) along C + s U +
+// t V (the images of the cone).  With e the unit vector along C, b = -O.e and p the unit vector from
+// the central ray towards the sphere's centre, rho away, take the plane through O that is p tilted
+// towards the rays until all of them lie under it: the tilt's tangent is tau = (|p.U| + |p.V|) /
+// (|C| - |e.U| - |e.V|), and the centre's height over the plane is (rho - b tau) / sqrt(1 + tau^2).
+// No ray reaches a sphere that lies over the plane.  Along e the sphere spans b -+ R and a ray moves
+// by (|C| -+ |e.U| -+ |e.V|) / |D| per unit of its parameter.  The margin, a thousandth of R and 1e-5
+// of |O|, is above the rounding of this test and of the exact one by a factor of ten.  NaN (a
+// Gaussian that is never hit, an overflow) keeps the leaf: the exact test decides.
+template <bool FAST, int CAP>
+__device__ __forceinline__ bool may_hit(const WarpSmem<FAST, CAP>& sm, const LeafRec& rec, float3 o, float t0, float t1,
+                                        float& t_first) {
+    const float4 q0 = *reinterpret_cast<const float4*>(sm.cone), q1 = *reinterpret_cast<const float4*>(sm.cone + 4),
+                 q2 = *reinterpret_cast<const float4*>(sm.cone + 8);
+    const float3 dc = f3(q0.x, q0.y, q0.z), du = f3(q0.w, q1.x, q1.y), dv = f3(q1.z, q1.w, q2.x);
+    const float3 r0 = f3(rec.r0.x, rec.r0.y, rec.r0.z), r1 = f3(rec.r1.x, rec.r1.y, rec.r1.z),
+                 r2 = f3(rec.r2.x, rec.r2.y, rec.r2.z);
+    const float3 v = f3(rec.a.x, rec.a.y, rec.a.z) - o;
+    const float3 O = f3(dot3(r0, v), dot3(r1, v), dot3(r2, v));   // -O: from the eye to the centre
+    const float3 C = f3(dot3(r0, dc), dot3(r1, dc), dot3(r2, dc));
+    const float3 U = f3(dot3(r0, du), dot3(r1, du), dot3(r2, du));
+    const float3 V = f3(dot3(r0, dv), dot3(r1, dv), dot3(r2, dv));
+    const float c2 = dot3(C, C), ic = rsqrtf(c2), c1 = c2 * ic;
+    const float3 e = C * ic;
+    const float b = dot3(O, e);
+    const float3 P = O - e * b;
+    const float rho2 = dot3(P, P), ir = rsqrtf(rho2);
+    const float rho = rho2 * ir;
+    const float width = (fabsf(dot3(P, U)) + fabsf(dot3(P, V))) * ir;
+    const float spread = fabsf(dot3(e, U)) + fabsf(dot3(e, V));
+    const float along = c1 - spread;
+    const float R = __fdividef(1.f, rec.r0.w) * 1.001f + 1e-5f * (rho + fabsf(b));
+    const bool miss = along > 0.f && rho * along - b * width > R * sqrtf(along * along + width * width);
+    t_first = __fdividef(fmaxf(b - R, 0.f) * q2.y, c1 + spread) * 0.99999f;
+    const bool before = along > 0.f && (b + R) * q2.z * 1.00001f < t0 * along, after = t_first > t1;
+    return !(miss || before || after);
+}
+
 __device__ __forceinline__ LeafRec load_rec(const LeafRec* p, int i) {
     const float4* q = reinterpret_cast<const float4*>(p + i);
     LeafRec r;
@@ -283,43 +351,30 @@ __device__ __noinline__ bool slab_k_hit(float tb, float tenter, float texit, int
     return th > tenter && fmaxf(t, root1) <= fminf(th, root2);
 }
 
-// Longer chunks map the interval arithmetically.  Slab k starts at tb_k, tb plus k slabs by repeated
-// FP32 addition, and is hit iff root1 <= tb_k + 0.02 and tb_k <= root2.  The range keeps a margin
-// that covers the drift of the repeated addition, so it holds every hit slab and at most one extra
-// slab at each end: the parity arithmetic settles the ends exactly here, the fast arithmetic
-// evaluates them (their samples fall outside the threshold ellipsoid).
+// The interval's slabs, mapped arithmetically.  Slab k starts at tb_k, tb plus k slabs by repeated FP32
+// addition, and is hit iff root1 <= tb_k + 0.02 and tb_k <= root2.  The range keeps a margin that
+// covers the drift of the repeated addition, so it holds every hit slab and at most one extra slab at
+// each end.  Chunks up to kExactChunk and the parity arithmetic settle the ends exactly here; in
+// longer chunks the fast arithmetic evaluates them (their samples fall outside the threshold
+// ellipsoid).
 template <bool FAST>
 __device__ __forceinline__ void slab_range(const RayState& r, int K, int nv, float seg_hi, float tclip, float root1,
                                            float root2, int& lo, int& hi) {
     lo = 255;
     hi = -1;
-    if (K <= kExactChunk) {
-        // exact: the reference's per-slab test max(tmin, root1) <= min(tmax, root2)
-        float t = r.tb;
-#pragma unroll
-        for (int kk = 0; kk < kExactChunk; ++kk) {
-            if (kk < nv) {
-                float tn = t + kSlab;
-                float th = fminf(tclip, tn);
-                if (th > r.tenter && fmaxf(t, root1) <= fminf(th, root2)) {
-                    lo = min(lo, kk);
-                    hi = kk;
-                }
-                t = tn;
-            }
-        }
-    } else if (fmaxf(r.tb, root1) <= fminf(seg_hi, root2)) {
+    if (fmaxf(r.tb, root1) <= fminf(seg_hi, root2)) {
+        // (the eight tests of a short chunk one after the other took twice the instructions)
         float a = fmaxf((root1 - r.tb) * kInvSlab, -1.f);
         float b = fminf((root2 - r.tb) * kInvSlab, 4096.f);
         // drift of tb_k in slab units: (K + 1) ulps of |tb| + K slabs, 2^-23 relative each (four
         // times the bound of round-to-nearest additions)
         const float m = (float)(K + 1) * (fabsf(r.tb) + (float)K * kSlab) * (kInvSlab * 2.4e-7f) + 1e-4f;
         lo = max(0, (int)ceilf(a - 1.f - m));
-        hi = min(K - 1, (int)floorf(b + m));
-        if (!FAST) {
-            // Parity: settle both ends exactly.  A slab whose hit or miss the margins cannot decide
-            // gets the reference's per-slab test (rare: its interval end lies within the margin
-            // of a slab edge or of the box exit).
+        hi = min(nv - 1, (int)floorf(b + m));
+        if (!FAST || K <= kExactChunk) {
+            // Settle both ends exactly.  A slab whose hit or miss the margins cannot decide gets the
+            // reference's per-slab test (rare: its interval end lies within the margin of a slab
+            // edge or of the box exit).
             const float e = fminf((tclip - r.tb) * kInvSlab, 4096.f);
             while (lo <= hi) {
                 const int c = classify_slab(lo, a, b, e, m);
@@ -484,32 +539,38 @@ __device__ __forceinline__ void chunk_extent(const RayState& r, bool on, int K, 
 }
 
 // Warp-cooperative traversal for the chunk [tb, seg_hi] of every active lane (the packet set by
-// set_packet).  At a wide node lane k tests child slot k against the packet.  Hit leaves go to a
-// candidate buffer (the leading ones of a node all at once); the first hit child that is a node is
+// set_packet).  At a wide node lane k tests child slot k against the packet.  Hit leaves wait in a
+// buffer (the leading ones of a node are taken all at once); the first hit child that is a node is
 // visited next and the children after it wait on the stack, the lowest index on top, so leaves are
-// reached in increasing index (the multi-pass cursor relies on it).  Candidates are taken 32 at a
-// time: the leaves with index > cursor get the exact test per ray, and those that any ray hits
-// are appended to the warp list, whose entry count is returned.
+// reached in increasing index (the multi-pass cursor relies on it).  Thirty-two waiting leaves at a
+// time, one per lane, may_hit drops those that no ray of the tile meets; the candidates that remain
+// keep the first slab that they can reach.  When the tree is through, the candidates get the exact
+// test per ray, and those that any ray hits are appended to the warp list, whose entry count is
+// returned.  A leaf costs a visit's warp 1/32 of may_hit instead of a whole exact test: on 1M
+// Gaussians x 16 views 214M exact tests instead of 581M (122M entries used), forward 214.7 -> 196.8
+// ms; 3M x 4 x 1080p: 118.4 -> 98.3 ms.
 //
-// A list that fills up shortens the chunk (K, nv and seg_hi) in place: K is halved until an entry drops
-// out (one starting at slab K or later holds no slab of the shorter chunk), the entries that stay get
-// the exact test again for the shorter chunk, and the traversal goes on from its stack with the
-// smaller packet.  The list is the one that a traversal started with the shorter chunk builds, and
-// nothing is visited twice.  (Starting over, a tile that came on dense space with a long chunk filled
-// and dropped the list once per halving: 1M Gaussians x 16 views, 13M rays, appended 300M entries for
-// 122M used.  With this, and with the list published a ballot at a time, that forward went from
-// 272.6 to 234.4 ms and its backward, which publishes replayed lists, from 273.6 to 260.9 ms.)
-// `ovf` is set when the list filled up for a single slab before the traversal finished.
+// A chunk with too many Gaussians is shortened in place (K, nv and seg_hi): when the candidates or the
+// list fill up, K is halved until there is room, what starts at slab K or later is dropped (it holds
+// no slab of the shorter chunk), entries of the list that stay get the exact test again, and the
+// traversal goes on from its stack with the smaller packet.  The list is the one that a traversal
+// started with the shorter chunk builds, and nothing is visited twice.  `ovf` is set when the list
+// filled up for a single slab before the traversal finished.
 template <bool FAST, int CAP, bool DIAG>
 __device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float t_end,
                         float& seg_hi, int& K, int& nv, int cursor, bool& ovf, int lane, WarpStats& ws, bool infer) {
     int count = 0;
     ++ws.traversals;
     ovf = false;
-    // candidates: the entry masks' space, which finish_list writes only afterwards
-    int* const cand = reinterpret_cast<int*>(&sm.smask[0][0]);
-    static_assert(sizeof(sm.smask) >= 96 * sizeof(int), "up to 63 candidates, read 32 at a time from any of the first 32");
-    int np = 0;              // candidates waiting
+    // Candidates [0, nc), then leaves still waiting for may_hit [nc, nc + nr): the entry masks' space,
+    // which finish_list writes only afterwards.  A candidate is leaf | (first slab / 2) << 25.
+    unsigned* const cand = &sm.smask[0][0];
+    constexpr int NC = 2 * CAP;
+    static_assert(sizeof(sm.smask) >= NC * sizeof(unsigned) && NC >= 256, "candidate buffer");
+    static_assert(kMaxGaussians == 1ll << 25, "25 bits of a candidate hold the leaf");
+    constexpr unsigned kLeafMask = (1u << 25) - 1u;
+    int nc = 0, nr = 0;
+    int done = 0;            // candidates that had the exact test
     int rt = 0, rn = 0;      // entries of the shortened chunk's old list still to test again: [rt, rn)
     int sp = 0;
     int cur = ~0;            // one Gaussian: the root is a leaf
@@ -521,20 +582,32 @@ __device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayS
     unsigned guard = 0, visits = 0;
     const unsigned guard_max = 2u * (unsigned)a.n_leaves + 64u;
     while (true) {
-        const bool again = rt < rn;
-        int mine = -1, m = 0;
-        unsigned todo;
-        if (again) {
-            // in registers before its places are written again (an entry never moves up)
-            const bool in = rt + lane < rn;
-            if (in) mine = sm.ids[rt + lane];
-            todo = __ballot_sync(kFull, in && (int)(sm.urng[rt + lane] & 0xffffu) < K);
-            rt += 32;
-        } else if (np >= 32 || (np > 0 && !walk)) {
-            m = min(np, 32);
-            if (lane < m) mine = cand[lane];
-            todo = __ballot_sync(kFull, mine > cursor);
-        } else if (walk) {
+        if (rt >= rn && done == 0 && (nr >= 32 || (nr > 0 && !walk))) {
+            // may_hit for up to 32 waiting leaves; the rest moves up behind the candidates
+            const int m = min(nr, 32);
+            const unsigned leaf = lane < m ? cand[nc + lane] : 0u;
+            const unsigned next = 32 + lane < nr ? cand[nc + 32 + lane] : 0u;
+            // slab s of a lane starts at tb + 0.02 s up to the drift of the repeated addition
+            const float tb0 = __uint_as_float(__reduce_min_sync(kFull, on ? __float_as_uint(r.tb) : 0x7f800000u));
+            const float tb1 = __uint_as_float(__reduce_max_sync(kFull, on ? __float_as_uint(r.tb) : 0u));
+            const float t1 = __uint_as_float(__reduce_max_sync(kFull, on ? __float_as_uint(seg_hi) : 0u));
+            bool may = lane < m && (int)leaf > cursor;
+            int first = 0;
+            if (may) {
+                float t;
+                may = may_hit<FAST, CAP>(sm, load_rec(a.rec, (int)leaf), r.o, tb0 * 0.99999f, t1 * 1.00001f, t);
+                const float drift = (float)(K + 1) * (tb1 + (float)K * kSlab) * (kInvSlab * 2.4e-7f);
+                first = min(255, max(0, (int)((t - tb1) * kInvSlab - 1.f - drift)));
+                may = may && first < K;
+            }
+            const unsigned mm = __ballot_sync(kFull, may);
+            if (may) cand[nc + __popc(mm & ((1u << lane) - 1u))] = leaf | ((unsigned)(first >> 1) << 25);
+            nc += __popc(mm);
+            nr -= m;
+            __syncwarp();
+            if (lane < nr) cand[nc + lane] = next;
+            __syncwarp();
+        } else if (walk && nc <= NC - 64 && rt >= rn && done == 0) {
             if (++guard > guard_max) {
                 if (lane == 0) atomicAdd(&a.st->watchdog_trips, 1ull);
                 walk = false;
@@ -554,8 +627,8 @@ __device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayS
                 }
                 const unsigned hm = __ballot_sync(kFull, hit), im = __ballot_sync(kFull, hit && cid >= 0);
                 const unsigned lead = hm & ((im & (0u - im)) - 1u);   // leaves before the first node (all: no node)
-                if ((lead >> lane) & 1u) cand[np + __popc(lead & ((1u << lane) - 1u))] = ~cid;
-                np += __popc(lead);
+                if ((lead >> lane) & 1u) cand[nc + nr + __popc(lead & ((1u << lane) - 1u))] = (unsigned)~cid;
+                nr += __popc(lead);
                 rest = hm & ~lead;
                 if (rest) {
                     // a hit lane's place on the stack is the number of hit children above it
@@ -573,54 +646,97 @@ __device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayS
                     continue;
                 }
             } else {
-                if (lane == 0) cand[np] = ~cur;
-                ++np;
+                if (lane == 0) cand[nc + nr] = (unsigned)~cur;
+                ++nr;
             }
             __syncwarp();
             if (sp == 0) walk = false;
             else cur = sm.stack[--sp];
-            continue;
-        } else {
-            break;
-        }
-        // the exact test of the batch's leaves, in order
-        while (todo) {
-            const int leaf = __shfl_sync(kFull, mine, __ffs(todo) - 1);
-            if (!leaf_entry<FAST, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, leaf, count, lane, ws, infer)) break;
-            todo &= todo - 1u;
-        }
-        if (todo) {
-            if (K == 1) {
-                ovf = true;
-                break;
-            }
-            // the list is full: shorten the chunk, then come back to this leaf
-            __syncwarp();
+        } else if (walk && nc > NC - 64 && K > 1 && rt >= rn && done == 0) {
+            // the candidates are many: shorten the chunk and drop those beyond it
             unsigned halvings = 0;
             int kept;
             do {
                 K >>= 1;
                 ++halvings;
                 kept = 0;
-                for (int e = lane; e < CAP; e += 32)
-                    kept += __popc(__ballot_sync(kFull, (int)(sm.urng[e] & 0xffffu) < K));
-            } while (K > 1 && kept >= CAP);
+                for (int e = 0; e < nc; e += 32)
+                    kept += __popc(__ballot_sync(kFull, e + lane < nc && 2 * (int)(cand[e + lane] >> 25) < K));
+            } while (K > 1 && kept > NC - 64);
             if (lane == 0) atomicAdd(&a.st->chunk_splits, (unsigned long long)halvings);
             chunk_extent(r, on, K, t_end, nv, seg_hi);
             set_packet<FAST, CAP>(sm, r, on, seg_hi, lane);
-            rt = 0;
-            rn = count;
-            count = 0;
-        }
-        __syncwarp();
-        if (!again) {
-            // the candidates after the last one tested move to the front
-            const int done = todo ? __ffs(todo) - 1 : m;
-            const int c0 = cand[done + lane], c1 = cand[done + 32 + lane];
+            int to = 0;
+            for (int e = 0; e < nc; e += 32) {
+                const unsigned c = e + lane < nc ? cand[e + lane] : 0u;
+                const unsigned km = __ballot_sync(kFull, e + lane < nc && 2 * (int)(c >> 25) < K);
+                if ((km >> lane) & 1u) cand[to + __popc(km & ((1u << lane) - 1u))] = c;
+                to += __popc(km);
+                __syncwarp();
+            }
+            // the waiting leaves move up behind the candidates
+            const unsigned w0 = lane < nr ? cand[nc + lane] : 0u, w1 = 32 + lane < nr ? cand[nc + 32 + lane] : 0u;
             __syncwarp();
-            cand[lane] = c0;
-            cand[32 + lane] = c1;
-            np -= done;
+            if (lane < nr) cand[to + lane] = w0;
+            if (32 + lane < nr) cand[to + 32 + lane] = w1;
+            nc = to;
+            __syncwarp();
+        } else {
+            // exact tests, in order: the list's entries again after a chunk was shortened, else candidates
+            const bool again = rt < rn;
+            unsigned todo;
+            unsigned mine = 0u;
+            if (again) {
+                // in registers before its places are written again (an entry never moves up)
+                const bool in = rt + lane < rn;
+                if (in) mine = (unsigned)sm.ids[rt + lane];
+                todo = __ballot_sync(kFull, in && (int)(sm.urng[rt + lane] & 0xffffu) < K);
+                rt += 32;
+            } else {
+                if (done >= nc) {
+                    if (!walk) break;
+                    // a single slab: its candidates are in the list, the tree goes on (under 32 leaves wait)
+                    const unsigned w = lane < nr ? cand[nc + lane] : 0u;
+                    __syncwarp();
+                    if (lane < nr) cand[lane] = w;
+                    nc = done = 0;
+                    __syncwarp();
+                    continue;
+                }
+                const bool in = done + lane < nc;
+                const unsigned c = in ? cand[done + lane] : 0u;
+                mine = c & kLeafMask;
+                todo = __ballot_sync(kFull, in && 2 * (int)(c >> 25) < K);
+            }
+            while (todo) {
+                const int leaf = (int)__shfl_sync(kFull, mine, __ffs(todo) - 1);
+                if (!leaf_entry<FAST, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, leaf, count, lane, ws, infer)) break;
+                todo &= todo - 1u;
+            }
+            if (!again) done = min(nc, done + (todo ? __ffs(todo) - 1 : 32));
+            if (todo) {
+                if (K == 1) {
+                    ovf = true;
+                    break;
+                }
+                // the list is full: shorten the chunk, test its entries again, then come back to this leaf
+                __syncwarp();
+                unsigned halvings = 0;
+                int kept;
+                do {
+                    K >>= 1;
+                    ++halvings;
+                    kept = 0;
+                    for (int e = lane; e < CAP; e += 32)
+                        kept += __popc(__ballot_sync(kFull, (int)(sm.urng[e] & 0xffffu) < K));
+                } while (K > 1 && kept >= CAP);
+                if (lane == 0) atomicAdd(&a.st->chunk_splits, (unsigned long long)halvings);
+                chunk_extent(r, on, K, t_end, nv, seg_hi);
+                set_packet<FAST, CAP>(sm, r, on, seg_hi, lane);
+                rt = 0;
+                rn = count;
+                count = 0;
+            }
             __syncwarp();
         }
     }
@@ -1150,6 +1266,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
             float inv = __fdiv_rn(1.f, __fsqrt_rn(dot_rn(dir, dir)));
             r.d = f3(__fmul_rn(dir.x, inv), __fmul_rn(dir.y, inv), __fmul_rn(dir.z, inv));
             r.o = f3(cam.eye[0], cam.eye[1], cam.eye[2]);
+            set_cone<FAST, CAP>(sm, cam, dx, dy, valid, lane);
         }
         {
             float scene[6];   // scene box, read per tile (not kept live through the tile's loops)
@@ -1438,6 +1555,9 @@ static_assert(sizeof(WarpSmem<false, 128>) * kWarpsPerBlock <= 48 * 1024, "stati
 using ParitySmem = WarpSmem<false, 128>;
 using FastSmem256 = WarpSmem<true, 256>;
 using FastSmem512 = WarpSmem<true, 512>;
+static_assert(offsetof(ParitySmem, cone) % 16 == 0 && offsetof(FastSmem256, cone) % 16 == 0 &&
+                  offsetof(FastSmem512, cone) % 16 == 0,
+              "cone alignment");
 static_assert(offsetof(ParitySmem, packet) % 16 == 0 && sizeof(ParitySmem) % 16 == 0, "packet alignment");
 static_assert(offsetof(FastSmem256, packet) % 16 == 0 && sizeof(FastSmem256) % 16 == 0, "packet alignment");
 static_assert(offsetof(FastSmem512, packet) % 16 == 0 && sizeof(FastSmem512) % 16 == 0, "packet alignment");
