@@ -100,7 +100,9 @@ __global__ void __launch_bounds__(128) k_color_fwd(long long n, const float* __r
                 if (k < nsh) res[c] += B[k] * coef[c][k];
             res[c] += 0.5f;
         }
-        rgb_leaf[(long long)v * n + leaf] = make_float4(res[0], res[1], res[2], 0.f);
+        // .w: 1 when a channel is not finite (the parity kernels then add only the samples that count)
+        const bool odd = !(isfinite(res[0]) && isfinite(res[1]) && isfinite(res[2]));
+        rgb_leaf[(long long)v * n + leaf] = make_float4(res[0], res[1], res[2], odd ? 1.f : 0.f);
         if (rgb_out) {
             float* o = rgb_out + ((long long)v * n + g) * 3;
             o[0] = res[0]; o[1] = res[1]; o[2] = res[2];

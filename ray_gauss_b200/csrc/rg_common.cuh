@@ -103,6 +103,40 @@ __device__ __forceinline__ float lg2_approx(float x) {
     return y;
 }
 
+// Two FP32 values in one 64-bit register pair: the packed instructions (f32x2, sm_100) do two IEEE
+// round-to-nearest operations per issue slot, and each half rounds like the scalar operation.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pk(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ f2 dup2(float a) { return pk(a, a); }
+__device__ __forceinline__ float lo2(f2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi2(f2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// The product as a fused multiply-add of `nz`, a pair of -0 that the assembler cannot see through (a
+// kernel argument): the same value, and never contracted with a following addition, which a packed
+// multiplication is even with its rounding given.
+__device__ __forceinline__ f2 mul2_rn(f2 a, f2 b, f2 nz) { return fma2(a, b, nz); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Half h (0 or 1, a constant after unrolling) of a pair, read and replaced.
+__device__ __forceinline__ float half2(f2 v, int h) { return h ? hi2(v) : lo2(v); }
+__device__ __forceinline__ f2 with_half2(f2 v, int h, float x) { return h ? pk(lo2(v), x) : pk(x, hi2(v)); }
+
 // tea<4>(v0, v1) seeding and LCG draws of the reference RNG (forward/gaussians_aabb.h:63-94).
 __device__ __forceinline__ unsigned tea4(unsigned v0, unsigned v1) {
     unsigned s0 = 0;

@@ -67,6 +67,7 @@ struct RenderArgs {
     // conic-space sample stepping (parity arithmetic), optional Gaussians per ray
     int infer;
     int* counts;
+    f2 neg_zero;               // a pair of -0 (see mul2_rn; set by launch_render)
     int diag;                  // 1: count the fine-grained traversal/list statistics (rg_tuning.diagnostics)
 };
 

@@ -779,47 +779,73 @@ __device__ __forceinline__ unsigned slab_offsets(int rnd_sample, unsigned seed, 
     return seed;
 }
 
-// Exponent -|M (o + t d - mu)|^2 / 2 of a sample in the reference's operation order.
-__device__ __forceinline__ float parity_power(float3 o, float3 d, float t, float3 mu, float3 r0, float3 r1,
-                                              float3 r2) {
-    const float3 x = f3(__fadd_rn(o.x, __fmul_rn(d.x, t)), __fadd_rn(o.y, __fmul_rn(d.y, t)),
-                        __fadd_rn(o.z, __fmul_rn(d.z, t)));
-    const float3 v = f3(__fsub_rn(x.x, mu.x), __fsub_rn(x.y, mu.y), __fsub_rn(x.z, mu.z));
-    const float3 m = rows_rn(r0, r1, r2, v);
-    return __fmul_rn(-0.5f, dot_rn(m, m));
-}
+// Parity arithmetic: the eight samples of a slab in four pairs (samples 2p and 2p + 1), each operation
+// a packed one with the reference's rounding and order.  The unfused multiplies and adds are what the
+// parity kernels spend their issue slots on, and a packed instruction does two of them.
+constexpr int kPairs = kBuf / 2;
 
-__device__ __forceinline__ float parity_time(float tb, int i, int rnd_sample, const float* roff) {
-    float t = __fadd_rn(tb, __fmul_rn((float)i, kDt));
-    if (rnd_sample) t = __fadd_rn(t, roff[i]);
-    return t;
-}
-
-// Reference-order weights w[i] of the 8 samples of a slab for one Gaussian, and the mask of the
-// samples whose density * weight exceeds 0.1.  The eight weights are computed first, without
-// branches, so their dependency chains interleave; a sample whose density * weight lies within the
-// exponential's error of 0.1 is then re-evaluated with a correctly rounded weight, so that the
-// threshold decision is the one of the FP32 reference arithmetic.
-__device__ __forceinline__ unsigned parity_weights(const RayState& r, int rnd_sample, const float* roff, float3 mu,
-                                                   float3 r0, float3 r1, float3 r2, float dn, float* w) {
-    unsigned near = 0u;
+// Sample times of a slab (the reference's order: tb + i dt, then the offset).
+__device__ __forceinline__ void parity_times(float tb, int rnd_sample, const float* roff, f2* t) {
 #pragma unroll
-    for (int i = 0; i < kBuf; ++i) {
-        w[i] = expf(parity_power(r.o, r.d, parity_time(r.tb, i, rnd_sample, roff), mu, r0, r1, r2));
-        near |= (fabsf(__fmul_rn(dn, w[i]) - kSigThr) < 4e-8f ? 1u : 0u) << i;
+    for (int p = 0; p < kPairs; ++p) {
+        t[p] = add2(dup2(tb), pk((float)(2 * p) * kDt, (float)(2 * p + 1) * kDt));
+        if (rnd_sample) t[p] = add2(t[p], pk(roff[2 * p], roff[2 * p + 1]));
     }
-    if (near) {
+}
+
+// Sample positions o + t d of a slab, the same for all its Gaussians.
+struct SlabPoints {
+    f2 x[kPairs], y[kPairs], z[kPairs];
+    __device__ __forceinline__ void set(const RayState& r, const f2* t, f2 nz) {
 #pragma unroll
-        for (int i = 0; i < kBuf; ++i) {
-            if ((near >> i) & 1u)
-                w[i] = (float)exp((double)parity_power(r.o, r.d, parity_time(r.tb, i, rnd_sample, roff), mu, r0, r1,
-                                                       r2));
+        for (int p = 0; p < kPairs; ++p) {
+            x[p] = add2(dup2(r.o.x), mul2_rn(dup2(r.d.x), t[p], nz));
+            y[p] = add2(dup2(r.o.y), mul2_rn(dup2(r.d.y), t[p], nz));
+            z[p] = add2(dup2(r.o.z), mul2_rn(dup2(r.d.z), t[p], nz));
         }
     }
-    unsigned in = 0u;
+};
+
+__device__ __forceinline__ f2 dot2_rn(f2 ax, f2 ay, f2 az, f2 bx, f2 by, f2 bz, f2 nz) {
+    return add2(add2(mul2_rn(ax, bx, nz), mul2_rn(ay, by, nz)), mul2_rn(az, bz, nz));
+}
+
+// exp of the eight exponents, correctly rounded (out of line: rare)
+__device__ __noinline__ float exp_exact(float x) { return (float)exp((double)x); }
+
+// Reference-order weights exp(-|M (x - mu)|^2 / 2) of the slab's samples, zero for the samples whose
+// density * weight does not exceed 0.1.  A sample whose density * weight lies within the
+// exponential's error of 0.1 is decided with a correctly rounded weight, so that the decision is the
+// one of the FP32 reference arithmetic.
+__device__ __forceinline__ void parity_weights(const SlabPoints& sp, const LeafRec& rec, f2* w, f2 nz) {
+    const f2 mx = dup2(-rec.a.x), my = dup2(-rec.a.y), mz = dup2(-rec.a.z), dn = dup2(rec.a.w);
+    const f2 r0x = dup2(rec.r0.x), r0y = dup2(rec.r0.y), r0z = dup2(rec.r0.z);
+    const f2 r1x = dup2(rec.r1.x), r1y = dup2(rec.r1.y), r1z = dup2(rec.r1.z);
+    const f2 r2x = dup2(rec.r2.x), r2y = dup2(rec.r2.y), r2z = dup2(rec.r2.z);
+    f2 q[kPairs], d[kPairs];
+    float near = INFINITY;
 #pragma unroll
-    for (int i = 0; i < kBuf; ++i) in |= (__fmul_rn(dn, w[i]) > kSigThr ? 1u : 0u) << i;
-    return in;
+    for (int p = 0; p < kPairs; ++p) {
+        const f2 vx = add2(sp.x[p], mx), vy = add2(sp.y[p], my), vz = add2(sp.z[p], mz);
+        const f2 m0 = dot2_rn(r0x, r0y, r0z, vx, vy, vz, nz), m1 = dot2_rn(r1x, r1y, r1z, vx, vy, vz, nz),
+                 m2 = dot2_rn(r2x, r2y, r2z, vx, vy, vz, nz);
+        q[p] = mul2(dup2(-0.5f), dot2_rn(m0, m1, m2, m0, m1, m2, nz));
+        w[p] = pk(expf(lo2(q[p])), expf(hi2(q[p])));
+        d[p] = mul2_rn(dn, w[p], nz);
+        const f2 off = add2(d[p], dup2(-kSigThr));
+        near = fminf(near, fminf(fabsf(lo2(off)), fabsf(hi2(off))));
+    }
+    if (near < 4e-8f) {
+#pragma unroll
+        for (int p = 0; p < kPairs; ++p) {
+            if (fabsf(lo2(d[p]) - kSigThr) < 4e-8f) w[p] = pk(exp_exact(lo2(q[p])), hi2(w[p]));
+            if (fabsf(hi2(d[p]) - kSigThr) < 4e-8f) w[p] = pk(lo2(w[p]), exp_exact(hi2(q[p])));
+            d[p] = mul2_rn(dn, w[p], nz);
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p)
+        w[p] = pk(lo2(d[p]) > kSigThr ? lo2(w[p]) : 0.f, hi2(d[p]) > kSigThr ? hi2(w[p]) : 0.f);
 }
 
 __device__ __forceinline__ bool in_range(unsigned short rg, int k) {
@@ -839,13 +865,59 @@ __device__ __forceinline__ bool lane_has_entry(const WarpSmem<FAST, CAP>& sm, co
     return k >= (int)(rg & 0xff) && k <= (int)(rg >> 8);
 }
 
-// Sample buffers of slab k: sum of density and density-weighted colour of the lane's hits.  The
-// backward (GDOT) needs the colour only through g . C, so it accumulates that scalar in gC instead.
+// Sample buffers of a slab: density sums and, in the forward, the density-weighted colours; in the
+// backward (GDOT), which needs the colour only through g . C, the sums of -(g . colour) * density (parity
+// arithmetic) or of (g . colour) * density (fast).
+template <bool FAST, bool GDOT>
+struct SlabBuf {
+    float sig[kBuf];
+    float3 C[GDOT ? 1 : kBuf];
+    float gC[GDOT ? kBuf : 1];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int i = 0; i < kBuf; ++i) {
+            sig[i] = 0.f;
+            if constexpr (GDOT) gC[i] = 0.f;
+            else C[i] = f3(0.f, 0.f, 0.f);
+        }
+    }
+    __device__ __forceinline__ bool any_density() const {
+        bool any = false;
+#pragma unroll
+        for (int i = 0; i < kBuf; ++i) any |= sig[i] > 0.f;
+        return any;
+    }
+};
+template <bool GDOT>
+struct SlabBuf<false, GDOT> {
+    f2 sig[kPairs];
+    f2 cx[GDOT ? 1 : kPairs], cy[GDOT ? 1 : kPairs], cz[GDOT ? 1 : kPairs];
+    f2 ng[GDOT ? kPairs : 1];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int p = 0; p < kPairs; ++p) {
+            sig[p] = 0ull;
+            if constexpr (GDOT) ng[p] = 0ull;
+            else cx[p] = cy[p] = cz[p] = 0ull;
+        }
+    }
+    // sums of densities are zero or positive: their bits are zero exactly where nothing was added
+    __device__ __forceinline__ bool any_density() const { return (sig[0] | sig[1] | sig[2] | sig[3]) != 0ull; }
+};
+static_assert(kPairs == 4, "four sample pairs per slab");
+
+// Sample buffers of slab k: the sums over the lane's hits.
 template <bool FAST, int CAP, bool GDOT, bool DIAG>
 __device__ __forceinline__ int slab_buffers(const WarpSmem<FAST, CAP>& sm, int k, int K, bool has, const RayState& r,
                                             const RenderArgs& a, int rgb_base, const float* roff,
-                                            float* sig, float3* C, float* gC, int nw, int lane, WarpStats& ws) {
+                                            SlabBuf<FAST, GDOT>& sb, int nw, int lane, WarpStats& ws) {
     int nh = 0;
+    SlabPoints sp;
+    if constexpr (!FAST) {
+        f2 t[kPairs];
+        parity_times(r.tb, a.rnd_sample, roff, t);
+        sp.set(r, t, a.neg_zero);
+    }
 #pragma unroll 1
     for (int w = 0; w < nw; ++w) {
         unsigned mw = sm.smask[k / WarpSmem<FAST, CAP>::MB][w];
@@ -864,7 +936,7 @@ __device__ __forceinline__ int slab_buffers(const WarpSmem<FAST, CAP>& sm, int k
             float3 r0 = f3(rec.r0.x, rec.r0.y, rec.r0.z), r1 = f3(rec.r1.x, rec.r1.y, rec.r1.z),
                    r2 = f3(rec.r2.x, rec.r2.y, rec.r2.z);
             ++nh;
-            if (FAST) {
+            if constexpr (FAST) {
                 // log2(dens * w_i) = log2(dens) - q_i log2(e) / 2, q_i quadratic in the sample index
                 float3 v0 = (r.o + r.d * r.tb) - mu;
                 float3 vb = r.d * kDt;
@@ -880,54 +952,101 @@ __device__ __forceinline__ int slab_buffers(const WarpSmem<FAST, CAP>& sm, int k
                     float e = fmaf(fi, fmaf(fi, Cq, B2), A);
                     if (e > kLog2SigThr) {
                         float dw = ex2_approx(e);
-                        sig[i] += dw;
-                        if (GDOT) gC[i] = fmaf(gcol, dw, gC[i]);
-                        else C[i] = C[i] + col * dw;
+                        sb.sig[i] += dw;
+                        if constexpr (GDOT) sb.gC[i] = fmaf(gcol, dw, sb.gC[i]);
+                        else sb.C[i] = sb.C[i] + col * dw;
                     }
-                }
-            } else if (!GDOT && a.infer) {
-                // Inference programs (cuda_test/gaussians_aabb.cu:282-295, :501-515): the samples step
-                // through the scaled conic space from the slab start, m_{i+1} = m_i + dt * M d, and
-                // weight * density multiplies the colour.  Reference operation order.
-                const LeafIS is = load_is(a.is_rec, leaf);
-                const float kf = is.u.w;   // sqrt(log(ratio^2)) of the Gaussian
-                const float3 U = f3(is.u.x, is.u.y, is.u.z), V = f3(is.v.x, is.v.y, is.v.z),
-                             W = f3(is.w.x, is.w.y, is.w.z);
-                const float3 xg = f3(__fsub_rn(__fadd_rn(r.o.x, __fmul_rn(r.tb, r.d.x)), mu.x),
-                                     __fsub_rn(__fadd_rn(r.o.y, __fmul_rn(r.tb, r.d.y)), mu.y),
-                                     __fsub_rn(__fadd_rn(r.o.z, __fmul_rn(r.tb, r.d.z)), mu.z));
-                float3 m = f3(__fmul_rn(dot_rn(U, xg), kf), __fmul_rn(dot_rn(V, xg), kf),
-                              __fmul_rn(dot_rn(W, xg), kf));
-                const float3 mdt = f3(__fmul_rn(__fmul_rn(dot_rn(U, r.d), kf), kDt),
-                                      __fmul_rn(__fmul_rn(dot_rn(V, r.d), kf), kDt),
-                                      __fmul_rn(__fmul_rn(dot_rn(W, r.d), kf), kDt));
-#pragma unroll
-                for (int i = 0; i < kBuf; ++i) {
-                    const float power = __fmul_rn(-0.5f, dot_rn(m, m));
-                    float w = expf(power);
-                    float wd = __fmul_rn(w, dn);
-                    if (fabsf(wd - kSigThr) < 4e-8f) wd = __fmul_rn((float)exp((double)power), dn);
-                    if (wd > kSigThr) {
-                        sig[i] = __fadd_rn(sig[i], wd);
-                        C[i] = f3(__fadd_rn(C[i].x, __fmul_rn(col4.x, wd)), __fadd_rn(C[i].y, __fmul_rn(col4.y, wd)),
-                                  __fadd_rn(C[i].z, __fmul_rn(col4.z, wd)));
-                    }
-                    m = f3(__fadd_rn(m.x, mdt.x), __fadd_rn(m.y, mdt.y), __fadd_rn(m.z, mdt.z));
                 }
             } else {
-                float ws[kBuf];
-                const unsigned in_mask = parity_weights(r, a.rnd_sample, roff, mu, r0, r1, r2, dn, ws);
+                f2 w[kPairs];                  // weights, or density * weight (inference)
+                const f2 dn2 = dup2(dn);
+                const bool infer = !GDOT && a.infer;
+                if (infer) {
+                    // Inference programs (cuda_test/gaussians_aabb.cu:282-295, :501-515): the samples step
+                    // through the scaled conic space from the slab start, m_{i+1} = m_i + dt * M d, and
+                    // weight * density multiplies the colour.  Reference operation order.
+                    const LeafIS is = load_is(a.is_rec, leaf);
+                    const float kf = is.u.w;   // sqrt(log(ratio^2)) of the Gaussian
+                    const float3 U = f3(is.u.x, is.u.y, is.u.z), V = f3(is.v.x, is.v.y, is.v.z),
+                                 W = f3(is.w.x, is.w.y, is.w.z);
+                    const float3 xg = f3(__fsub_rn(__fadd_rn(r.o.x, __fmul_rn(r.tb, r.d.x)), mu.x),
+                                         __fsub_rn(__fadd_rn(r.o.y, __fmul_rn(r.tb, r.d.y)), mu.y),
+                                         __fsub_rn(__fadd_rn(r.o.z, __fmul_rn(r.tb, r.d.z)), mu.z));
+                    float3 m = f3(__fmul_rn(dot_rn(U, xg), kf), __fmul_rn(dot_rn(V, xg), kf),
+                                  __fmul_rn(dot_rn(W, xg), kf));
+                    const float3 mdt = f3(__fmul_rn(__fmul_rn(dot_rn(U, r.d), kf), kDt),
+                                          __fmul_rn(__fmul_rn(dot_rn(V, r.d), kf), kDt),
+                                          __fmul_rn(__fmul_rn(dot_rn(W, r.d), kf), kDt));
+                    float near = INFINITY;
+                    f2 q[kPairs];
 #pragma unroll
-                for (int i = 0; i < kBuf; ++i) {
-                    const float w = ws[i];
-                    if ((in_mask >> i) & 1u) {
-                        sig[i] = __fadd_rn(sig[i], __fmul_rn(dn, w));
-                        if (GDOT) {
-                            gC[i] += (r.g.x * col4.x + r.g.y * col4.y + r.g.z * col4.z) * (w * dn);
+                    for (int p = 0; p < kPairs; ++p) {
+                        const float3 n = f3(__fadd_rn(m.x, mdt.x), __fadd_rn(m.y, mdt.y), __fadd_rn(m.z, mdt.z));
+                        const f2 mx = pk(m.x, n.x), my = pk(m.y, n.y), mz = pk(m.z, n.z);
+                        q[p] = mul2(dup2(-0.5f), dot2_rn(mx, my, mz, mx, my, mz, a.neg_zero));
+                        w[p] = mul2_rn(pk(expf(lo2(q[p])), expf(hi2(q[p]))), dn2, a.neg_zero);
+                        const f2 off = add2(w[p], dup2(-kSigThr));
+                        near = fminf(near, fminf(fabsf(lo2(off)), fabsf(hi2(off))));
+                        m = f3(__fadd_rn(n.x, mdt.x), __fadd_rn(n.y, mdt.y), __fadd_rn(n.z, mdt.z));
+                    }
+                    if (near < 4e-8f) {
+#pragma unroll
+                        for (int p = 0; p < kPairs; ++p) {
+                            if (fabsf(lo2(w[p]) - kSigThr) < 4e-8f)
+                                w[p] = pk(__fmul_rn(exp_exact(lo2(q[p])), dn), hi2(w[p]));
+                            if (fabsf(hi2(w[p]) - kSigThr) < 4e-8f)
+                                w[p] = pk(lo2(w[p]), __fmul_rn(exp_exact(hi2(q[p])), dn));
+                        }
+                    }
+#pragma unroll
+                    for (int p = 0; p < kPairs; ++p)
+                        w[p] = pk(lo2(w[p]) > kSigThr ? lo2(w[p]) : 0.f, hi2(w[p]) > kSigThr ? hi2(w[p]) : 0.f);
+                } else {
+                    parity_weights(sp, rec, w, a.neg_zero);
+                }
+                if constexpr (GDOT) {
+                    const float ngcol = -(r.g.x * col4.x + r.g.y * col4.y + r.g.z * col4.z);
+                    if (fabsf(ngcol) < INFINITY) {
+#pragma unroll
+                        for (int p = 0; p < kPairs; ++p) {
+                            sb.sig[p] = add2(sb.sig[p], mul2_rn(dn2, w[p], a.neg_zero));
+                            sb.ng[p] = fma2(dup2(ngcol), mul2(w[p], dn2), sb.ng[p]);
+                        }
+                    } else {
+                        // not finite: 0 * inf must not reach the samples under the threshold
+#pragma unroll
+                        for (int p = 0; p < kPairs; ++p) {
+                            const f2 dw = mul2_rn(dn2, w[p], a.neg_zero);
+                            sb.sig[p] = add2(sb.sig[p], dw);
+#pragma unroll
+                            for (int h = 0; h < 2; ++h)
+                                if (half2(dw, h) > 0.f)
+                                    sb.ng[p] = with_half2(sb.ng[p], h, fmaf(ngcol, half2(dw, h), half2(sb.ng[p], h)));
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int p = 0; p < kPairs; ++p) {
+                        // inference: colour * (weight * density); training: (colour * weight) * density
+                        const f2 dw = infer ? w[p] : mul2_rn(dn2, w[p], a.neg_zero);
+                        const f2 one = infer ? dup2(1.f) : dn2;
+                        sb.sig[p] = add2(sb.sig[p], dw);
+                        const f2 cx = mul2_rn(mul2(dup2(col4.x), w[p]), one, a.neg_zero),
+                                 cy = mul2_rn(mul2(dup2(col4.y), w[p]), one, a.neg_zero),
+                                 cz = mul2_rn(mul2(dup2(col4.z), w[p]), one, a.neg_zero);
+                        if (col4.w == 0.f) {
+                            sb.cx[p] = add2(sb.cx[p], cx);
+                            sb.cy[p] = add2(sb.cy[p], cy);
+                            sb.cz[p] = add2(sb.cz[p], cz);
                         } else {
-                            C[i] = f3(__fadd_rn(C[i].x, __fmul_rn(__fmul_rn(col4.x, w), dn)),
-                                      __fadd_rn(C[i].y, __fmul_rn(__fmul_rn(col4.y, w), dn)),
-                                      __fadd_rn(C[i].z, __fmul_rn(__fmul_rn(col4.z, w), dn)));
+                            // a colour that is not finite
+#pragma unroll
+                            for (int h = 0; h < 2; ++h)
+                                if (half2(dw, h) > 0.f) {
+                                    sb.cx[p] = with_half2(sb.cx[p], h, __fadd_rn(half2(sb.cx[p], h), half2(cx, h)));
+                                    sb.cy[p] = with_half2(sb.cy[p], h, __fadd_rn(half2(sb.cy[p], h), half2(cy, h)));
+                                    sb.cz[p] = with_half2(sb.cz[p], h, __fadd_rn(half2(sb.cz[p], h), half2(cz, h)));
+                                }
                         }
                     }
                 }
@@ -937,48 +1056,77 @@ __device__ __forceinline__ int slab_buffers(const WarpSmem<FAST, CAP>& sm, int k
     return nh;
 }
 
-template <bool FAST>
-__device__ __forceinline__ float exp_neg(float x) {
-    return FAST ? ex2_approx(-x * 1.4426950408889634f) : (float)exp(-(double)x);
-}
+__device__ __forceinline__ float exp_neg_fast(float x) { return ex2_approx(-x * 1.4426950408889634f); }
 
-__device__ __forceinline__ bool any_density(const float* sig) {
-    bool any = false;
+// exp(-sig dt) of a slab's samples, correctly rounded (parity arithmetic: one ulp of the exponential is
+// ~1e-5 of the opacity, enough to move T > 0.003).  For x = sig dt <= 1/4 the sum 1 - x + x^2 / 2 -
+// x^3 / 6 + ... (the Taylor series to x^8) is carried as t + tail with |tail| under half an ulp of t
+// or so: 1 - x and its rounding error, x^2 / 2 and the error of the square are exact, and the rest is
+// x^3 P(x), whose rounding stays under d = 5e-8 x^3 + 2^-43.  Rounding t + tail gives the correctly
+// rounded value unless the remainder comes within d of half an ulp, 2^-25 (results are in [1/2, 1)):
+// then, and above 1/4, double precision decides.  Checked against it for every float in [2e-4, 1/4]:
+// the largest error is 0.73 d, one argument in a thousand is handed on.  14 packed FP32 issue slots
+// per sample instead of a double-precision exp().
+__device__ __forceinline__ void exp_neg_slab(const f2* sig, f2* ex, f2 nz) {
+    float worst = 0.f, top = 0.f;
 #pragma unroll
-    for (int i = 0; i < kBuf; ++i) any |= sig[i] > 0.f;
-    return any;
+    for (int p = 0; p < kPairs; ++p) {
+        const f2 x = mul2_rn(sig[p], dup2(kDt), nz), m1 = dup2(-1.f), one = dup2(1.f);
+        const f2 s = fma2(x, m1, one), nx = mul2_rn(x, m1, nz);
+        const f2 sl = add2(fma2(s, m1, one), nx);
+        const f2 x2 = mul2_rn(x, x, nz), x2l = fma2(x, x, mul2_rn(x2, m1, nz)), h = mul2_rn(x2, dup2(0.5f), nz);
+        f2 P = fma2(x, dup2(1.f / 40320.f), dup2(-1.f / 5040.f));
+        P = fma2(x, P, dup2(1.f / 720.f));
+        P = fma2(x, P, dup2(-1.f / 120.f));
+        P = fma2(x, P, dup2(1.f / 24.f));
+        P = fma2(x, P, dup2(-1.f / 6.f));
+        const f2 x3 = mul2_rn(x2, x, nz), t = add2(s, h);
+        const f2 e = add2(fma2(t, m1, s), h);
+        const f2 tail = fma2(x3, P, add2(fma2(x2l, dup2(0.5f), sl), e));
+        const f2 r = add2(t, tail);
+        const f2 rest = add2(tail, fma2(r, m1, t));   // tail - (r - t)
+        const f2 d = fma2(x3, dup2(5e-8f), dup2(0x1p-43f));
+        worst = max3f(worst, fabsf(lo2(rest)) + lo2(d), fabsf(hi2(rest)) + hi2(d));
+        top = max3f(top, lo2(x), hi2(x));
+        ex[p] = r;
+    }
+    if (worst > 0x1p-25f || top > 0.25f) {
+#pragma unroll
+        for (int p = 0; p < kPairs; ++p)
+            ex[p] = pk(exp_exact(-__fmul_rn(lo2(sig[p]), kDt)), exp_exact(-__fmul_rn(hi2(sig[p]), kDt)));
+    }
 }
 
 // Alpha compositing of one slab's 8 samples (forward/gaussians_aabb.cu:500-519).  A slab whose
 // samples all fell under the threshold composites to exactly nothing (alpha = 1 - exp(0) = 0).
 template <bool FAST>
-__device__ __forceinline__ void composite(RayState& r, const float* sig, const float3* C) {
-    if (!any_density(sig)) return;
-    float ex[kBuf];
-    if (!FAST) {
-        // the eight exponentials are independent of the transmittance chain: evaluate them first
+__device__ __forceinline__ void composite(RayState& r, const SlabBuf<FAST, false>& sb, f2 nz) {
+    if (!sb.any_density()) return;
+    if constexpr (FAST) {
 #pragma unroll
-        for (int i = 0; i < kBuf; ++i) ex[i] = exp_neg<false>(__fmul_rn(sig[i], kDt));
-    }
-#pragma unroll
-    for (int i = 0; i < kBuf; ++i) {
-        if (FAST) {
+        for (int i = 0; i < kBuf; ++i) {
             // C[i] is zero wherever sig[i] is (both sum the same above-threshold samples)
-            float alpha = 1.f - exp_neg<true>(sig[i] * kDt);
-            float s = sig[i] > 0.f ? __fdividef(r.T * alpha, sig[i]) : 0.f;
-            r.C = r.C + C[i] * s;
+            float alpha = 1.f - exp_neg_fast(sb.sig[i] * kDt);
+            float s = sb.sig[i] > 0.f ? __fdividef(r.T * alpha, sb.sig[i]) : 0.f;
+            r.C = r.C + sb.C[i] * s;
             r.T *= 1.f - alpha;
-        } else {
-            float alpha = __fsub_rn(1.f, ex[i]);
-            float3 c = C[i];
-            if (sig[i] > 0.f) {
-                float inv = __fdiv_rn(1.f, sig[i]);
-                c = f3(__fmul_rn(c.x, inv), __fmul_rn(c.y, inv), __fmul_rn(c.z, inv));
-            }
-            float ta = __fmul_rn(r.T, alpha);
-            r.C = f3(__fadd_rn(r.C.x, __fmul_rn(c.x, ta)), __fadd_rn(r.C.y, __fmul_rn(c.y, ta)),
-                     __fadd_rn(r.C.z, __fmul_rn(c.z, ta)));
-            r.T = __fmul_rn(r.T, __fsub_rn(1.f, alpha));
+        }
+    } else {
+        // the exponentials are independent of the transmittance chain: evaluate them first
+        f2 ex[kPairs];
+        exp_neg_slab(sb.sig, ex, nz);
+#pragma unroll
+        for (int p = 0; p < kPairs; ++p) {
+            const f2 alpha = fma2(ex[p], dup2(-1.f), dup2(1.f)), om = fma2(alpha, dup2(-1.f), dup2(1.f));
+            const float s0 = lo2(sb.sig[p]), s1 = hi2(sb.sig[p]);
+            const f2 inv = pk(s0 > 0.f ? __frcp_rn(s0) : 0.f, s1 > 0.f ? __frcp_rn(s1) : 0.f);   // colours are 0 there
+            const float T1 = __fmul_rn(r.T, lo2(om));
+            const f2 ta = mul2_rn(pk(r.T, T1), alpha, nz);
+            const f2 cx = mul2_rn(mul2(sb.cx[p], inv), ta, nz), cy = mul2_rn(mul2(sb.cy[p], inv), ta, nz),
+                     cz = mul2_rn(mul2(sb.cz[p], inv), ta, nz);
+            r.C = f3(__fadd_rn(__fadd_rn(r.C.x, lo2(cx)), hi2(cx)), __fadd_rn(__fadd_rn(r.C.y, lo2(cy)), hi2(cy)),
+                     __fadd_rn(__fadd_rn(r.C.z, lo2(cz)), hi2(cz)));
+            r.T = __fmul_rn(T1, hi2(om));
         }
     }
 }
@@ -1028,13 +1176,31 @@ __device__ __forceinline__ float transpose_reduce16(float* v, int lane) {
     return v[0];
 }
 
+// Compositing adjoint scalars of a slab's samples (slab_adjoint_scalars).
+template <bool FAST>
+struct AdjBuf {
+    float H[kBuf], F[kBuf];
+};
+template <>
+struct AdjBuf<false> {
+    f2 H[kPairs], F[kPairs];
+};
+
 // Adjoint of slab k for all list entries: per-lane gradient of each hit Gaussian, warp reduction,
 // one atomic per value.  Value order: ddens, S1.xyz, M2 (xx yy zz xy xz yz), 0, drgb.xyz.
 template <bool FAST, int CAP, bool DIAG>
 __device__ __forceinline__ void slab_adjoint(const WarpSmem<FAST, CAP>& sm, int k, int K, bool has, const RayState& r,
                                              const RenderArgs& a, int rgb_base, const float* roff,
-                                             const float* H, const float* F, int nw, int lane,
+                                             const AdjBuf<FAST>& ad, int nw, int lane,
                                              WarpStats& ws, int view) {
+    SlabPoints sp;
+    f2 xt[kPairs];   // parity: sample times from the slab's start
+    if constexpr (!FAST) {
+        parity_times(r.tb, a.rnd_sample, roff, xt);
+        sp.set(r, xt, a.neg_zero);
+#pragma unroll
+        for (int p = 0; p < kPairs; ++p) xt[p] = add2(xt[p], dup2(-r.tb));
+    }
     const int vid = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
 #pragma unroll 1
     for (int w = 0; w < nw; ++w) {
@@ -1071,7 +1237,7 @@ __device__ __forceinline__ void slab_adjoint(const WarpSmem<FAST, CAP>& sm, int 
             const float3 v0 = (r.o + r.d * r.tb) - mu;
             const float3 vb = FAST ? r.d * kDt : r.d;
             float U0 = 0.f, U1 = 0.f, U2 = 0.f;
-            if (FAST) {
+            if constexpr (FAST) {
                 // dw_i = dens * w_i in the exponent domain (as in the forward); accumulates
                 // sum dw F, sum dw h and the moments of u = dw h, then divides by dens once
                 const float3 m0 = f3(dot3(r0, v0), dot3(r1, v0), dot3(r2, v0));
@@ -1084,8 +1250,8 @@ __device__ __forceinline__ void slab_adjoint(const WarpSmem<FAST, CAP>& sm, int 
                     float e = fmaf(fi, fmaf(fi, Cq, B2), A);
                     if (e > kLog2SigThr) {
                         float dw = ex2_approx(e);
-                        float u = fmaf(F[i], gcol, H[i]) * dw;
-                        gc = fmaf(dw, F[i], gc);
+                        float u = fmaf(ad.F[i], gcol, ad.H[i]) * dw;
+                        gc = fmaf(dw, ad.F[i], gc);
                         U0 += u;
                         U1 = fmaf(fi, u, U1);
                         U2 = fmaf(fi * fi, u, U2);
@@ -1093,23 +1259,38 @@ __device__ __forceinline__ void slab_adjoint(const WarpSmem<FAST, CAP>& sm, int 
                 }
                 dd = (U0 != 0.f) ? U0 * rec.r2.w : 0.f;                   // r2.w = 1 / dens
             } else {
-                float ws[kBuf];
-                const unsigned in_mask = parity_weights(r, a.rnd_sample, roff, mu, r0, r1, r2, dn, ws);
+                f2 w[kPairs];
+                parity_weights(sp, rec, w, a.neg_zero);
+                f2 gc2 = 0ull, s0 = 0ull, s1 = 0ull, s2 = 0ull;
 #pragma unroll
-                for (int i = 0; i < kBuf; ++i) {
-                    if ((in_mask >> i) & 1u) {
-                        const float wt = ws[i];
-                        const float t = parity_time(r.tb, i, a.rnd_sample, roff);
-                        float h = fmaf(F[i], gcol, H[i]);
-                        gc += wt * F[i];
-                        dd += wt * h;
-                        float u = h * wt;
-                        float x = t - r.tb;
-                        U0 += u;
-                        U1 += x * u;
-                        U2 += x * x * u;
+                for (int p = 0; p < kPairs; ++p) {
+                    const f2 u = mul2(fma2(ad.F[p], dup2(gcol), ad.H[p]), w[p]);
+                    gc2 = fma2(w[p], ad.F[p], gc2);
+                    s0 = add2(s0, u);
+                    s1 = fma2(xt[p], u, s1);
+                    s2 = fma2(mul2(xt[p], xt[p]), u, s2);
+                }
+                gc = lo2(gc2) + hi2(gc2);
+                U0 = lo2(s0) + hi2(s0);
+                U1 = lo2(s1) + hi2(s1);
+                U2 = lo2(s2) + hi2(s2);
+                if (!(fabsf(U0) + fabsf(U1) + fabsf(U2) + fabsf(gc) < INFINITY)) {
+                    // not finite: take in only the samples above the threshold
+                    gc = U0 = U1 = U2 = 0.f;
+#pragma unroll
+                    for (int i = 0; i < kBuf; ++i) {
+                        const float wt = half2(w[i >> 1], i & 1), x = half2(xt[i >> 1], i & 1);
+                        if (wt > 0.f) {
+                            const float Fi = half2(ad.F[i >> 1], i & 1);
+                            const float u = fmaf(Fi, gcol, half2(ad.H[i >> 1], i & 1)) * wt;
+                            gc += wt * Fi;
+                            U0 += u;
+                            U1 += x * u;
+                            U2 += x * x * u;
+                        }
                     }
                 }
+                dd = U0;
                 gc *= dn;
                 U0 *= dn; U1 *= dn; U2 *= dn;
             }
@@ -1159,33 +1340,48 @@ __device__ __forceinline__ void slab_adjoint(const WarpSmem<FAST, CAP>& sm, int 
 // E = dt (T gc - g.R), H = E - F gc, and g.R drops by gc T alpha per sample.
 // Returns H and F; advances T and g.R over the slab.
 template <bool FAST>
-__device__ __forceinline__ void slab_adjoint_scalars(const RayState& r, const float* sig, const float* gC, float* H,
-                                                     float* F, float& Ta, float& gRa) {
+__device__ __forceinline__ void slab_adjoint_scalars(const RayState& r, const SlabBuf<FAST, true>& sb, AdjBuf<FAST>& ad,
+                                                     float& Ta, float& gRa, f2 nz) {
     Ta = r.T;
     gRa = r.gR;
-    float ex[kBuf];
-    if (!FAST) {
+    if constexpr (FAST) {
 #pragma unroll
-        for (int i = 0; i < kBuf; ++i) ex[i] = exp_neg<false>(__fmul_rn(sig[i], kDt));
-    }
+        for (int i = 0; i < kBuf; ++i) {
+            const float cd = sb.sig[i];
+            float inv = 0.f;
+            if (cd > 0.f) inv = __fdividef(1.f, cd);
+            const float gc = sb.gC[i] * inv;
+            const float alpha = 1.f - exp_neg_fast(cd * kDt);
+            const float ta = Ta * alpha;
+            ad.F[i] = ta * inv;
+            ad.H[i] = kDt * (Ta * gc - gRa) - ad.F[i] * gc;
+            gRa -= gc * ta;
+            Ta = Ta * (1.f - alpha);
+        }
+    } else {
+        f2 ex[kPairs];
+        exp_neg_slab(sb.sig, ex, nz);
 #pragma unroll
-    for (int i = 0; i < kBuf; ++i) {
-        const float cd = sig[i];
-        float inv = 0.f;
-        if (cd > 0.f) inv = FAST ? __fdividef(1.f, cd) : 1.f / cd;
-        const float gc = gC[i] * inv;
-        const float alpha = FAST ? 1.f - exp_neg<true>(cd * kDt) : __fsub_rn(1.f, ex[i]);
-        const float ta = Ta * alpha;
-        F[i] = ta * inv;
-        H[i] = kDt * (Ta * gc - gRa) - F[i] * gc;
-        gRa -= gc * ta;
-        Ta = FAST ? Ta * (1.f - alpha) : __fmul_rn(Ta, __fsub_rn(1.f, alpha));
+        for (int p = 0; p < kPairs; ++p) {
+            const f2 alpha = fma2(ex[p], dup2(-1.f), dup2(1.f)), om = fma2(alpha, dup2(-1.f), dup2(1.f));
+            const float s0 = lo2(sb.sig[p]), s1 = hi2(sb.sig[p]);
+            const f2 inv = pk(s0 > 0.f ? __frcp_rn(s0) : 0.f, s1 > 0.f ? __frcp_rn(s1) : 0.f);
+            const float T1 = __fmul_rn(Ta, lo2(om));
+            const f2 T2 = pk(Ta, T1), ngc = mul2(sb.ng[p], inv), ta = mul2(T2, alpha);   // ngc = -g.C / sigma
+            ad.F[p] = mul2(ta, inv);
+            const float gR1 = fmaf(lo2(ngc), lo2(ta), gRa);
+            ad.H[p] = fma2(ad.F[p], ngc, mul2(fma2(T2, ngc, pk(gRa, gR1)), dup2(-kDt)));
+            gRa = fmaf(hi2(ngc), hi2(ta), gR1);
+            Ta = __fmul_rn(T1, hi2(om));
+        }
     }
 }
 
-// Resident blocks per SM each kernel is compiled for (0: the compiler's choice).  The defaults
+// Resident blocks per SM each kernel is compiled for (0: the compiler's choice).  The fast defaults
 // fit the shared memory of the 64-entry tuning (256-entry fast lists) and were measured best on
-// 1M Gaussians x 16 views.
+// 1M Gaussians x 16 views.  The parity kernels want registers for the slab's points and sums rather
+// than warps (300k-Gaussian object, forward / backward: 12.8 / 24.7 ms at 4 blocks, 128 registers and
+// 400 B of spills; 12.3 / 22.5 at 3; 13.4 / 22.2 at 2, without spills).
 #ifndef RG_FAST_FWD_MIN_BLOCKS
 #define RG_FAST_FWD_MIN_BLOCKS 7
 #endif
@@ -1193,10 +1389,10 @@ __device__ __forceinline__ void slab_adjoint_scalars(const RayState& r, const fl
 #define RG_FAST_BWD_MIN_BLOCKS 7
 #endif
 #ifndef RG_PAR_FWD_MIN_BLOCKS
-#define RG_PAR_FWD_MIN_BLOCKS 4
+#define RG_PAR_FWD_MIN_BLOCKS 3
 #endif
 #ifndef RG_PAR_BWD_MIN_BLOCKS
-#define RG_PAR_BWD_MIN_BLOCKS 4
+#define RG_PAR_BWD_MIN_BLOCKS 2
 #endif
 template <bool BWD, bool FAST>
 constexpr int min_blocks() {
@@ -1382,32 +1578,26 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                     if (DIAG) ++ws.slab_steps;
                     float roff[kBuf];
                     unsigned seed_next = slab_offsets(a.rnd_sample, r.seed, roff);
-                    float sig[kBuf];
-                    float3 Cb[BWD ? 1 : kBuf];
-                    float gC[BWD ? kBuf : 1];
-#pragma unroll
-                    for (int i = 0; i < kBuf; ++i) {
-                        sig[i] = 0.f;
-                        if (BWD) gC[i] = 0.f;
-                        else Cb[i] = f3(0.f, 0.f, 0.f);
-                    }
-                    int nh = slab_buffers<FAST, CAP, BWD, DIAG>(sm, k, K, has, r, a, rgb_base, roff, sig, Cb, gC,
-                                                          nwords(count), lane, ws);
+                    SlabBuf<FAST, BWD> sb;
+                    sb.clear();
+                    int nh = slab_buffers<FAST, CAP, BWD, DIAG>(sm, k, K, has, r, a, rgb_base, roff, sb, nwords(count),
+                                                                lane, ws);
                     if (has) {
                         ++slabs_acc;
                         hits_acc += (!BWD && a.counts) ? min(nh, a.max_prim_slice) : nh;
                         if (nh > a.max_prim_slice) atomicAdd(&a.st->slab_cap_exceeded, 1ull);
                     }
-                    if (!BWD) {
+                    if constexpr (!BWD) {
                         if (has && nh > 0) {
-                            composite<FAST>(r, sig, Cb);
+                            composite<FAST>(r, sb, a.neg_zero);
                             r.seed = seed_next;
                         }
                     } else {
-                        float H[kBuf], F[kBuf], Ta, gRa;
-                        slab_adjoint_scalars<FAST>(r, sig, gC, H, F, Ta, gRa);
-                        bool act = has && nh > 0 && any_density(sig);
-                        slab_adjoint<FAST, CAP, DIAG>(sm, k, K, act, r, a, rgb_base, roff, H, F, nwords(count), lane, ws,
+                        AdjBuf<FAST> ad;
+                        float Ta, gRa;
+                        slab_adjoint_scalars<FAST>(r, sb, ad, Ta, gRa, a.neg_zero);
+                        bool act = has && nh > 0 && sb.any_density();
+                        slab_adjoint<FAST, CAP, DIAG>(sm, k, K, act, r, a, rgb_base, roff, ad, nwords(count), lane, ws,
                                                       view);
                         if (has && nh > 0) {
                             r.T = Ta;
@@ -1427,45 +1617,39 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                 bool has = on && nv > 0 && r.T > kTeps;
                 float roff[kBuf];
                 unsigned seed_next = slab_offsets(a.rnd_sample, r.seed, roff);
-                float sig[kBuf];
-                float3 Cb[BWD ? 1 : kBuf];
-                float gC[BWD ? kBuf : 1];
-#pragma unroll
-                for (int i = 0; i < kBuf; ++i) {
-                    sig[i] = 0.f;
-                    if (BWD) gC[i] = 0.f;
-                    else Cb[i] = f3(0.f, 0.f, 0.f);
-                }
-                int nh = slab_buffers<FAST, CAP, BWD, DIAG>(sm, 0, 1, has, r, a, rgb_base, roff, sig, Cb, gC, nwords(count),
-                                                      lane, ws);
+                SlabBuf<FAST, BWD> sb;
+                sb.clear();
+                int nh = slab_buffers<FAST, CAP, BWD, DIAG>(sm, 0, 1, has, r, a, rgb_base, roff, sb, nwords(count), lane,
+                                                            ws);
                 bool more = ovf;
                 while (more) {
                     int cursor = sm.ids[count - 1];
                     __syncwarp();
                     if (lane == 0) atomicAdd(&a.st->list_passes, 1ull);
                     count = traverse<FAST, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, more, lane, ws, infer);
-                    nh += slab_buffers<FAST, CAP, BWD, DIAG>(sm, 0, 1, has, r, a, rgb_base, roff, sig, Cb, gC,
-                                                       nwords(count), lane, ws);
+                    nh += slab_buffers<FAST, CAP, BWD, DIAG>(sm, 0, 1, has, r, a, rgb_base, roff, sb, nwords(count), lane,
+                                                             ws);
                 }
                 if (has) {
                     ++slabs_acc;
                     hits_acc += (!BWD && a.counts) ? min(nh, a.max_prim_slice) : nh;
                     if (nh > a.max_prim_slice) atomicAdd(&a.st->slab_cap_exceeded, 1ull);
                 }
-                if (!BWD) {
+                if constexpr (!BWD) {
                     if (has && nh > 0) {
-                        composite<FAST>(r, sig, Cb);
+                        composite<FAST>(r, sb, a.neg_zero);
                         r.seed = seed_next;
                     }
                 } else {
-                    float H[kBuf], F[kBuf], Ta, gRa;
-                    slab_adjoint_scalars<FAST>(r, sig, gC, H, F, Ta, gRa);
-                    bool act = has && nh > 0 && any_density(sig);
+                    AdjBuf<FAST> ad;
+                        float Ta, gRa;
+                    slab_adjoint_scalars<FAST>(r, sb, ad, Ta, gRa, a.neg_zero);
+                    bool act = has && nh > 0 && sb.any_density();
                     int cursor = -1;
                     bool more2 = true;
                     while (more2) {
                         count = traverse<FAST, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, more2, lane, ws, infer);
-                        slab_adjoint<FAST, CAP, DIAG>(sm, 0, 1, act, r, a, rgb_base, roff, H, F, nwords(count), lane, ws,
+                        slab_adjoint<FAST, CAP, DIAG>(sm, 0, 1, act, r, a, rgb_base, roff, ad, nwords(count), lane, ws,
                                                       view);
                         if (more2) cursor = sm.ids[count - 1];
                         __syncwarp();
@@ -1600,7 +1784,9 @@ int render_occupancy(bool backward, int mode, int cap) {
     return fast ? occ_cap<false, true>(cap) : occ_cap<false, false>(cap);
 }
 
-cudaError_t launch_render(bool backward, int mode, int cap, int grid, const RenderArgs& a, cudaStream_t s) {
+cudaError_t launch_render(bool backward, int mode, int cap, int grid, const RenderArgs& args, cudaStream_t s) {
+    RenderArgs a = args;
+    a.neg_zero = 0x8000000080000000ull;
     bool fast = (mode == RG_MODE_FAST) && a.rnd_sample == 0;
     if (backward) return fast ? launch_cap<true, true>(cap, grid, a, s) : launch_cap<true, false>(cap, grid, a, s);
     return fast ? launch_cap<false, true>(cap, grid, a, s) : launch_cap<false, false>(cap, grid, a, s);
