@@ -131,6 +131,7 @@ SIGNATURES = {
     "rg_create": (ctypes.c_int, [ctypes.POINTER(_P), ctypes.c_int]),
     "rg_destroy": (ctypes.c_int, [_P]),
     "rg_reserve": (ctypes.c_int, [_P, ctypes.c_int64, ctypes.c_int32, ctypes.c_int64]),
+    "rg_expect_rays": (ctypes.c_int, [_P, ctypes.c_int64]),
     "rg_set_tuning": (ctypes.c_int, [_P, ctypes.POINTER(rg_tuning)]),
     "rg_get_tuning": (ctypes.c_int, [_P, ctypes.POINTER(rg_tuning)]),
     "rg_ellipsoids_bbox": (ctypes.c_int, [_P, ctypes.POINTER(rg_gaussians), _P, _P, _P]),

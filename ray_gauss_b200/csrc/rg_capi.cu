@@ -39,6 +39,8 @@ struct rg_engine {
     const rg_camera* rec_cams = nullptr;
     int rec_n_cams = 0;
     rg_settings rec_settings{};
+    int rec_split = 1;               // the split of its tiles
+    long long expect_rays = 0;       // rays of the launches that follow (rg_expect_rays; 0: unknown)
     rg_tuning tuning{64, 0, 64, 1, 0};
     unsigned long long launches = 0;
     char last_err[256] = {0};
@@ -122,6 +124,12 @@ int ensure_views(rg_engine* e, int views) {
 constexpr long long kRecordWordsPerRay = 24;
 constexpr long long kRecordBaseWords = 4096;
 
+// Tiles that a record sized for `tiles` whole ones covers: four times as many split ones, which only
+// small launches have.
+long long record_heads(long long tiles, int split) {
+    return split > 1 ? std::max(tiles, std::min(4 * tiles, 1ll << 22)) : tiles;
+}
+
 // Hit-list record storage for launches of up to n_rays rays (tiles <= rays).
 int ensure_record(rg_engine* e, long long n_rays) {
     long long words = std::min(n_rays * kRecordWordsPerRay + kRecordBaseWords, (long long)0xfffffff0ll);
@@ -135,7 +143,7 @@ int ensure_record(rg_engine* e, long long n_rays) {
     }
     if (tiles > e->rec_tiles) {
         e->rec_tiles = 0;
-        if ((rc = grow(e, e->rec_tile, (size_t)tiles))) return rc;
+        if ((rc = grow(e, e->rec_tile, (size_t)record_heads(tiles, 4)))) return rc;
         e->rec_tiles = (int)tiles;
     }
     e->rec_valid = false;
@@ -190,9 +198,14 @@ int kernel_mode(const rg_settings* s) {
     return (s->mode == RG_MODE_FAST && s->rnd_sample == 0) ? RG_MODE_FAST : RG_MODE_PARITY;
 }
 
-int render_grid(rg_engine* e, bool bwd, int mode) {
+// Slabs of a ray side by side: more in launches of fewer rays.
+int launch_split(const rg_engine* e, const rg_settings* s) {
+    return rg::render_split(s->mode, s->rnd_sample, e->tuning.list_capacity, e->n_built, e->expect_rays);
+}
+
+int render_grid(rg_engine* e, bool bwd, int mode, int split) {
     int per_sm = e->tuning.blocks_per_sm;
-    int occ = rg::render_occupancy(bwd, mode, e->tuning.list_capacity);
+    int occ = rg::render_occupancy(bwd, mode, e->tuning.list_capacity, split);
     if (per_sm <= 0 || per_sm > occ) per_sm = occ > 0 ? occ : 1;
     return e->num_sms * per_sm;
 }
@@ -314,6 +327,12 @@ int rg_reserve(rg_engine* e, int64_t n, int32_t n_views, int64_t n_rays) {
     return RG_OK;
 }
 
+int rg_expect_rays(rg_engine* e, int64_t n_rays) {
+    if (!e || n_rays < 0) return RG_ERR_INVALID_ARG;
+    e->expect_rays = n_rays;
+    return RG_OK;
+}
+
 int rg_set_tuning(rg_engine* e, const rg_tuning* t) {
     if (!e || !t) return RG_ERR_INVALID_ARG;
     if (t->chunk_slabs < 0 || t->chunk_slabs > rg::kMaxChunk) return RG_ERR_INVALID_ARG;
@@ -414,7 +433,8 @@ int rg_launch_forward(rg_engine* e, const rg_camera* cams, int32_t n_cams, const
     if (e->n_built <= 0 || e->colors_views < n_cams) return RG_ERR_STATE;
     DeviceScope dev_scope;
     if ((rc = dev_scope.enter(e))) return rc;
-    RG_CUDA(rg::launch_setup_views(cams, n_cams, e->vt, e->work_counter, S(stream)), "setup views");
+    const int split = launch_split(e, s);
+    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->vt, e->work_counter, S(stream)), "setup views");
     rg::RenderArgs a;
     fill_args(e, cams, s, a);
     a.ray_colors = ray_colors;
@@ -427,16 +447,17 @@ int rg_launch_forward(rg_engine* e, const rg_camera* cams, int32_t n_cams, const
         a.rec_top = e->rec_top;
         a.rec_cap = e->rec_cap;
         a.rec_tile = e->rec_tile;
-        a.rec_tiles = e->rec_tiles;
+        a.rec_tiles = (int)record_heads(e->rec_tiles, split);
     }
-    int grid = render_grid(e, false, kernel_mode(s));
-    RG_CUDA(rg::launch_render(false, s->mode, e->tuning.list_capacity, grid, a, S(stream)), "render forward");
+    int grid = render_grid(e, false, kernel_mode(s), split);
+    RG_CUDA(rg::launch_render(false, s->mode, e->tuning.list_capacity, split, grid, a, S(stream)), "render forward");
     e->launches += 2;
     if (record) {
         e->rec_valid = true;
         e->rec_cams = cams;
         e->rec_n_cams = n_cams;
         e->rec_settings = *s;
+        e->rec_split = split;
     }
     return RG_OK;
 }
@@ -453,14 +474,15 @@ int rg_launch_inference(rg_engine* e, const rg_camera* cams, int32_t n_cams, con
     rg_settings si = *s;
     si.jitter = 0;
     si.rnd_sample = 0;
-    RG_CUDA(rg::launch_setup_views(cams, n_cams, e->vt, e->work_counter, S(stream)), "setup views");
+    const int split = launch_split(e, &si);
+    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->vt, e->work_counter, S(stream)), "setup views");
     rg::RenderArgs a;
     fill_args(e, cams, &si, a);
     a.ray_colors = ray_colors;
     a.infer = 1;
     a.counts = gaussians_per_ray;
-    int grid = render_grid(e, false, kernel_mode(&si));
-    RG_CUDA(rg::launch_render(false, si.mode, e->tuning.list_capacity, grid, a, S(stream)), "render inference");
+    int grid = render_grid(e, false, kernel_mode(&si), split);
+    RG_CUDA(rg::launch_render(false, si.mode, e->tuning.list_capacity, split, grid, a, S(stream)), "render inference");
     e->launches += 2;
     return RG_OK;
 }
@@ -488,7 +510,13 @@ int rg_launch_backward(rg_engine* e, const rg_camera* cams, int32_t n_cams, cons
     size_t N = (size_t)e->n_built;
     RG_CUDA(cudaMemsetAsync(e->gacc_geo, 0, sizeof(float4) * 3 * N, S(stream)), "zero grads");
     RG_CUDA(cudaMemsetAsync(e->gacc_rgb, 0, sizeof(float4) * N * (size_t)n_cams, S(stream)), "zero grads");
-    RG_CUDA(rg::launch_setup_views(cams, n_cams, e->vt, e->work_counter, S(stream)), "setup views");
+    // Replay the last forward's hit lists when nothing changed the engine state since that forward
+    // (bbox, BVH, colour and tuning calls invalidate the record) and this backward uses the same
+    // camera table, view count and settings: the chunk sequence is then the forward's, over its tiles.
+    const bool replay = e->rec_valid && e->tuning.record_hits == 1 && e->rec_cams == cams && e->rec_n_cams == n_cams &&
+                        std::memcmp(&e->rec_settings, s, sizeof(rg_settings)) == 0;
+    const int split = replay ? e->rec_split : launch_split(e, s);
+    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->vt, e->work_counter, S(stream)), "setup views");
     rg::RenderArgs a;
     fill_args(e, cams, s, a);
     a.ray_colors_in = ray_colors;
@@ -496,19 +524,15 @@ int rg_launch_backward(rg_engine* e, const rg_camera* cams, int32_t n_cams, cons
     a.gacc_geo = e->gacc_geo;
     a.gacc_rgb = e->gacc_rgb;
     a.n_views = n_cams;
-    // Replay the last forward's hit lists when nothing changed the engine state since that forward
-    // (bbox, BVH, colour and tuning calls invalidate the record) and this backward uses the same
-    // camera table, view count and settings: the chunk sequence is then the forward's.
-    if (e->rec_valid && e->tuning.record_hits == 1 && e->rec_cams == cams && e->rec_n_cams == n_cams &&
-        std::memcmp(&e->rec_settings, s, sizeof(rg_settings)) == 0) {
+    if (replay) {
         a.rec_arena = e->rec_arena;
         a.rec_cap = e->rec_cap;
         a.rec_tile = e->rec_tile;
-        a.rec_tiles = e->rec_tiles;
+        a.rec_tiles = (int)record_heads(e->rec_tiles, split);
         a.replay = 1;
     }
-    int grid = render_grid(e, true, kernel_mode(s));
-    RG_CUDA(rg::launch_render(true, s->mode, e->tuning.list_capacity, grid, a, S(stream)), "render backward");
+    int grid = render_grid(e, true, kernel_mode(s), split);
+    RG_CUDA(rg::launch_render(true, s->mode, e->tuning.list_capacity, split, grid, a, S(stream)), "render backward");
     RG_CUDA(rg::launch_moment_grads((int)N, e->bvh.leaf_rec, e->bvh.leaf_ext, e->gacc_geo, S(stream)), "moments");
     e->launches += 3;
     return RG_OK;

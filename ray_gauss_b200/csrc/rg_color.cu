@@ -42,7 +42,8 @@ __device__ __forceinline__ void sh_basis(float x, float y, float z, int deg, flo
     B[15] = cSH3[6] * x * (xx - 3.f * yy);
 }
 
-__global__ void k_setup_views(const rg_camera* __restrict__ cams, int n, ViewTable* vt, int* work_counter) {
+__global__ void k_setup_views(const rg_camera* __restrict__ cams, int n, int tile_w, int tile_h, ViewTable* vt,
+                              int* work_counter) {
     if (threadIdx.x != 0) return;
     int tiles = 0;
     long long rays = 0;
@@ -50,7 +51,7 @@ __global__ void k_setup_views(const rg_camera* __restrict__ cams, int n, ViewTab
         vt->tile_prefix[v] = tiles;
         vt->ray_prefix[v] = rays;
         int w = cams[v].width, h = cams[v].height;
-        tiles += ((w + kTileW - 1) / kTileW) * ((h + kTileH - 1) / kTileH);
+        tiles += ((w + tile_w - 1) / tile_w) * ((h + tile_h - 1) / tile_h);
         rays += (long long)w * h;
     }
     vt->tile_prefix[n] = tiles;
@@ -277,8 +278,9 @@ __global__ void __launch_bounds__(128) k_color_bwd_sg(long long n, const float* 
     out.positions[3 * g + 2] += dpos[2];
 }
 
-cudaError_t launch_setup_views(const rg_camera* cams, int n_cams, ViewTable* vt, int* work_counter, cudaStream_t s) {
-    k_setup_views<<<1, 32, 0, s>>>(cams, n_cams, vt, work_counter);
+cudaError_t launch_setup_views(const rg_camera* cams, int n_cams, int split, ViewTable* vt, int* work_counter,
+                               cudaStream_t s) {
+    k_setup_views<<<1, 32, 0, s>>>(cams, n_cams, tile_w(split), tile_h(split), vt, work_counter);
     return cudaGetLastError();
 }
 

@@ -19,6 +19,9 @@ constexpr float kSigThr = 0.1f;         // per-sample density threshold
 constexpr int kWarp = 32;
 constexpr int kTileW = 8;               // a warp renders an 8x4 pixel tile
 constexpr int kTileH = 4;
+// ... or, with two or four slabs of a ray side by side (split), a 4x4 or 4x2 one
+__host__ __device__ constexpr int tile_w(int split) { return split == 1 ? kTileW : 4; }
+__host__ __device__ constexpr int tile_h(int split) { return split == 4 ? 2 : 4; }
 constexpr int kMaxChunk = 255;          // slabs per traversal chunk (slab ranges are bytes)
 constexpr int kStack = 256;             // warp traversal stack depth (up to 31 pushes per wide node on the path)
 

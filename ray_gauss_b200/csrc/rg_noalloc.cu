@@ -183,7 +183,7 @@ extern "C" RG_API int rg_render_forward_noalloc(const rg_gaussians* g, const rg_
     if (rg::launch_prepass(g, rec, aabb, scene_ord, status, st) != cudaSuccess) return RG_ERR_CUDA;
     if (rg::launch_build(n, aabb, scene_ord, rec, g, bvh, st) != cudaSuccess) return RG_ERR_CUDA;
     if (rg::launch_color_forward(g, cams, n_cams, bvh.rank, rgb_leaf, nullptr, st) != cudaSuccess) return RG_ERR_CUDA;
-    if (rg::launch_setup_views(cams, n_cams, vt, work, st) != cudaSuccess) return RG_ERR_CUDA;
+    if (rg::launch_setup_views(cams, n_cams, 1, vt, work, st) != cudaSuccess) return RG_ERR_CUDA;
 
     rg::RenderArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -211,9 +211,9 @@ extern "C" RG_API int rg_render_forward_noalloc(const rg_gaussians* g, const rg_
     // random sample offsets run the parity kernel in either mode (launch_render picks it): size the
     // grid for the kernel that runs
     const int run_mode = (s->mode == RG_MODE_FAST && s->rnd_sample == 0) ? RG_MODE_FAST : RG_MODE_PARITY;
-    int per_sm = rg::render_occupancy(false, run_mode, cap);
+    int per_sm = rg::render_occupancy(false, run_mode, cap, 1);
     int grid = d->num_sms * (per_sm > 0 ? per_sm : 1);
-    if (rg::launch_render(false, s->mode, cap, grid, a, st) != cudaSuccess) return RG_ERR_CUDA;
+    if (rg::launch_render(false, s->mode, cap, 1, grid, a, st) != cudaSuccess) return RG_ERR_CUDA;
     return RG_OK;
 }
 

@@ -50,28 +50,49 @@ constexpr float kLog2SigThr = -3.3219280948873623f;   // log2(0.1): per-sample d
 constexpr float kInvSlab = 50.0f;          // 1 / 0.02
 constexpr int kExactChunk = 8;             // chunks up to this length use exact slab ranges
 constexpr int kCounters = 9;
+#ifndef RG_SPLIT_DIRECT_ATOMIC_LANES
+// ... and on split tiles, whose lanes are few rays' slabs: a Gaussian near the camera gets 10^5 and more of
+// them, and what is added alone to its large sum is lost below the sum's last bit (24 here: 3e-3 off on 4
+// views at 1920x1080; 4: as exact as whole tiles at the sizes that are split)
+#define RG_SPLIT_DIRECT_ATOMIC_LANES 4
+#endif
 #ifndef RG_DIRECT_ATOMIC_LANES
 #define RG_DIRECT_ATOMIC_LANES 24  // up to this many contributing lanes add with float4 atomics directly
 #endif               // per-warp counters: the WarpStats fields, hit pairs, slabs
 constexpr unsigned kNoRecord = 0xffffffffu;     // hit-list record: no (next) chunk record
 constexpr unsigned kRecordMulti = 0x80000000u;  // chunk consumed in several traversal passes
-constexpr unsigned kRecordFailed = 0xfffffffeu; // the tile's record did not fit the arena
+constexpr unsigned kRecordFailed = 0xfffffffeu; // the tile's last chunk did not fit the arena
 
-// Warp hit-list layout.  Parity arithmetic keeps, per entry and lane, the exact range of the
-// chunk's slabs the lane's interval covers (64 B per entry); the fast arithmetic keeps only the mask
-// of lanes whose interval overlaps the chunk (4 B per entry) and lets those lanes evaluate every
-// slab of the entry's union range (samples outside the lane's interval fall outside the threshold
-// ellipsoid and are masked out), which allows 4x longer lists and so 4x longer chunks in dense
-// regions.
-template <bool FAST, int CAP>
+// Rays and slabs of a warp.  SUB == 1: 32 rays (8x4 pixels), a slab at a time.  SUB == 2 or 4: 16 (4x4) or 8
+// (4x2) rays, the lanes SUB r .. SUB r + SUB - 1 holding ray r's slabs k .. k + SUB - 1.  Their sums are
+// independent; only the transmittance runs through them in turn, by the same operations as slab after
+// slab.  A Gaussian spans a few slabs, so a list entry is evaluated once for them all, by a tile that is
+// smaller: not many more evaluations in all, but a fraction of them in one tile's chain, and a launch
+// of few tiles lasts as long as its slowest one.  Leaves are tested SUB at a time.  render_split has the
+// lines between them.
+template <int SUB>
+struct TileShape {
+    static constexpr int rays = 32 / SUB;
+    static constexpr int w = tile_w(SUB), h = tile_h(SUB);
+    static_assert(w * h == rays, "a ray per pixel");
+    // the lanes of sub-slab 0
+    static constexpr unsigned lanes = SUB == 1 ? 0xffffffffu : SUB == 2 ? 0x55555555u : 0x11111111u;
+};
+
+// Warp hit-list layout.  Parity arithmetic keeps, per entry and ray, the exact range of the chunk's
+// slabs the ray's interval covers (2 B per entry and ray); the fast arithmetic keeps only the mask of
+// rays whose interval overlaps the chunk (4 B per entry) and lets those rays evaluate every slab of the
+// entry's union range (samples outside the ray's interval fall outside the threshold ellipsoid and
+// are masked out), which allows longer lists and so longer chunks in dense regions.
+template <bool FAST, int SUB, int CAP>
 struct WarpSmem {
-    static constexpr int MB = FAST ? 4 : 2;         // slabs per entry-mask block
-    static constexpr int NB = 64;                   // entry-mask blocks
-    static constexpr int KM = FAST ? 255 : 128;     // longest chunk (MB * NB, slab ranges are bytes)
+    static constexpr int MB = FAST || SUB > 1 ? 4 : 2;   // slabs per entry-mask block (a multiple of SUB)
+    static constexpr int NB = 64;                        // entry-mask blocks
+    static constexpr int KM = MB == 4 ? 255 : 128;       // longest chunk (MB * NB, slab ranges are bytes)
     int ids[CAP];
     unsigned urng[CAP];                              // union of the lanes' slab ranges: lo | hi << 16
-    unsigned lmask[FAST ? CAP : 1];                  // fast: lanes whose interval overlaps the chunk
-    unsigned short lrng[FAST ? 1 : CAP][32];         // parity: per lane lo | hi << 8 (lo > hi: no hit)
+    unsigned lmask[FAST ? CAP : 1];                  // fast: rays (sub-slab 0 lanes) whose interval overlaps the chunk
+    unsigned short lrng[FAST ? 1 : CAP][32 / SUB];   // parity: per ray lo | hi << 8 (lo > hi: no hit)
     unsigned smask[NB][CAP / 32];                    // entries whose union range meets block k / MB
     unsigned long long occ[4];                       // slabs holding any entry (union occupancy)
     __align__(16) float packet[24];                  // the chunk's ray packet (set_packet), read as float4
@@ -138,8 +159,8 @@ __device__ __forceinline__ void load_slot(const WideSlot* p, float3& lo, float3&
 // inside the leaf boxes' 1e-5 inflation, so the bound needs no slack of its own; a small one in t
 // covers the ends of the segments.  (A slack that grows with 1/|d| would stretch the packets of
 // rays nearly parallel to a coordinate plane over most of their length.)
-template <bool FAST, int CAP>
-__device__ __forceinline__ void set_packet(WarpSmem<FAST, CAP>& sm, const RayState& r, bool on, float seg_hi,
+template <bool FAST, int SUB, int CAP>
+__device__ __forceinline__ void set_packet(WarpSmem<FAST, SUB, CAP>& sm, const RayState& r, bool on, float seg_hi,
                                            int lane) {
     float dmin[3], dmax[3];
     const float dv[3] = {r.d.x, r.d.y, r.d.z};
@@ -201,8 +222,8 @@ __device__ __forceinline__ bool packet_hit(const float* F, float3 lo, float3 hi)
 // The tile's ray directions before normalisation, w + u dx + v dy, as centre + s * cone_u + t * cone_v
 // with s and t in [-1, 1]: {centre.xyz, cone_u.x}, {cone_u.yz, cone_v.xy}, {cone_v.z,
 // smallest and largest length, -}.
-template <bool FAST, int CAP>
-__device__ __forceinline__ void set_cone(WarpSmem<FAST, CAP>& sm, const rg_camera& cam, float dx, float dy, bool valid,
+template <bool FAST, int SUB, int CAP>
+__device__ __forceinline__ void set_cone(WarpSmem<FAST, SUB, CAP>& sm, const rg_camera& cam, float dx, float dy, bool valid,
                                          int lane) {
     const float x0 = ord2f(__reduce_min_sync(kFull, valid ? f2ord(dx) : 0x7fffffff));
     const float x1 = ord2f(__reduce_max_sync(kFull, valid ? f2ord(dx) : (int)0x80000000));
@@ -236,8 +257,8 @@ __device__ __forceinline__ void set_cone(WarpSmem<FAST, CAP>& sm, const rg_camer
 // by (|C| -+ |e.U| -+ |e.V|) / |D| per unit of its parameter.  The margin, a thousandth of R and 1e-5
 // of |O|, is above the rounding of this test and of the exact one by a factor of ten.  NaN (a
 // Gaussian that is never hit, an overflow) keeps the leaf: the exact test decides.
-template <bool FAST, int CAP>
-__device__ __forceinline__ bool may_hit(const WarpSmem<FAST, CAP>& sm, const LeafRec& rec, float3 o, float t0, float t1,
+template <bool FAST, int SUB, int CAP>
+__device__ __forceinline__ bool may_hit(const WarpSmem<FAST, SUB, CAP>& sm, const LeafRec& rec, float3 o, float t0, float t1,
                                         float& t_first) {
     const float4 q0 = *reinterpret_cast<const float4*>(sm.cone), q1 = *reinterpret_cast<const float4*>(sm.cone + 4),
                  q2 = *reinterpret_cast<const float4*>(sm.cone + 8);
@@ -398,6 +419,10 @@ __device__ __forceinline__ int nwords(int count) { return (count + 31) >> 5; }
 __device__ __forceinline__ bool occ_test(const unsigned long long* occ, int k) {
     return (occ[k >> 6] >> (k & 63)) & 1ull;
 }
+// whether any of the slabs k .. k + n - 1 is occupied (n <= 4, k a multiple of n: one word)
+__device__ __forceinline__ bool occ_any(const unsigned long long* occ, int k, int n) {
+    return (occ[k >> 6] >> (k & 63)) & ((1ull << n) - 1ull);
+}
 // first occupied slab >= k (K when none)
 __device__ __forceinline__ int occ_next(const unsigned long long* occ, int k, int K) {
     for (int w = k >> 6; w < 4 && 64 * w < K; ++w) {
@@ -409,8 +434,8 @@ __device__ __forceinline__ int occ_next(const unsigned long long* occ, int k, in
 }
 
 // Adds the tile's counters to the warp's totals and resets them.
-template <bool FAST, int CAP, bool DIAG>
-__device__ __forceinline__ void flush_stats(WarpSmem<FAST, CAP>& sm, WarpStats& ws, unsigned hits, unsigned slabs,
+template <bool FAST, int SUB, int CAP, bool DIAG>
+__device__ __forceinline__ void flush_stats(WarpSmem<FAST, SUB, CAP>& sm, WarpStats& ws, unsigned hits, unsigned slabs,
                                             int lane) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
@@ -433,16 +458,16 @@ __device__ __forceinline__ void flush_stats(WarpSmem<FAST, CAP>& sm, WarpStats& 
     ws = WarpStats();
 }
 
-// Exact leaf test of every active lane for the chunk [tb, seg_hi]: appends the leaf to the warp
-// list when any lane's interval meets one of the chunk's slabs.  Returns false (leaf not taken)
-// when the list is already full.
-template <bool FAST, int CAP, bool DIAG>
-__device__ __forceinline__ bool leaf_entry(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayState& r, bool on,
-                                           float seg_hi, int K, int nv, int leaf, int& count, int lane,
-                                           WarpStats& ws, bool infer) {
-    if (DIAG) ++ws.leaf_tests;
+// Exact test of SUB leaves at a time, each by the 32 / SUB rays of the tile (`leaf`: the one of the
+// lane's sub-slab, < 0 for none).  Leaves that any ray hits are appended to the list, in order.  Returns
+// how many leaves were dealt with: SUB, or the number of those before the one that found the list full.
+template <bool FAST, int SUB, int CAP, bool DIAG>
+__device__ __forceinline__ int leaf_batch(WarpSmem<FAST, SUB, CAP>& sm, const RenderArgs& a, const RayState& r, bool on,
+                                          float seg_hi, int K, int nv, int leaf, int& count, int lane,
+                                          WarpStats& ws, bool infer) {
+    if (DIAG) ws.leaf_tests += __popc(__ballot_sync(kFull, lane < SUB && leaf >= 0));
     int lo = 255, hi = -1;
-    if (on) {
+    if (on && (SUB == 1 || leaf >= 0)) {
         float root1, root2;
         bool ok;
         if (FAST) {
@@ -456,22 +481,61 @@ __device__ __forceinline__ bool leaf_entry(WarpSmem<FAST, CAP>& sm, const Render
         const float tclip = infer ? INFINITY : r.texit;
         if (ok) slab_range<FAST>(r, K, nv, seg_hi, tclip, root1, root2, lo, hi);
     }
-    unsigned any = __ballot_sync(kFull, lo <= hi);
-    if (!any) return true;
-    if (count == CAP) return false;
-    int ulo = (int)__reduce_min_sync(kFull, (unsigned)lo);
-    int uhi = (int)__reduce_max_sync(kFull, (unsigned)(hi + 1)) - 1;
-    if (FAST) {
-        if (lane == 0) sm.lmask[count] = any;
+    const unsigned any = __ballot_sync(kFull, lo <= hi);
+    if (!any) return SUB;
+    if constexpr (SUB == 1) {
+        if (count == CAP) return 0;
+        int ulo = (int)__reduce_min_sync(kFull, (unsigned)lo);
+        int uhi = (int)__reduce_max_sync(kFull, (unsigned)(hi + 1)) - 1;
+        if (FAST) {
+            if (lane == 0) sm.lmask[count] = any;
+        } else {
+            sm.lrng[count][lane] = (unsigned short)((lo & 0xff) | ((hi & 0xff) << 8));
+        }
+        if (lane == 0) {
+            sm.ids[count] = leaf;
+            sm.urng[count] = (unsigned)ulo | ((unsigned)uhi << 16);
+        }
+        ++count;
+        return 1;
     } else {
-        sm.lrng[count][lane] = (unsigned short)((lo & 0xff) | ((hi & 0xff) << 8));
+        const int sub = lane % SUB;
+        int ulo = lo, uhi = hi;
+        unsigned hit = any;          // bit q: some ray hits the leaf of sub-slab q
+#pragma unroll
+        for (int o = SUB; o < 32; o <<= 1) {
+            ulo = min(ulo, __shfl_xor_sync(kFull, ulo, o));
+            uhi = max(uhi, __shfl_xor_sync(kFull, uhi, o));
+            hit |= hit >> o;
+        }
+        hit &= (1u << SUB) - 1u;
+        const int at = count + __popc(hit & ((1u << sub) - 1u)), n = __popc(hit);
+        if (((hit >> sub) & 1u) && at < CAP) {
+            if (!FAST) sm.lrng[at][lane / SUB] = (unsigned short)((lo & 0xff) | ((hi & 0xff) << 8));
+            if (lane < SUB) {
+                if (FAST) sm.lmask[at] = (any >> sub) & TileShape<SUB>::lanes;
+                sm.ids[at] = leaf;
+                sm.urng[at] = (unsigned)ulo | ((unsigned)uhi << 16);
+            }
+        }
+        const int room = CAP - count;
+        count += min(n, room);
+        if (n <= room) return SUB;
+        // the first leaf without room: bit number `room` of the hits
+        for (int i = 0; i < room; ++i) hit &= hit - 1u;
+        return __ffs(hit) - 1;
     }
-    if (lane == 0) {
-        sm.ids[count] = leaf;
-        sm.urng[count] = (unsigned)ulo | ((unsigned)uhi << 16);
-    }
-    ++count;
-    return true;
+}
+
+// The lane's leaf of the next SUB in `todo` (bits of lanes whose `mine` holds a leaf): its sub-slab's, or -1.
+template <int SUB>
+__device__ __forceinline__ int next_leaf(unsigned todo, unsigned mine, int lane) {
+    unsigned t = todo;
+#pragma unroll
+    for (int i = 0; i < SUB - 1; ++i)
+        if (i < lane % SUB) t &= t - 1u;
+    const int leaf = (int)__shfl_sync(kFull, mine, __ffs(t) - 1);
+    return SUB == 1 || t ? leaf : -1;
 }
 
 // Bits lo..hi of 64-slab word w (none where the range does not meet it).
@@ -483,11 +547,11 @@ __device__ __forceinline__ unsigned long long range_bits(int lo, int hi, int w) 
 // Publishes the chunk list: occupancy bits and the entry masks per block of MB slabs.  One lane per
 // entry: a word of 32 entries costs a ballot per block and an OR-reduction per 32 slabs, against a
 // serial walk of all entries per block and, for the occupancy, by lane 0 as entries were appended.
-template <bool FAST, int CAP, bool DIAG>
-__device__ __forceinline__ void finish_list(WarpSmem<FAST, CAP>& sm, int count, int K, int lane, WarpStats& ws) {
+template <bool FAST, int SUB, int CAP, bool DIAG>
+__device__ __forceinline__ void finish_list(WarpSmem<FAST, SUB, CAP>& sm, int count, int K, int lane, WarpStats& ws) {
     __syncwarp();
     if (DIAG) ws.entries += count;
-    constexpr int MB = WarpSmem<FAST, CAP>::MB;
+    constexpr int MB = WarpSmem<FAST, SUB, CAP>::MB;
     const int nblk = (K + MB - 1) / MB, nocc = (K + 63) >> 6;
     const int nw = nwords(count);
     if (lane < 4) sm.occ[lane] = 0ull;
@@ -556,8 +620,8 @@ __device__ __forceinline__ void chunk_extent(const RayState& r, bool on, int K, 
 // traversal goes on from its stack with the smaller packet.  The list is the one that a traversal
 // started with the shorter chunk builds, and nothing is visited twice.  `ovf` is set when the list
 // filled up for a single slab before the traversal finished.
-template <bool FAST, int CAP, bool DIAG>
-__device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float t_end,
+template <bool FAST, int SUB, int CAP, bool DIAG>
+__device__ int traverse(WarpSmem<FAST, SUB, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float t_end,
                         float& seg_hi, int& K, int& nv, int cursor, bool& ovf, int lane, WarpStats& ws, bool infer) {
     int count = 0;
     ++ws.traversals;
@@ -595,7 +659,7 @@ __device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayS
             int first = 0;
             if (may) {
                 float t;
-                may = may_hit<FAST, CAP>(sm, load_rec(a.rec, (int)leaf), r.o, tb0 * 0.99999f, t1 * 1.00001f, t);
+                may = may_hit<FAST, SUB, CAP>(sm, load_rec(a.rec, (int)leaf), r.o, tb0 * 0.99999f, t1 * 1.00001f, t);
                 const float drift = (float)(K + 1) * (tb1 + (float)K * kSlab) * (kInvSlab * 2.4e-7f);
                 first = min(255, max(0, (int)((t - tb1) * kInvSlab - 1.f - drift)));
                 may = may && first < K;
@@ -665,7 +729,7 @@ __device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayS
             } while (K > 1 && kept > NC - 64);
             if (lane == 0) atomicAdd(&a.st->chunk_splits, (unsigned long long)halvings);
             chunk_extent(r, on, K, t_end, nv, seg_hi);
-            set_packet<FAST, CAP>(sm, r, on, seg_hi, lane);
+            set_packet<FAST, SUB, CAP>(sm, r, on, seg_hi, lane);
             int to = 0;
             for (int e = 0; e < nc; e += 32) {
                 const unsigned c = e + lane < nc ? cand[e + lane] : 0u;
@@ -709,9 +773,12 @@ __device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayS
                 todo = __ballot_sync(kFull, in && 2 * (int)(c >> 25) < K);
             }
             while (todo) {
-                const int leaf = (int)__shfl_sync(kFull, mine, __ffs(todo) - 1);
-                if (!leaf_entry<FAST, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, leaf, count, lane, ws, infer)) break;
-                todo &= todo - 1u;
+                const int leaf = next_leaf<SUB>(todo, mine, lane);
+                const int n = leaf_batch<FAST, SUB, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, leaf, count, lane, ws, infer);
+#pragma unroll
+                for (int i = 0; i < SUB; ++i)
+                    if (i < n) todo &= todo - 1u;
+                if (n < SUB) break;
             }
             if (!again) done = min(nc, done + (todo ? __ffs(todo) - 1 : 32));
             if (todo) {
@@ -732,7 +799,7 @@ __device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayS
                 } while (K > 1 && kept >= CAP);
                 if (lane == 0) atomicAdd(&a.st->chunk_splits, (unsigned long long)halvings);
                 chunk_extent(r, on, K, t_end, nv, seg_hi);
-                set_packet<FAST, CAP>(sm, r, on, seg_hi, lane);
+                set_packet<FAST, SUB, CAP>(sm, r, on, seg_hi, lane);
                 rt = 0;
                 rn = count;
                 count = 0;
@@ -741,28 +808,28 @@ __device__ int traverse(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayS
         }
     }
     if (DIAG) ws.node_visits += visits;
-    finish_list<FAST, CAP, DIAG>(sm, count, K, lane, ws);
+    finish_list<FAST, SUB, CAP, DIAG>(sm, count, K, lane, ws);
     return count;
 }
 
 // The chunk list from the forward's record: the recorded leaves (at most the list capacity) get
 // the same exact leaf test as in a traversal, without the traversal.
-template <bool FAST, int CAP, bool DIAG>
-__device__ int replay_list(WarpSmem<FAST, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float seg_hi,
+template <bool FAST, int SUB, int CAP, bool DIAG>
+__device__ int replay_list(WarpSmem<FAST, SUB, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float seg_hi,
                            int K, int nv, const unsigned* ids, int n, int lane, WarpStats& ws) {
     int count = 0;
     n = min(n, CAP);
     for (int base = 0; base < n; base += 32) {
-        const int m = min(32, n - base);
-        const int mine = lane < m ? (int)ids[base + lane] : 0;
-#pragma unroll 1
-        for (int j = 0; j < m; ++j) {
-            const int leaf = __shfl_sync(kFull, mine, j);
-            if (leaf >= 0 && leaf < a.n_leaves)
-                leaf_entry<FAST, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, leaf, count, lane, ws, false);
+        const int mine = base + lane < n ? (int)ids[base + lane] : -1;
+        unsigned todo = __ballot_sync(kFull, mine >= 0 && mine < a.n_leaves);
+        while (todo) {
+            const int leaf = next_leaf<SUB>(todo, (unsigned)mine, lane);
+            leaf_batch<FAST, SUB, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, leaf, count, lane, ws, false);
+#pragma unroll
+            for (int i = 0; i < SUB; ++i) todo &= todo - 1u;
         }
     }
-    finish_list<FAST, CAP, DIAG>(sm, count, K, lane, ws);
+    finish_list<FAST, SUB, CAP, DIAG>(sm, count, K, lane, ws);
     return count;
 }
 
@@ -848,21 +915,22 @@ __device__ __forceinline__ void parity_weights(const SlabPoints& sp, const LeafR
         w[p] = pk(lo2(d[p]) > kSigThr ? lo2(w[p]) : 0.f, hi2(d[p]) > kSigThr ? hi2(w[p]) : 0.f);
 }
 
-__device__ __forceinline__ bool in_range(unsigned short rg, int k) {
-    return k >= (int)(rg & 0xff) && k <= (int)(rg >> 8);
-}
 __device__ __forceinline__ bool in_urange(unsigned u, int k) {
     return k >= (int)(u & 0xffff) && k <= (int)(u >> 16);
 }
 
-// Whether the lane holds list entry e in slab k: the fast lists keep the lanes whose interval meets
-// the chunk, the parity lists each lane's exact slab range.
-template <bool FAST, int CAP>
-__device__ __forceinline__ bool lane_has_entry(const WarpSmem<FAST, CAP>& sm, const RenderArgs& a, int e, int k, int K,
-                                               int leaf, const RayState& r, int lane) {
-    if (FAST) return (sm.lmask[e] >> lane) & 1u;
-    const unsigned short rg = sm.lrng[e][lane];
-    return k >= (int)(rg & 0xff) && k <= (int)(rg >> 8);
+// Whether the lane's ray holds list entry e in its slab kl: the fast lists keep the rays whose interval
+// meets the chunk, the parity lists each ray's exact slab range.
+template <bool FAST, int SUB, int CAP>
+__device__ __forceinline__ bool lane_has_entry(const WarpSmem<FAST, SUB, CAP>& sm, int e, int kl, int lane) {
+    if (FAST) return ((sm.lmask[e] >> (lane / SUB * SUB)) & 1u) && (SUB == 1 || in_urange(sm.urng[e], kl));
+    const unsigned short rg = sm.lrng[e][lane / SUB];
+    return kl >= (int)(rg & 0xff) && kl <= (int)(rg >> 8);
+}
+// Whether an entry's union range meets the slabs k .. k + SUB - 1.
+template <int SUB>
+__device__ __forceinline__ bool meets_group(unsigned u, int k) {
+    return k + SUB - 1 >= (int)(u & 0xffff) && k <= (int)(u >> 16);
 }
 
 // Sample buffers of a slab: density sums and, in the forward, the density-weighted colours; in the
@@ -907,8 +975,8 @@ struct SlabBuf<false, GDOT> {
 static_assert(kPairs == 4, "four sample pairs per slab");
 
 // Sample buffers of slab k: the sums over the lane's hits.
-template <bool FAST, int CAP, bool GDOT, bool DIAG>
-__device__ __forceinline__ int slab_buffers(const WarpSmem<FAST, CAP>& sm, int k, int K, bool has, const RayState& r,
+template <bool FAST, int SUB, int CAP, bool GDOT, bool DIAG>
+__device__ __forceinline__ int slab_buffers(const WarpSmem<FAST, SUB, CAP>& sm, int k, int K, bool has, const RayState& r,
                                             const RenderArgs& a, int rgb_base, const float* roff,
                                             SlabBuf<FAST, GDOT>& sb, int nw, int lane, WarpStats& ws) {
     int nh = 0;
@@ -920,15 +988,15 @@ __device__ __forceinline__ int slab_buffers(const WarpSmem<FAST, CAP>& sm, int k
     }
 #pragma unroll 1
     for (int w = 0; w < nw; ++w) {
-        unsigned mw = sm.smask[k / WarpSmem<FAST, CAP>::MB][w];
+        unsigned mw = sm.smask[k / WarpSmem<FAST, SUB, CAP>::MB][w];
         while (mw) {
             const int e = 32 * w + __ffs(mw) - 1;
             mw &= mw - 1u;
-            if (!in_urange(sm.urng[e], k)) continue;
+            if (!meets_group<SUB>(sm.urng[e], k)) continue;
             if (DIAG) ++ws.entry_slabs;
             if (!has) continue;
             const int leaf = sm.ids[e];
-            if (!lane_has_entry<FAST, CAP>(sm, a, e, k, K, leaf, r, lane)) continue;
+            if (!lane_has_entry<FAST, SUB, CAP>(sm, e, k + lane % SUB, lane)) continue;
             LeafRec rec = load_rec(a.rec, leaf);
             float4 col4 = __ldg(a.rgb + rgb_base + leaf);
             float3 mu = f3(rec.a.x, rec.a.y, rec.a.z);
@@ -1097,31 +1165,43 @@ __device__ __forceinline__ void exp_neg_slab(const f2* sig, f2* ex, f2 nz) {
     }
 }
 
-// Alpha compositing of one slab's 8 samples (forward/gaussians_aabb.cu:500-519).  A slab whose
-// samples all fell under the threshold composites to exactly nothing (alpha = 1 - exp(0) = 0).
-template <bool FAST>
-__device__ __forceinline__ void composite(RayState& r, const SlabBuf<FAST, false>& sb, f2 nz) {
-    if (!sb.any_density()) return;
+// Opacities 1 - exp(-sig dt) of a slab's samples, in pairs.
+template <bool FAST, bool GDOT>
+__device__ __forceinline__ void slab_alpha(const SlabBuf<FAST, GDOT>& sb, f2* alpha, f2 nz) {
     if constexpr (FAST) {
 #pragma unroll
-        for (int i = 0; i < kBuf; ++i) {
-            // C[i] is zero wherever sig[i] is (both sum the same above-threshold samples)
-            float alpha = 1.f - exp_neg_fast(sb.sig[i] * kDt);
-            float s = sb.sig[i] > 0.f ? __fdividef(r.T * alpha, sb.sig[i]) : 0.f;
-            r.C = r.C + sb.C[i] * s;
-            r.T *= 1.f - alpha;
-        }
+        for (int p = 0; p < kPairs; ++p)
+            alpha[p] = pk(1.f - exp_neg_fast(sb.sig[2 * p] * kDt), 1.f - exp_neg_fast(sb.sig[2 * p + 1] * kDt));
     } else {
-        // the exponentials are independent of the transmittance chain: evaluate them first
         f2 ex[kPairs];
         exp_neg_slab(sb.sig, ex, nz);
 #pragma unroll
-        for (int p = 0; p < kPairs; ++p) {
-            const f2 alpha = fma2(ex[p], dup2(-1.f), dup2(1.f)), om = fma2(alpha, dup2(-1.f), dup2(1.f));
+        for (int p = 0; p < kPairs; ++p) alpha[p] = fma2(ex[p], dup2(-1.f), dup2(1.f));
+    }
+}
+
+// Alpha compositing of one slab's 8 samples (forward/gaussians_aabb.cu:500-519).  A slab whose
+// samples all fell under the threshold composites to exactly nothing (alpha = 1 - exp(0) = 0).
+template <bool FAST>
+__device__ __forceinline__ void composite(RayState& r, const SlabBuf<FAST, false>& sb, const f2* alpha, f2 nz) {
+    if (!sb.any_density()) return;
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) {
+        const f2 om = fma2(alpha[p], dup2(-1.f), dup2(1.f));
+        if constexpr (FAST) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                // C[i] is zero wherever sig[i] is (both sum the same above-threshold samples)
+                const int i = 2 * p + h;
+                const float s = sb.sig[i] > 0.f ? __fdividef(r.T * half2(alpha[p], h), sb.sig[i]) : 0.f;
+                r.C = r.C + sb.C[i] * s;
+                r.T *= half2(om, h);
+            }
+        } else {
             const float s0 = lo2(sb.sig[p]), s1 = hi2(sb.sig[p]);
             const f2 inv = pk(s0 > 0.f ? __frcp_rn(s0) : 0.f, s1 > 0.f ? __frcp_rn(s1) : 0.f);   // colours are 0 there
             const float T1 = __fmul_rn(r.T, lo2(om));
-            const f2 ta = mul2_rn(pk(r.T, T1), alpha, nz);
+            const f2 ta = mul2_rn(pk(r.T, T1), alpha[p], nz);
             const f2 cx = mul2_rn(mul2(sb.cx[p], inv), ta, nz), cy = mul2_rn(mul2(sb.cy[p], inv), ta, nz),
                      cz = mul2_rn(mul2(sb.cz[p], inv), ta, nz);
             r.C = f3(__fadd_rn(__fadd_rn(r.C.x, lo2(cx)), hi2(cx)), __fadd_rn(__fadd_rn(r.C.y, lo2(cy)), hi2(cy)),
@@ -1186,10 +1266,20 @@ struct AdjBuf<false> {
     f2 H[kPairs], F[kPairs];
 };
 
+// Adds the same value to every H.
+__device__ __forceinline__ void add_start(AdjBuf<true>& ad, float x) {
+#pragma unroll
+    for (int i = 0; i < kBuf; ++i) ad.H[i] += x;
+}
+__device__ __forceinline__ void add_start(AdjBuf<false>& ad, float x) {
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) ad.H[p] = add2(ad.H[p], dup2(x));
+}
+
 // Adjoint of slab k for all list entries: per-lane gradient of each hit Gaussian, warp reduction,
 // one atomic per value.  Value order: ddens, S1.xyz, M2 (xx yy zz xy xz yz), 0, drgb.xyz.
-template <bool FAST, int CAP, bool DIAG>
-__device__ __forceinline__ void slab_adjoint(const WarpSmem<FAST, CAP>& sm, int k, int K, bool has, const RayState& r,
+template <bool FAST, int SUB, int CAP, bool DIAG>
+__device__ __forceinline__ void slab_adjoint(const WarpSmem<FAST, SUB, CAP>& sm, int k, int K, bool has, const RayState& r,
                                              const RenderArgs& a, int rgb_base, const float* roff,
                                              const AdjBuf<FAST>& ad, int nw, int lane,
                                              WarpStats& ws, int view) {
@@ -1204,14 +1294,14 @@ __device__ __forceinline__ void slab_adjoint(const WarpSmem<FAST, CAP>& sm, int 
     const int vid = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
 #pragma unroll 1
     for (int w = 0; w < nw; ++w) {
-      unsigned mw = sm.smask[k / WarpSmem<FAST, CAP>::MB][w];
+      unsigned mw = sm.smask[k / WarpSmem<FAST, SUB, CAP>::MB][w];
       while (mw) {
         const int e = 32 * w + __ffs(mw) - 1;
         mw &= mw - 1u;
-        if (!in_urange(sm.urng[e], k)) continue;
+        if (!meets_group<SUB>(sm.urng[e], k)) continue;
         const int leaf = sm.ids[e];
         if (DIAG) ++ws.entry_slabs;
-        bool act = has && lane_has_entry<FAST, CAP>(sm, a, e, k, K, leaf, r, lane);
+        bool act = has && lane_has_entry<FAST, SUB, CAP>(sm, e, k + lane % SUB, lane);
         unsigned am = __ballot_sync(kFull, act);
         if (am == 0u) continue;
         float v[16];
@@ -1314,7 +1404,7 @@ __device__ __forceinline__ void slab_adjoint(const WarpSmem<FAST, CAP>& sm, int 
                                 v[12] != 0.f || v[13] != 0.f);
         const unsigned zm = __ballot_sync(kFull, nz);
         if (zm == 0u) continue;
-        if (__popc(zm) <= RG_DIRECT_ATOMIC_LANES) {
+        if (__popc(zm) <= (SUB == 1 ? RG_DIRECT_ATOMIC_LANES : RG_SPLIT_DIRECT_ATOMIC_LANES)) {
             if (nz) {
                 float4* g4 = reinterpret_cast<float4*>(gg);
                 atomicAdd(g4, make_float4(v[0], v[1], v[2], v[3]));
@@ -1340,34 +1430,32 @@ __device__ __forceinline__ void slab_adjoint(const WarpSmem<FAST, CAP>& sm, int 
 // E = dt (T gc - g.R), H = E - F gc, and g.R drops by gc T alpha per sample.
 // Returns H and F; advances T and g.R over the slab.
 template <bool FAST>
-__device__ __forceinline__ void slab_adjoint_scalars(const RayState& r, const SlabBuf<FAST, true>& sb, AdjBuf<FAST>& ad,
-                                                     float& Ta, float& gRa, f2 nz) {
+__device__ __forceinline__ void slab_adjoint_scalars(const RayState& r, const SlabBuf<FAST, true>& sb, const f2* alpha,
+                                                     AdjBuf<FAST>& ad, float& Ta, float& gRa, f2 nz) {
     Ta = r.T;
     gRa = r.gR;
-    if constexpr (FAST) {
 #pragma unroll
-        for (int i = 0; i < kBuf; ++i) {
-            const float cd = sb.sig[i];
-            float inv = 0.f;
-            if (cd > 0.f) inv = __fdividef(1.f, cd);
-            const float gc = sb.gC[i] * inv;
-            const float alpha = 1.f - exp_neg_fast(cd * kDt);
-            const float ta = Ta * alpha;
-            ad.F[i] = ta * inv;
-            ad.H[i] = kDt * (Ta * gc - gRa) - ad.F[i] * gc;
-            gRa -= gc * ta;
-            Ta = Ta * (1.f - alpha);
-        }
-    } else {
-        f2 ex[kPairs];
-        exp_neg_slab(sb.sig, ex, nz);
+    for (int p = 0; p < kPairs; ++p) {
+        const f2 om = fma2(alpha[p], dup2(-1.f), dup2(1.f));
+        if constexpr (FAST) {
 #pragma unroll
-        for (int p = 0; p < kPairs; ++p) {
-            const f2 alpha = fma2(ex[p], dup2(-1.f), dup2(1.f)), om = fma2(alpha, dup2(-1.f), dup2(1.f));
+            for (int h = 0; h < 2; ++h) {
+                const int i = 2 * p + h;
+                const float cd = sb.sig[i];
+                float inv = 0.f;
+                if (cd > 0.f) inv = __fdividef(1.f, cd);
+                const float gc = sb.gC[i] * inv;
+                const float ta = Ta * half2(alpha[p], h);
+                ad.F[i] = ta * inv;
+                ad.H[i] = kDt * (Ta * gc - gRa) - ad.F[i] * gc;
+                gRa -= gc * ta;
+                Ta = Ta * half2(om, h);
+            }
+        } else {
             const float s0 = lo2(sb.sig[p]), s1 = hi2(sb.sig[p]);
             const f2 inv = pk(s0 > 0.f ? __frcp_rn(s0) : 0.f, s1 > 0.f ? __frcp_rn(s1) : 0.f);
             const float T1 = __fmul_rn(Ta, lo2(om));
-            const f2 T2 = pk(Ta, T1), ngc = mul2(sb.ng[p], inv), ta = mul2(T2, alpha);   // ngc = -g.C / sigma
+            const f2 T2 = pk(Ta, T1), ngc = mul2(sb.ng[p], inv), ta = mul2(T2, alpha[p]);   // ngc = -g.C / sigma
             ad.F[p] = mul2(ta, inv);
             const float gR1 = fmaf(lo2(ngc), lo2(ta), gRa);
             ad.H[p] = fma2(ad.F[p], ngc, mul2(fma2(T2, ngc, pk(gRa, gR1)), dup2(-kDt)));
@@ -1375,6 +1463,32 @@ __device__ __forceinline__ void slab_adjoint_scalars(const RayState& r, const Sl
             Ta = __fmul_rn(T1, hi2(om));
         }
     }
+}
+
+// The slabs of a group (SUB > 1) in turn: the transmittance runs through them lane by lane, by the same
+// multiplications in the same order as slab after slab.  `has` (the lane marches its slab, as far as
+// its place on the ray goes) loses the lanes whose ray ended before (T <= 0.003); returns the
+// transmittance at the lane's start and leaves the group's end in r.T.
+template <int SUB>
+__device__ __forceinline__ float group_transmittance(RayState& r, const f2* alpha, bool dense, bool& has, int lane) {
+    float T = r.T, mine = r.T;
+#pragma unroll
+    for (int q = 0; q < SUB; ++q) {
+        if (lane % SUB == q) {
+            mine = T;
+            has = has && T > kTeps;
+            if (has && dense) {
+#pragma unroll
+                for (int p = 0; p < kPairs; ++p) {
+                    const f2 om = fma2(alpha[p], dup2(-1.f), dup2(1.f));
+                    T = __fmul_rn(__fmul_rn(T, lo2(om)), hi2(om));
+                }
+            }
+        }
+        T = __shfl_sync(kFull, T, lane / SUB * SUB + q);
+    }
+    r.T = T;
+    return mine;
 }
 
 // Resident blocks per SM each kernel is compiled for (0: the compiler's choice).  The fast defaults
@@ -1394,19 +1508,34 @@ __device__ __forceinline__ void slab_adjoint_scalars(const RayState& r, const Sl
 #ifndef RG_PAR_BWD_MIN_BLOCKS
 #define RG_PAR_BWD_MIN_BLOCKS 2
 #endif
-template <bool BWD, bool FAST>
+#ifndef RG_FAST_SPLIT_FWD_MIN_BLOCKS
+#define RG_FAST_SPLIT_FWD_MIN_BLOCKS 4
+#endif
+#ifndef RG_FAST_SPLIT_BWD_MIN_BLOCKS
+#define RG_FAST_SPLIT_BWD_MIN_BLOCKS 4
+#endif
+#ifndef RG_PAR_SPLIT_FWD_MIN_BLOCKS
+#define RG_PAR_SPLIT_FWD_MIN_BLOCKS 3
+#endif
+#ifndef RG_PAR_SPLIT_BWD_MIN_BLOCKS
+#define RG_PAR_SPLIT_BWD_MIN_BLOCKS 3
+#endif
+template <bool BWD, bool FAST, int SUB>
 constexpr int min_blocks() {
+    if (SUB > 1)
+        return FAST ? (BWD ? RG_FAST_SPLIT_BWD_MIN_BLOCKS : RG_FAST_SPLIT_FWD_MIN_BLOCKS)
+                    : (BWD ? RG_PAR_SPLIT_BWD_MIN_BLOCKS : RG_PAR_SPLIT_FWD_MIN_BLOCKS);
     return FAST ? (BWD ? RG_FAST_BWD_MIN_BLOCKS : RG_FAST_FWD_MIN_BLOCKS)
                 : (BWD ? RG_PAR_BWD_MIN_BLOCKS : RG_PAR_FWD_MIN_BLOCKS);
 }
 
 // DIAG: also count node visits, leaf tests, list entries, slab steps and entry-slabs (rg_status);
 // without it those counters compile away and the kernel holds fewer live registers.
-template <bool BWD, bool FAST, int CAP, bool DIAG>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) k_render(RenderArgs a) {
-    __shared__ WarpSmem<FAST, CAP> smem[kWarpsPerBlock];
+template <bool BWD, bool FAST, int SUB, int CAP, bool DIAG>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB>()) k_render(RenderArgs a) {
+    __shared__ WarpSmem<FAST, SUB, CAP> smem[kWarpsPerBlock];
     const int lane = threadIdx.x & 31;
-    WarpSmem<FAST, CAP>& sm = smem[threadIdx.x >> 5];
+    WarpSmem<FAST, SUB, CAP>& sm = smem[threadIdx.x >> 5];
     const ViewTable* vt = a.views;
     const float bg = a.white_bg ? 1.f : 0.f;
     if (lane == 0) {
@@ -1414,7 +1543,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
         for (int c = 0; c < kCounters; ++c) sm.cnt[c] = 0ull;
     }
     const int kmax =
-        min((a.rnd_sample == 1) ? min(a.chunk_slabs, kExactChunk) : a.chunk_slabs, WarpSmem<FAST, CAP>::KM);
+        min((a.rnd_sample == 1) ? min(a.chunk_slabs, kExactChunk) : a.chunk_slabs, WarpSmem<FAST, SUB, CAP>::KM);
 
     while (true) {
         int tile = 0;
@@ -1430,10 +1559,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
         const int view = lo;
         const rg_camera cam = a.cams[view];
         const int W = cam.width, H = cam.height;
-        const int tiles_x = (W + kTileW - 1) / kTileW;
+        using TS = TileShape<SUB>;
+        const int tiles_x = (W + TS::w - 1) / TS::w;
         const int local = tile - vt->tile_prefix[view];
-        const int px = (local % tiles_x) * kTileW + (lane & (kTileW - 1));
-        const int py = (local / tiles_x) * kTileH + (lane / kTileW);
+        const int ray = lane / SUB, sub = lane % SUB;
+        const int px = (local % tiles_x) * TS::w + ray % TS::w;
+        const int py = (local / tiles_x) * TS::h + ray / TS::w;
         const bool valid = px < W && py < H;
         const unsigned ray_l = (unsigned)(py * W + px);
         const int rgb_base = view * a.n_leaves;   // views x leaves < 2^31 (checked by the host)
@@ -1462,7 +1593,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
             float inv = __fdiv_rn(1.f, __fsqrt_rn(dot_rn(dir, dir)));
             r.d = f3(__fmul_rn(dir.x, inv), __fmul_rn(dir.y, inv), __fmul_rn(dir.z, inv));
             r.o = f3(cam.eye[0], cam.eye[1], cam.eye[2]);
-            set_cone<FAST, CAP>(sm, cam, dx, dy, valid, lane);
+            set_cone<FAST, SUB, CAP>(sm, cam, dx, dy, valid, lane);
         }
         {
             float scene[6];   // scene box, read per tile (not kept live through the tile's loops)
@@ -1525,17 +1656,17 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
             bool ovf = false;
             int count;
             const bool replayed = BWD && rec_cur != kNoRecord && !(rec_hdr & kRecordMulti);
-            if (!replayed) set_packet<FAST, CAP>(sm, r, on, seg_hi, lane);
+            if (!replayed) set_packet<FAST, SUB, CAP>(sm, r, on, seg_hi, lane);
             if (replayed) {
                 const unsigned n_ids = min(rec_hdr & 0xffffu, a.rec_cap - rec_cur - 2u);
-                count = replay_list<FAST, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, a.rec_arena + rec_cur + 2, (int)n_ids,
+                count = replay_list<FAST, SUB, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, a.rec_arena + rec_cur + 2, (int)n_ids,
                                                lane, ws);
                 ++ws.replays;
             } else {
-                count = traverse<FAST, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, -1, ovf, lane, ws, infer);
+                count = traverse<FAST, SUB, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, -1, ovf, lane, ws, infer);
             }
             const unsigned long long* occ = sm.occ;
-            if (!BWD && rec_here && sm.rec_first != kRecordFailed) {
+            if (!BWD && rec_here && sm.rec_prev != kRecordFailed) {
                 // chunk record: header (multi-pass flag | K << 16 | id count), next record, ids
                 const unsigned n_ids = ovf ? 0u : (unsigned)count;
                 const unsigned words = 2u + n_ids;
@@ -1550,7 +1681,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                         if (sm.rec_first == kNoRecord) sm.rec_first = off;
                         sm.rec_prev = off;
                     } else {
-                        sm.rec_first = kRecordFailed;
+                        sm.rec_prev = kRecordFailed;   // the chunks so far stay: the backward traverses after them
                         atomicAdd(&a.st->record_overflows, 1ull);
                     }
                 }
@@ -1560,52 +1691,130 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                 __syncwarp();
             }
             if (!ovf) {
-                for (int k = 0; k < K; ++k) {
-                    bool has = on && r.tb < r.texit && r.T > kTeps;
-                    if (!__any_sync(kFull, has)) break;
-                    if (!occ_test(occ, k)) {
-                        // no lane has a hit in slabs [k, k2): march them (tb only; T is unchanged)
-                        int k2 = occ_next(occ, k, K);
+                if constexpr (SUB == 1) {
+                    for (int k = 0; k < K; ++k) {
+                        bool has = on && r.tb < r.texit && r.T > kTeps;
+                        if (!__any_sync(kFull, has)) break;
+                        if (!occ_test(occ, k)) {
+                            // no lane has a hit in slabs [k, k2): march them (tb only; T is unchanged)
+                            int k2 = occ_next(occ, k, K);
+                            if (has) {
+                                for (int j = k; j < k2 && r.tb < r.texit; ++j) {
+                                    r.tb = r.tb + kSlab;
+                                    ++slabs_acc;
+                                }
+                            }
+                            k = k2 - 1;
+                            continue;
+                        }
+                        if (DIAG) ++ws.slab_steps;
+                        float roff[kBuf];
+                        unsigned seed_next = slab_offsets(a.rnd_sample, r.seed, roff);
+                        SlabBuf<FAST, BWD> sb;
+                        sb.clear();
+                        int nh = slab_buffers<FAST, SUB, CAP, BWD, DIAG>(sm, k, K, has, r, a, rgb_base, roff, sb, nwords(count),
+                                                                    lane, ws);
                         if (has) {
-                            for (int j = k; j < k2 && r.tb < r.texit; ++j) {
-                                r.tb = r.tb + kSlab;
-                                ++slabs_acc;
+                            ++slabs_acc;
+                            hits_acc += (!BWD && a.counts) ? min(nh, a.max_prim_slice) : nh;
+                            if (nh > a.max_prim_slice) atomicAdd(&a.st->slab_cap_exceeded, 1ull);
+                        }
+                        if constexpr (!BWD) {
+                            if (has && nh > 0) {
+                                f2 alpha[kPairs];
+                                slab_alpha(sb, alpha, a.neg_zero);
+                                composite<FAST>(r, sb, alpha, a.neg_zero);
+                                r.seed = seed_next;
+                            }
+                        } else {
+                            AdjBuf<FAST> ad;
+                            float Ta, gRa;
+                            f2 alpha[kPairs];
+                            slab_alpha(sb, alpha, a.neg_zero);
+                            slab_adjoint_scalars<FAST>(r, sb, alpha, ad, Ta, gRa, a.neg_zero);
+                            bool act = has && nh > 0 && sb.any_density();
+                            slab_adjoint<FAST, SUB, CAP, DIAG>(sm, k, K, act, r, a, rgb_base, roff, ad, nwords(count), lane, ws,
+                                                          view);
+                            if (has && nh > 0) {
+                                r.T = Ta;
+                                r.gR = gRa;
+                                r.seed = seed_next;
                             }
                         }
-                        k = k2 - 1;
-                        continue;
+                        if (has) r.tb = r.tb + kSlab;
                     }
-                    if (DIAG) ++ws.slab_steps;
-                    float roff[kBuf];
-                    unsigned seed_next = slab_offsets(a.rnd_sample, r.seed, roff);
-                    SlabBuf<FAST, BWD> sb;
-                    sb.clear();
-                    int nh = slab_buffers<FAST, CAP, BWD, DIAG>(sm, k, K, has, r, a, rgb_base, roff, sb, nwords(count),
-                                                                lane, ws);
-                    if (has) {
-                        ++slabs_acc;
-                        hits_acc += (!BWD && a.counts) ? min(nh, a.max_prim_slice) : nh;
-                        if (nh > a.max_prim_slice) atomicAdd(&a.st->slab_cap_exceeded, 1ull);
-                    }
-                    if constexpr (!BWD) {
-                        if (has && nh > 0) {
-                            composite<FAST>(r, sb, a.neg_zero);
-                            r.seed = seed_next;
+                } else {
+                    for (int k = 0; k < K; k += SUB) {
+                        const bool base = on && r.tb < r.texit && r.T > kTeps;
+                        if (!__any_sync(kFull, base)) break;
+                        const int n = min(SUB, K - k);   // slabs of the group inside the chunk
+                        if (!occ_any(occ, k, n)) {
+                            // march the groups without a hit (tb only; T is unchanged)
+                            const int k2 = occ_next(occ, k, K), stop = k2 < K ? k2 / SUB * SUB : K;
+                            if (base) {
+                                for (int j = k; j < stop && r.tb < r.texit; ++j) {
+                                    r.tb = r.tb + kSlab;
+                                    if (sub == 0) ++slabs_acc;
+                                }
+                            }
+                            k = stop - SUB;
+                            if (stop == K) break;
+                            continue;
                         }
-                    } else {
-                        AdjBuf<FAST> ad;
-                        float Ta, gRa;
-                        slab_adjoint_scalars<FAST>(r, sb, ad, Ta, gRa, a.neg_zero);
-                        bool act = has && nh > 0 && sb.any_density();
-                        slab_adjoint<FAST, CAP, DIAG>(sm, k, K, act, r, a, rgb_base, roff, ad, nwords(count), lane, ws,
-                                                      view);
-                        if (has && nh > 0) {
-                            r.T = Ta;
-                            r.gR = gRa;
-                            r.seed = seed_next;
+                        if (DIAG) ++ws.slab_steps;
+                        // the lane's slab starts sub slabs on, by repeated addition; r.tb while it is marched
+                        const float tb0 = r.tb;
+#pragma unroll
+                        for (int j = 0; j < SUB - 1; ++j)
+                            if (j < sub) r.tb = r.tb + kSlab;
+                        const float tb_end = r.tb + kSlab;
+                        bool has = base && sub < n && r.tb < r.texit;
+                        float roff[kBuf];
+                        slab_offsets(a.rnd_sample, r.seed, roff);
+                        SlabBuf<FAST, BWD> sb;
+                        sb.clear();
+                        const int nh = slab_buffers<FAST, SUB, CAP, BWD, DIAG>(sm, k, K, has, r, a, rgb_base, roff, sb,
+                                                                               nwords(count), lane, ws);
+                        const bool dense = nh > 0 && sb.any_density();
+                        f2 alpha[kPairs];
+                        slab_alpha(sb, alpha, a.neg_zero);
+                        const float T0 = group_transmittance<SUB>(r, alpha, dense, has, lane);
+                        const float T_end = r.T;
+                        r.T = T0;
+                        if (has) {
+                            ++slabs_acc;
+                            hits_acc += (!BWD && a.counts) ? min(nh, a.max_prim_slice) : nh;
+                            if (nh > a.max_prim_slice) atomicAdd(&a.st->slab_cap_exceeded, 1ull);
                         }
+                        if constexpr (!BWD) {
+                            // each lane keeps the colour of its own slabs
+                            if (has && dense) composite<FAST>(r, sb, alpha, a.neg_zero);
+                        } else {
+                            // g . R is linear through the scalars: from 0 first, then the lane's start, which
+                            // is the group's less what the slabs before the lane's took
+                            AdjBuf<FAST> ad;
+                            float Ta, took;
+                            const float gR0 = r.gR;
+                            r.gR = 0.f;
+                            slab_adjoint_scalars<FAST>(r, sb, alpha, ad, Ta, took, a.neg_zero);
+                            if (!(has && dense)) took = 0.f;
+                            float upto = took;
+#pragma unroll
+                            for (int o = 1; o < SUB; o <<= 1) {
+                                const float v = __shfl_up_sync(kFull, upto, o);
+                                if (sub >= o) upto += v;
+                            }
+                            const float all = __shfl_sync(kFull, upto, ray * SUB + SUB - 1);
+                            add_start(ad, -kDt * (gR0 + (upto - took)));
+                            slab_adjoint<FAST, SUB, CAP, DIAG>(sm, k, K, has && dense, r, a, rgb_base, roff, ad,
+                                                               nwords(count), lane, ws, view);
+                            r.gR = gR0 + all;
+                        }
+                        r.T = T_end;
+                        // on to the next group (or the end of the chunk)
+                        const float t_next = __shfl_sync(kFull, tb_end, ray * SUB + n - 1);
+                        r.tb = base ? t_next : tb0;
                     }
-                    if (has) r.tb = r.tb + kSlab;
                 }
                 // next chunk length: aim at half a list, grow at most 2x per chunk
                 {
@@ -1614,20 +1823,20 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                 }
             } else {
                 // K == 1 and more hits than the list holds: consume the slab in several passes
-                bool has = on && nv > 0 && r.T > kTeps;
+                const bool has_ray = on && nv > 0 && r.T > kTeps, has = has_ray && sub == 0;
                 float roff[kBuf];
                 unsigned seed_next = slab_offsets(a.rnd_sample, r.seed, roff);
                 SlabBuf<FAST, BWD> sb;
                 sb.clear();
-                int nh = slab_buffers<FAST, CAP, BWD, DIAG>(sm, 0, 1, has, r, a, rgb_base, roff, sb, nwords(count), lane,
+                int nh = slab_buffers<FAST, SUB, CAP, BWD, DIAG>(sm, 0, 1, has, r, a, rgb_base, roff, sb, nwords(count), lane,
                                                             ws);
                 bool more = ovf;
                 while (more) {
                     int cursor = sm.ids[count - 1];
                     __syncwarp();
                     if (lane == 0) atomicAdd(&a.st->list_passes, 1ull);
-                    count = traverse<FAST, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, more, lane, ws, infer);
-                    nh += slab_buffers<FAST, CAP, BWD, DIAG>(sm, 0, 1, has, r, a, rgb_base, roff, sb, nwords(count), lane,
+                    count = traverse<FAST, SUB, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, more, lane, ws, infer);
+                    nh += slab_buffers<FAST, SUB, CAP, BWD, DIAG>(sm, 0, 1, has, r, a, rgb_base, roff, sb, nwords(count), lane,
                                                              ws);
                 }
                 if (has) {
@@ -1637,19 +1846,23 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                 }
                 if constexpr (!BWD) {
                     if (has && nh > 0) {
-                        composite<FAST>(r, sb, a.neg_zero);
+                        f2 alpha[kPairs];
+                        slab_alpha(sb, alpha, a.neg_zero);
+                        composite<FAST>(r, sb, alpha, a.neg_zero);
                         r.seed = seed_next;
                     }
                 } else {
                     AdjBuf<FAST> ad;
-                        float Ta, gRa;
-                    slab_adjoint_scalars<FAST>(r, sb, ad, Ta, gRa, a.neg_zero);
+                    float Ta, gRa;
+                    f2 alpha[kPairs];
+                    slab_alpha(sb, alpha, a.neg_zero);
+                    slab_adjoint_scalars<FAST>(r, sb, alpha, ad, Ta, gRa, a.neg_zero);
                     bool act = has && nh > 0 && sb.any_density();
                     int cursor = -1;
                     bool more2 = true;
                     while (more2) {
-                        count = traverse<FAST, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, more2, lane, ws, infer);
-                        slab_adjoint<FAST, CAP, DIAG>(sm, 0, 1, act, r, a, rgb_base, roff, ad, nwords(count), lane, ws,
+                        count = traverse<FAST, SUB, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, more2, lane, ws, infer);
+                        slab_adjoint<FAST, SUB, CAP, DIAG>(sm, 0, 1, act, r, a, rgb_base, roff, ad, nwords(count), lane, ws,
                                                       view);
                         if (more2) cursor = sm.ids[count - 1];
                         __syncwarp();
@@ -1660,16 +1873,28 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST>()) 
                         r.seed = seed_next;
                     }
                 }
-                if (has) r.tb = r.tb + kSlab;
+                if constexpr (SUB > 1) {
+                    r.T = __shfl_sync(kFull, r.T, ray * SUB);
+                    r.gR = __shfl_sync(kFull, r.gR, ray * SUB);
+                }
+                if (has_ray) r.tb = r.tb + kSlab;
             }
             if (on) r.alive = r.alive && (r.T > kTeps) && (r.tb < r.texit);
             if (BWD && lane == 0) sm.rec_cur = (rec_cur != kNoRecord) ? a.rec_arena[rec_cur + 1] : kNoRecord;
             __syncwarp();
         }
         if (!BWD && rec_here && lane == 0)
-            a.rec_tile[tile] = (sm.rec_first == kRecordFailed) ? kNoRecord : sm.rec_first;
-        flush_stats<FAST, CAP, DIAG>(sm, ws, hits_acc, slabs_acc, lane);
-        if (!BWD && valid) {
+            a.rec_tile[tile] = sm.rec_first;
+        flush_stats<FAST, SUB, CAP, DIAG>(sm, ws, hits_acc, slabs_acc, lane);
+        if constexpr (!BWD && SUB > 1) {
+#pragma unroll
+            for (int o = 1; o < SUB; o <<= 1) {
+                r.C = f3(r.C.x + __shfl_xor_sync(kFull, r.C.x, o), r.C.y + __shfl_xor_sync(kFull, r.C.y, o),
+                         r.C.z + __shfl_xor_sync(kFull, r.C.z, o));
+                hits_acc += __shfl_xor_sync(kFull, hits_acc, o);
+            }
+        }
+        if (!BWD && valid && sub == 0) {
             const long long ray_g = vt->ray_prefix[view] + (long long)ray_l;
             a.ray_colors[3 * ray_g] = __fadd_rn(r.C.x, __fmul_rn(r.T, bg));
             a.ray_colors[3 * ray_g + 1] = __fadd_rn(r.C.y, __fmul_rn(r.T, bg));
@@ -1732,64 +1957,82 @@ cudaError_t launch_moment_grads(int n, const LeafRec* rec, const float4* ext, fl
 }
 
 // List capacity per arithmetic: 4x the tuning value (64 or 128) for the fast lists; 128 for the
-// parity lists at either value (their per-lane slab ranges make an entry 64 B; shorter lists turn
-// dense slabs into multi-pass traversals, which the backward cannot replay).
-static_assert(sizeof(WarpSmem<false, 128>) * kWarpsPerBlock <= 48 * 1024, "static shared memory limit");
-// the packet is read as float4: 16-byte aligned in every warp's slice of the block's array
-using ParitySmem = WarpSmem<false, 128>;
-using FastSmem256 = WarpSmem<true, 256>;
-using FastSmem512 = WarpSmem<true, 512>;
-static_assert(offsetof(ParitySmem, cone) % 16 == 0 && offsetof(FastSmem256, cone) % 16 == 0 &&
-                  offsetof(FastSmem512, cone) % 16 == 0,
-              "cone alignment");
-static_assert(offsetof(ParitySmem, packet) % 16 == 0 && sizeof(ParitySmem) % 16 == 0, "packet alignment");
-static_assert(offsetof(FastSmem256, packet) % 16 == 0 && sizeof(FastSmem256) % 16 == 0, "packet alignment");
-static_assert(offsetof(FastSmem512, packet) % 16 == 0 && sizeof(FastSmem512) % 16 == 0, "packet alignment");
-static_assert(sizeof(WarpSmem<true, 512>) * kWarpsPerBlock <= 48 * 1024, "static shared memory limit");
+// parity lists of whole tiles at either value (their slab ranges make an entry 72 B; shorter lists turn
+// dense slabs into multi-pass traversals, which the backward cannot replay).  The split tiles hold 256
+// entries in either arithmetic.
+using ParitySmem = WarpSmem<false, 1, 128>;
+using FastSmem256 = WarpSmem<true, 1, 256>;
+using FastSmem512 = WarpSmem<true, 1, 512>;
+using ParitySplit2Smem = WarpSmem<false, 2, 192>;
+using ParitySplitSmem = WarpSmem<false, 4, 256>;
+using FastSplit2Smem = WarpSmem<true, 2, 256>;
+using FastSplitSmem = WarpSmem<true, 4, 256>;
+// packet and cone are read as float4: 16-byte aligned in every warp's slice of the block's array
+template <typename S>
+constexpr bool smem_fits() {
+    return offsetof(S, packet) % 16 == 0 && offsetof(S, cone) % 16 == 0 && sizeof(S) % 16 == 0 &&
+           sizeof(S) * kWarpsPerBlock <= 48 * 1024;
+}
+static_assert(smem_fits<ParitySmem>() && smem_fits<FastSmem256>() && smem_fits<FastSmem512>() &&
+                  smem_fits<ParitySplit2Smem>() && smem_fits<FastSplit2Smem>() && smem_fits<ParitySplitSmem>() &&
+                  smem_fits<FastSplitSmem>(),
+              "alignment, static shared memory limit");
 
-template <bool BWD, bool FAST>
-static cudaError_t launch_cap(int cap, int grid, const RenderArgs& a, cudaStream_t s) {
-    const int threads = kWarpsPerBlock * 32;
-    if constexpr (FAST) {
-        if (cap <= 64) {
-            if (a.diag) k_render<BWD, FAST, 256, true><<<grid, threads, 0, s>>>(a);
-            else k_render<BWD, FAST, 256, false><<<grid, threads, 0, s>>>(a);
-        } else {
-            if (a.diag) k_render<BWD, FAST, 512, true><<<grid, threads, 0, s>>>(a);
-            else k_render<BWD, FAST, 512, false><<<grid, threads, 0, s>>>(a);
-        }
-    } else {
-        if (a.diag) k_render<BWD, FAST, 128, true><<<grid, threads, 0, s>>>(a);
-        else k_render<BWD, FAST, 128, false><<<grid, threads, 0, s>>>(a);
-    }
-    return cudaGetLastError();
+// The kernel of a launch: calls f(kernel).
+template <bool BWD, bool FAST, bool DIAG, typename F>
+static void with_kernel(int cap, int split, F f) {
+    if (split == 4) f(k_render<BWD, FAST, 4, 256, DIAG>);
+    else if (split == 2) f(k_render<BWD, FAST, 2, FAST ? 256 : 192, DIAG>);
+    else if constexpr (!FAST) f(k_render<BWD, FAST, 1, 128, DIAG>);
+    else if (cap <= 64) f(k_render<BWD, FAST, 1, 256, DIAG>);
+    else f(k_render<BWD, FAST, 1, 512, DIAG>);
+}
+template <bool DIAG, typename F>
+static void with_kernel(bool backward, bool fast, int cap, int split, F f) {
+    if (backward) fast ? with_kernel<true, true, DIAG>(cap, split, f) : with_kernel<true, false, DIAG>(cap, split, f);
+    else fast ? with_kernel<false, true, DIAG>(cap, split, f) : with_kernel<false, false, DIAG>(cap, split, f);
 }
 
-template <bool BWD, bool FAST>
-static int occ_cap(int cap) {
+int render_occupancy(bool backward, int mode, int cap, int split) {
     int nb = 0;
-    const int threads = kWarpsPerBlock * 32;
-    if constexpr (FAST) {
-        if (cap <= 64) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_render<BWD, FAST, 256, false>, threads, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_render<BWD, FAST, 512, false>, threads, 0);
-    } else {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_render<BWD, FAST, 128, false>, threads, 0);
-    }
+    with_kernel<false>(backward, mode == RG_MODE_FAST, cap, split, [&](auto kernel) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, kWarpsPerBlock * 32, 0);
+    });
     return nb;
 }
 
-int render_occupancy(bool backward, int mode, int cap) {
-    bool fast = mode == RG_MODE_FAST;
-    if (backward) return fast ? occ_cap<true, true>(cap) : occ_cap<true, false>(cap);
-    return fast ? occ_cap<false, true>(cap) : occ_cap<false, false>(cap);
+// Slabs side by side, by the launch's number of 8x4-pixel tiles.  Forward + backward in ms with 4 / 2 / 1
+// slabs, one view of SH-1 Gaussians:
+//   fast     1536 tiles:  300k on shells  9.2 / 18.3 / 41.0   1M in a ball with a far field  7.9 /  9.3 / 15.6
+//            7350         300k shells     7.8 / 10.1 / 18.2   1M ball                       19.0 / 14.8 / 14.8
+//           15000         50k shells      2.0 /  1.6 /  2.0   1M ball                       35.0 / 26.0 / 21.5
+//           28359         50k shells      3.3 /  2.3 /  2.2   1M ball                       62.1 / 45.1 / 34.1
+//   parity   7350         300k shells    12.8 / 19.8 / 35.6   50k shells                     2.9 /  2.6 /  3.9
+//           15000         300k shells    18.3 / 22.6 / 34.9   50k shells                     5.1 /  3.7 /  4.2
+//           28359         300k shells    27.4 / 26.7 / 41.5   50k shells                     8.9 /  5.8 /  5.1
+// Few tiles wait for the slowest one, which the split shortens; many share the traversal better when
+// they are whole.  The parity kernels' lists hold fewer entries of a whole tile, so that dense tiles
+// (many Gaussians per tile) gain from the split for longer.  The lines lie where the geometric means
+// over these scenes and some of several views cross.  Whole steps: 10k Gaussians at 200x200, drop-in,
+// 1.56 ms whole and 0.86 split; 300k on shells at 797x801, drop-in, 35.2 and 19.0; three uneven views of
+// 60k on shells, fast, 8.9 and 2.4.
+int render_split(int mode, int rnd_sample, int cap, long long n, long long n_rays) {
+    const bool fast = mode == RG_MODE_FAST && rnd_sample == 0;
+    // random offsets draw slab after slab; long lists are whole tiles' (the autotuner's choice)
+    if (rnd_sample == 1 || cap > 64 || n_rays <= 0) return 1;
+    const long long tiles = n_rays / (kTileW * kTileH);
+    if (tiles <= (fast ? 8000 : 5000) || (!fast && tiles <= 30000 && tiles <= n / 10)) return 4;
+    return tiles <= (fast ? 22000 : 40000) ? 2 : 1;
 }
 
-cudaError_t launch_render(bool backward, int mode, int cap, int grid, const RenderArgs& args, cudaStream_t s) {
+cudaError_t launch_render(bool backward, int mode, int cap, int split, int grid, const RenderArgs& args, cudaStream_t s) {
     RenderArgs a = args;
     a.neg_zero = 0x8000000080000000ull;
-    bool fast = (mode == RG_MODE_FAST) && a.rnd_sample == 0;
-    if (backward) return fast ? launch_cap<true, true>(cap, grid, a, s) : launch_cap<true, false>(cap, grid, a, s);
-    return fast ? launch_cap<false, true>(cap, grid, a, s) : launch_cap<false, false>(cap, grid, a, s);
+    const bool fast = (mode == RG_MODE_FAST) && a.rnd_sample == 0;
+    auto launch = [&](auto kernel) { kernel<<<grid, kWarpsPerBlock * 32, 0, s>>>(a); };
+    if (a.diag) with_kernel<true>(backward, fast, cap, split, launch);
+    else with_kernel<false>(backward, fast, cap, split, launch);
+    return cudaGetLastError();
 }
 
 }  // namespace rg

@@ -232,11 +232,13 @@ class Engine:
         self.generation += 1
 
     def launch_forward(self, cams_t, n_cams, settings, ray_colors, final_T=None):
+        self.lib.rg_expect_rays(self.h, ray_colors.shape[0])
         with self._timed("launch_forward"):
                 check(self.lib.rg_launch_forward(self.h, _ptr(cams_t), int(n_cams), ctypes.byref(settings),
                                              _ptr(ray_colors), _ptr(final_T), _stream(self.device)), self.h, "rg_launch_forward")
 
     def launch_backward(self, cams_t, n_cams, settings, ray_colors, dL):
+        self.lib.rg_expect_rays(self.h, ray_colors.shape[0])
         with self._timed("launch_backward"):
             check(self.lib.rg_launch_backward(self.h, _ptr(cams_t), int(n_cams), ctypes.byref(settings),
                                               _ptr(ray_colors), _ptr(dL), _stream(self.device)), self.h, "rg_launch_backward")
@@ -269,6 +271,7 @@ class Engine:
         return ray_colors, fT
 
     def launch_inference(self, cams_t, n_cams, settings, ray_colors, counts=None):
+        self.lib.rg_expect_rays(self.h, ray_colors.shape[0])
         with self._timed("launch_inference"):
             check(self.lib.rg_launch_inference(self.h, _ptr(cams_t), int(n_cams), ctypes.byref(settings),
                                                _ptr(ray_colors), _ptr(counts), _stream(self.device)), self.h,

@@ -1,4 +1,4 @@
-"""The traversal's leaf culling and its shortened chunks where they can go wrong: wide and narrow tile
+"""The traversal's leaf culling and its shortened chunks, in both tile layouts, where they can go wrong: wide and narrow tile
 cones, a camera inside Gaussians, needles, far and dense clusters that overfill a long chunk or a
 single slab.  Parity images equal the oracle's within the drop-in's image bound; the fast
 arithmetic, whose samples differ by rounding, is held to its own bound on small scenes (5e-4)."""
@@ -15,7 +15,7 @@ TOL = {"parity": 1e-4, "fast": 5e-4}
 def _scene(kind):
     from ray_gauss_b200 import synthetic as S
     rng = np.random.default_rng(11)
-    n = 3000 if kind in ("dense", "far_dense") else 800
+    n = 12000 if kind in ("dense", "far_dense") else 800
     p, _, _ = S.workload("small_object", n=n, seed=5)
     eye, fov = [0.0, -3.0, 0.4], 40.0
     if kind == "needles":
@@ -33,9 +33,11 @@ def _scene(kind):
     return {k: v.contiguous() for k, v in p.items()}, eye, fov
 
 
+# a launch this small runs on split tiles with the list capacity of 64, on whole ones with 128
+@pytest.mark.parametrize("capacity", [64, 128])
 @pytest.mark.parametrize("mode", ["parity", "fast"])
 @pytest.mark.parametrize("kind", ["needles", "inside", "dense", "far_dense"])
-def test_traversal_against_oracle(cuda, oracle, kind, mode):
+def test_traversal_against_oracle(cuda, oracle, kind, mode, capacity):
     from ray_gauss_b200 import synthetic as S
     from ray_gauss_b200.batched import BatchedViews, render_views
     from ray_gauss_b200.engine import Engine
@@ -46,6 +48,7 @@ def test_traversal_against_oracle(cuda, oracle, kind, mode):
     N = {k: v.numpy() for k, v in p.items()}
     P = {k: v.to(cuda) for k, v in p.items()}
     eng = Engine()
+    eng.set_tuning(list_capacity=capacity)
     img = render_views(P, BatchedViews([cam], mode=mode, engine=eng)).cpu().numpy()
     rgb = oracle.forward_sh(cv[:3], N["positions"], N["color_features"], None, None, None)
     ref, _, _ = oracle.render_forward(N["positions"], N["scales"], N["quaternions"], N["densities"], rgb, cv, w, h, True)
