@@ -8,13 +8,21 @@
 // entries (two neighbours: about FLT_MAX / 3; one or none: +inf).  Its Morton boxes only prune the
 // search.
 //
-// This engine's search: points sorted by a 30-bit Morton code (k_knn_bounds, k_knn_morton, CUB
-// radix sort), boxes of kBox consecutive sorted points (k_knn_boxes), then one warp per 32
-// consecutive sorted points (k_knn_query): the warp's own box and its neighbours first, then every
-// other box whose distance to the warp's query box is at most the warp's largest third-best
-// distance; a surviving box's points are loaded once and broadcast by shuffle to all 32 queries.
+// This engine's search: points sorted by a 48-bit Morton code (k_knn_bounds, k_knn_morton, CUB radix
+// sort) and copied in that order, boxes of kBox consecutive points and groups of kGroup boxes
+// (k_knn_boxes), then one warp per 32 consecutive points (k_knn_query): the warp's own box and its
+// neighbours first, then groups and their boxes, nearest first, as long as their distance to the warp's
+// query box is at most the warp's largest third-best distance; a box that some lane's own point is
+// near enough to is staged in shared memory and read by all 32 queries.
+//
+// Bound by instruction issue in dense regions and by the warps of sparse ones, whose 32 points lie far
+// apart: they decide when the launch ends, and prune the sooner the nearer boxes come first.  200k
+// points (80 % in a ball, 20 % out to 50 times its radius): 1.11 ms before the finer code (ten bits an
+// axis left hundreds of points of a dense core in one cell), the nearest-first order, the groups and the
+// points in sorted order, 0.50 ms now; a million 5.85 and 1.47 ms.
 #include <cfloat>
 #include <cstdint>
+#include <type_traits>
 
 #include <cub/device/device_radix_sort.cuh>
 
@@ -25,17 +33,22 @@ namespace {
 using rg::f2ord;
 using rg::ord2f;
 
-constexpr int kBox = 64;          // sorted points per box: two per lane
+constexpr int kBox = 32;          // sorted points per box: one per lane, and a warp's queries
+constexpr int kGroup = 32;        // boxes per group: one per lane
 constexpr int kNear = 2;          // boxes on each side of the warp's own box scanned first
+constexpr int kMortonBits = 16;   // per axis
 
 struct KnnWs {
     int* bounds;                  // 6 ordered ints: scene min, max
-    unsigned* keys_in;
-    unsigned* keys_out;
+    unsigned long long* keys_in;
+    unsigned long long* keys_out;
     int* vals_in;
     int* vals_out;                // sorted point ids
+    float4* pts;                  // points in sorted order
     float4* box_lo;
     float4* box_hi;
+    float4* group_lo;
+    float4* group_hi;
     void* sort_temp;
     size_t sort_bytes;
 };
@@ -44,31 +57,41 @@ size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
 
 size_t sort_bytes(long long n) {
     size_t b = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, b, (const unsigned*)nullptr, (unsigned*)nullptr, (const int*)nullptr,
-                                    (int*)nullptr, (int)n, 0, 30);
+    cub::DeviceRadixSort::SortPairs(nullptr, b, (const unsigned long long*)nullptr, (unsigned long long*)nullptr,
+                                    (const int*)nullptr, (int*)nullptr, (int)n, 0, 3 * kMortonBits);
     return b;
 }
 
-size_t ws_bytes(long long n) {
-    const long long nb = (n + kBox - 1) / kBox;
-    return 256 + a256(6 * sizeof(int)) + 4 * a256(sizeof(int) * n) + 2 * a256(sizeof(float4) * nb) +
-           a256(sort_bytes(n));
-}
+long long n_boxes(long long n) { return (n + kBox - 1) / kBox; }
+long long n_groups(long long n) { return (n_boxes(n) + kGroup - 1) / kGroup; }
 
-KnnWs carve(void* base, long long n) {
+KnnWs carve(void* base, long long n, size_t* end = nullptr) {
     uintptr_t p = (reinterpret_cast<uintptr_t>(base) + 255) & ~uintptr_t(255);
-    const long long nb = (n + kBox - 1) / kBox;
+    auto take = [&](auto*& q, size_t count) {
+        q = reinterpret_cast<std::remove_reference_t<decltype(q)>>(p);
+        p += a256(sizeof(*q) * count);
+    };
     KnnWs w;
-    w.bounds = reinterpret_cast<int*>(p); p += a256(6 * sizeof(int));
-    w.keys_in = reinterpret_cast<unsigned*>(p); p += a256(sizeof(int) * n);
-    w.keys_out = reinterpret_cast<unsigned*>(p); p += a256(sizeof(int) * n);
-    w.vals_in = reinterpret_cast<int*>(p); p += a256(sizeof(int) * n);
-    w.vals_out = reinterpret_cast<int*>(p); p += a256(sizeof(int) * n);
-    w.box_lo = reinterpret_cast<float4*>(p); p += a256(sizeof(float4) * nb);
-    w.box_hi = reinterpret_cast<float4*>(p); p += a256(sizeof(float4) * nb);
+    take(w.bounds, 6);
+    take(w.keys_in, n);
+    take(w.keys_out, n);
+    take(w.vals_in, n);
+    take(w.vals_out, n);
+    take(w.pts, n);
+    take(w.box_lo, n_boxes(n));
+    take(w.box_hi, n_boxes(n));
+    take(w.group_lo, n_groups(n));
+    take(w.group_hi, n_groups(n));
     w.sort_temp = reinterpret_cast<void*>(p);
     w.sort_bytes = sort_bytes(n);
+    if (end) *end = p + a256(w.sort_bytes);
     return w;
+}
+
+size_t ws_bytes(long long n) {
+    size_t end = 0;
+    carve(nullptr, n, &end);
+    return end + 256;             // the base is rounded up to 256 bytes
 }
 
 __global__ void k_knn_init_bounds(int* b) {
@@ -76,83 +99,110 @@ __global__ void k_knn_init_bounds(int* b) {
     else if (threadIdx.x < 6) b[threadIdx.x] = f2ord(-INFINITY);
 }
 
+__device__ __forceinline__ float warp_min(float v) {
+    for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// Grid-stride, a handful of blocks per SM: the six atomics of a block are on the same addresses.
 __global__ void __launch_bounds__(256) k_knn_bounds(long long n, const float* __restrict__ p, int* __restrict__ b) {
-    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    if (i < n) {
-        for (int a = 0; a < 3; ++a) lo[a] = hi[a] = p[3 * i + a];
-    }
-    for (int a = 0; a < 3; ++a) {
-        for (int o = 16; o; o >>= 1) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-        }
-    }
-    if ((threadIdx.x & 31) == 0) {
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += 256ll * gridDim.x) {
         for (int a = 0; a < 3; ++a) {
-            atomicMin(b + a, f2ord(lo[a]));
-            atomicMax(b + 3 + a, f2ord(hi[a]));
+            const float v = p[3 * i + a];
+            lo[a] = fminf(lo[a], v);
+            hi[a] = fmaxf(hi[a], v);
         }
+    }
+    __shared__ float red[6][8];
+    for (int a = 0; a < 3; ++a) {
+        const float l = warp_min(lo[a]), h = warp_max(hi[a]);
+        if ((threadIdx.x & 31) == 0) {
+            red[a][threadIdx.x >> 5] = l;
+            red[3 + a][threadIdx.x >> 5] = h;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        float v = red[threadIdx.x][0];
+        for (int w = 1; w < 8; ++w)
+            v = threadIdx.x < 3 ? fminf(v, red[threadIdx.x][w]) : fmaxf(v, red[threadIdx.x][w]);
+        if (threadIdx.x < 3) atomicMin(b + threadIdx.x, f2ord(v));
+        else atomicMax(b + threadIdx.x, f2ord(v));
     }
 }
 
-__device__ __forceinline__ unsigned spread10(unsigned v) {
-    v &= 0x3ffu;
-    v = (v | (v << 16)) & 0x030000ffu;
-    v = (v | (v << 8)) & 0x0300f00fu;
-    v = (v | (v << 4)) & 0x030c30c3u;
-    v = (v | (v << 2)) & 0x09249249u;
+// Spread the low 16 bits of v so that bit i lands at bit 3i.
+__device__ __forceinline__ unsigned long long spread16(unsigned long long v) {
+    v = (v | (v << 32)) & 0x1f00000000ffffull;
+    v = (v | (v << 16)) & 0x1f0000ff0000ffull;
+    v = (v | (v << 8)) & 0x100f00f00f00f00full;
+    v = (v | (v << 4)) & 0x10c30c30c30c30c3ull;
+    v = (v | (v << 2)) & 0x1249249249249249ull;
     return v;
 }
 
 __global__ void __launch_bounds__(256) k_knn_morton(long long n, const float* __restrict__ p,
-                                                    const int* __restrict__ b, unsigned* __restrict__ keys,
+                                                    const int* __restrict__ b, unsigned long long* __restrict__ keys,
                                                     int* __restrict__ vals) {
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
+    constexpr float top = (float)((1 << kMortonBits) - 1);
     unsigned q[3];
     for (int a = 0; a < 3; ++a) {
         const float lo = ord2f(b[a]), hi = ord2f(b[3 + a]);
         const float u = hi > lo ? (p[3 * i + a] - lo) / (hi - lo) : 0.f;
-        q[a] = (unsigned)fminf(fmaxf(u * 1023.f, 0.f), 1023.f);
+        q[a] = (unsigned)fminf(fmaxf(u * top, 0.f), top);
     }
-    keys[i] = spread10(q[0]) | (spread10(q[1]) << 1) | (spread10(q[2]) << 2);
+    keys[i] = spread16(q[0]) | (spread16(q[1]) << 1) | (spread16(q[2]) << 2);
     vals[i] = (int)i;
 }
 
-__global__ void __launch_bounds__(kBox) k_knn_boxes(long long n, const float* __restrict__ p,
-                                                    const int* __restrict__ sorted, float4* __restrict__ blo,
-                                                    float4* __restrict__ bhi) {
-    const long long i = (long long)blockIdx.x * kBox + threadIdx.x;
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    if (i < n) {
-        const long long s = sorted[i];
-        for (int a = 0; a < 3; ++a) lo[a] = hi[a] = p[3 * s + a];
-    }
-    __shared__ float red[2][3][kBox / 32];
-    for (int a = 0; a < 3; ++a) {
-        for (int o = 16; o; o >>= 1) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-        }
-        if ((threadIdx.x & 31) == 0) {
-            red[0][a][threadIdx.x >> 5] = lo[a];
-            red[1][a][threadIdx.x >> 5] = hi[a];
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float l[3], h[3];
-        for (int a = 0; a < 3; ++a) {
-            l[a] = red[0][a][0];
-            h[a] = red[1][a][0];
-            for (int w = 1; w < kBox / 32; ++w) {
-                l[a] = fminf(l[a], red[0][a][w]);
-                h[a] = fmaxf(h[a], red[1][a][w]);
+// A block per group: its points in sorted order, its boxes (a warp per box, four in turn) and their union.
+__global__ void __launch_bounds__(256) k_knn_boxes(long long n, const float* __restrict__ p,
+                                                   const int* __restrict__ sorted, float4* __restrict__ pts,
+                                                   float4* __restrict__ blo, float4* __restrict__ bhi,
+                                                   float4* __restrict__ glo, float4* __restrict__ ghi) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float g[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    for (int j = warp; j < kGroup; j += 8) {
+        const long long bx = (long long)blockIdx.x * kGroup + j;
+        if (bx * kBox >= n) break;
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        const long long i = bx * kBox + lane;
+        if (i < n) {
+            const long long s = sorted[i];
+            const float x[3] = {p[3 * s], p[3 * s + 1], p[3 * s + 2]};
+            pts[i] = make_float4(x[0], x[1], x[2], 0.f);
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = fminf(lo[a], x[a]);
+                hi[a] = fmaxf(hi[a], x[a]);
             }
         }
-        blo[blockIdx.x] = make_float4(l[0], l[1], l[2], 0.f);
-        bhi[blockIdx.x] = make_float4(h[0], h[1], h[2], 0.f);
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = warp_min(lo[a]);
+            hi[a] = warp_max(hi[a]);
+            g[a] = fminf(g[a], lo[a]);
+            g[3 + a] = fmaxf(g[3 + a], hi[a]);
+        }
+        if (lane == 0) {
+            blo[bx] = make_float4(lo[0], lo[1], lo[2], 0.f);
+            bhi[bx] = make_float4(hi[0], hi[1], hi[2], 0.f);
+        }
+    }
+    __shared__ float red[6][8];
+    if (lane == 0)
+        for (int a = 0; a < 6; ++a) red[a][warp] = g[a];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w)
+            for (int a = 0; a < 6; ++a) g[a] = a < 3 ? fminf(g[a], red[a][w]) : fmaxf(g[a], red[a][w]);
+        glo[blockIdx.x] = make_float4(g[0], g[1], g[2], 0.f);
+        ghi[blockIdx.x] = make_float4(g[3], g[4], g[5], 0.f);
     }
 }
 
@@ -167,94 +217,104 @@ __device__ __forceinline__ void insert3(float d, float (&best)[3]) {
     }
 }
 
-// The distances from this lane's query to the kBox points of box `bx` (two loaded per lane,
-// broadcast by shuffle).
-__device__ __forceinline__ void scan_box(long long n, const float* __restrict__ p, const int* __restrict__ sorted,
-                                         long long bx, long long me, float3 q, bool active, float (&best)[3],
-                                         int lane) {
-    float3 v[2];
-    long long idx[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        idx[h] = bx * kBox + h * 32 + lane;
-        if (idx[h] < n) {
-            const long long s = sorted[idx[h]];
-            v[h] = make_float3(p[3 * s], p[3 * s + 1], p[3 * s + 2]);
-        } else {
-            v[h] = make_float3(0.f, 0.f, 0.f);
-        }
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const long long base = bx * kBox + h * 32;
-        const int m = (int)min(32ll, n - base);
-        for (int j = 0; j < m; ++j) {
-            const float px = __shfl_sync(0xffffffffu, v[h].x, j);
-            const float py = __shfl_sync(0xffffffffu, v[h].y, j);
-            const float pz = __shfl_sync(0xffffffffu, v[h].z, j);
-            if (active && base + j != me) {
-                const float dx = px - q.x, dy = py - q.y, dz = pz - q.z;
-                insert3(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))), best);
-            }
-        }
+// The distances from this lane's query to the kBox points of box `bx`, staged in `stage` (the end of
+// the last box at infinity).
+__device__ __forceinline__ void scan_box(long long n, const float4* __restrict__ pts, float4* stage, long long bx,
+                                         long long me, float3 q, float (&best)[3], int lane) {
+    __syncwarp();
+    const long long i = bx * kBox + lane;
+    stage[lane] = i < n ? pts[i] : make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+    __syncwarp();
+    const long long self = me - bx * kBox;            // this lane's own point, when it is in the box
+#pragma unroll 8
+    for (int j = 0; j < kBox; ++j) {
+        const float4 v = stage[j];
+        const float dx = v.x - q.x, dy = v.y - q.y, dz = v.z - q.z;
+        const float d = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+        if (d < best[2] && j != self) insert3(d, best);
     }
 }
 
-__global__ void __launch_bounds__(128) k_knn_query(long long n, const float* __restrict__ p,
+// Squared gap between two boxes, a little less than it is (a relative margin keeps its rounding from
+// dropping a point at the tie distance).
+__device__ __forceinline__ float gap2(float4 l, float4 h, const float (&ql)[3], const float (&qh)[3]) {
+    const float gx = fmaxf(0.f, fmaxf(l.x - qh[0], ql[0] - h.x));
+    const float gy = fmaxf(0.f, fmaxf(l.y - qh[1], ql[1] - h.y));
+    const float gz = fmaxf(0.f, fmaxf(l.z - qh[2], ql[2] - h.z));
+    return __fmul_rn(gx * gx + gy * gy + gz * gz, 0.999999f);
+}
+
+__global__ void __launch_bounds__(128) k_knn_query(long long n, const float4* __restrict__ pts,
                                                    const int* __restrict__ sorted, const float4* __restrict__ blo,
-                                                   const float4* __restrict__ bhi, float* __restrict__ out) {
+                                                   const float4* __restrict__ bhi, const float4* __restrict__ glo,
+                                                   const float4* __restrict__ ghi, float* __restrict__ out) {
+    __shared__ float4 stage_all[4][kBox];
+    float4* const stage = stage_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long me = warp * 32 + lane;
     if (warp * 32 >= n) return;                       // whole warp past the end
     const bool active = me < n;
-    const long long nb = (n + kBox - 1) / kBox;
+    const long long nb = (n + kBox - 1) / kBox, ng = (nb + kGroup - 1) / kGroup;
     float3 q = make_float3(0.f, 0.f, 0.f);
     if (active) {
-        const long long s = sorted[me];
-        q = make_float3(p[3 * s], p[3 * s + 1], p[3 * s + 2]);
+        const float4 v = pts[me];
+        q = make_float3(v.x, v.y, v.z);
     }
     // the warp's query box
     float ql[3] = {active ? q.x : INFINITY, active ? q.y : INFINITY, active ? q.z : INFINITY};
     float qh[3] = {active ? q.x : -INFINITY, active ? q.y : -INFINITY, active ? q.z : -INFINITY};
+    const float own_lo[3] = {q.x, q.y, q.z};
     for (int a = 0; a < 3; ++a) {
-        for (int o = 16; o; o >>= 1) {
-            ql[a] = fminf(ql[a], __shfl_xor_sync(0xffffffffu, ql[a], o));
-            qh[a] = fmaxf(qh[a], __shfl_xor_sync(0xffffffffu, qh[a], o));
-        }
+        ql[a] = warp_min(ql[a]);
+        qh[a] = warp_max(qh[a]);
     }
     float best[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
-    const long long own = (warp * 32) / kBox;
+    const long long own = warp;
     const long long n0 = own - kNear > 0 ? own - kNear : 0;
     const long long n1 = own + kNear < nb - 1 ? own + kNear : nb - 1;
-    for (long long bx = n0; bx <= n1; ++bx) scan_box(n, p, sorted, bx, me, q, active, best, lane);
-    // every other box within the warp's largest third-best distance of the query box
-    for (long long b0 = 0; b0 < nb; b0 += 32) {
-        const unsigned lim = __reduce_max_sync(0xffffffffu, active ? __float_as_uint(best[2]) : 0u);
-        const float limf = __uint_as_float(lim);
-        const long long bx = b0 + lane;
-        bool need = false;
-        if (bx < nb && (bx < n0 || bx > n1)) {
-            const float4 l = blo[bx], h = bhi[bx];
-            const float gx = fmaxf(0.f, fmaxf(l.x - qh[0], ql[0] - h.x));
-            const float gy = fmaxf(0.f, fmaxf(l.y - qh[1], ql[1] - h.y));
-            const float gz = fmaxf(0.f, fmaxf(l.z - qh[2], ql[2] - h.z));
-            // skipped only when clearly farther than every lane's third best (a relative margin
-            // keeps rounding of the gap from dropping a point at the tie distance)
-            need = !(__fmul_rn(gx * gx + gy * gy + gz * gz, 0.999999f) > limf);
+    for (long long bx = n0; bx <= n1; ++bx) scan_box(n, pts, stage, bx, me, q, best, lane);
+    // Every other box within the warp's largest third-best distance of the query box, nearest first: a
+    // box (or a group) is left out only when clearly farther than every lane's third best.
+    auto reach = [&]() {
+        return __uint_as_float(__reduce_max_sync(0xffffffffu, active ? __float_as_uint(best[2]) : 0u));
+    };
+    // calls visit(lane) for the lanes' candidates by increasing gap, as far as the reach of the moment goes
+    auto nearest_first = [&](bool in, float gap, auto visit) {
+        unsigned key = in ? __float_as_uint(gap) : 0xffffffffu;
+        while (true) {
+            const unsigned k = __reduce_min_sync(0xffffffffu, key);
+            if (k == 0xffffffffu || __uint_as_float(k) > reach()) break;
+            const int j = __ffs(__ballot_sync(0xffffffffu, key == k)) - 1;
+            if (lane == j) key = 0xffffffffu;
+            visit(j);
         }
-        unsigned m = __ballot_sync(0xffffffffu, need);
-        while (m) {
-            const int j = __ffs(m) - 1;
-            m &= m - 1;
-            // the box passed the warp test; scan it only when some lane's own point is close enough
-            const float4 l = blo[b0 + j], h = bhi[b0 + j];
-            const float gx = fmaxf(0.f, fmaxf(l.x - q.x, q.x - h.x));
-            const float gy = fmaxf(0.f, fmaxf(l.y - q.y, q.y - h.y));
-            const float gz = fmaxf(0.f, fmaxf(l.z - q.z, q.z - h.z));
-            const bool mine = active && !(__fmul_rn(gx * gx + gy * gy + gz * gz, 0.999999f) > best[2]);
-            if (__any_sync(0xffffffffu, mine)) scan_box(n, p, sorted, b0 + j, me, q, active, best, lane);
-        }
+    };
+    // whether some lane's own point is close enough to a box: the query box of a warp whose points straddle
+    // a jump of the Morton curve can hold half the scene
+    auto wanted = [&](float4 l, float4 h) {
+        return __any_sync(0xffffffffu, active && !(gap2(l, h, own_lo, own_lo) > best[2]));
+    };
+    auto visit_group = [&](long long g) {
+        if (!wanted(glo[g], ghi[g])) return;
+        const long long b0 = g * kGroup, bx = b0 + lane;
+        const bool in = bx < nb && (bx < n0 || bx > n1);
+        const float4 l = in ? blo[bx] : make_float4(0.f, 0.f, 0.f, 0.f), h = in ? bhi[bx] : l;
+        nearest_first(in, gap2(l, h, ql, qh), [&](int j) {
+            if (wanted(blo[b0 + j], bhi[b0 + j])) scan_box(n, pts, stage, b0 + j, me, q, best, lane);
+        });
+    };
+    // the warp's own group, then 32 groups at a time outwards from it
+    const long long own_g = own / kGroup, nc = (ng + 31) / 32, own_c = own_g / 32;
+    const long long far_c = own_c > nc - 1 - own_c ? own_c : nc - 1 - own_c;
+    visit_group(own_g);
+    for (long long k = 0; k <= 2 * far_c; ++k) {
+        const long long c = k & 1 ? own_c + (k + 1) / 2 : own_c - k / 2;
+        if (c < 0 || c >= nc) continue;
+        const long long g = c * 32 + lane;
+        const bool in = g < ng && g != own_g;
+        const float4 l = in ? glo[g] : make_float4(0.f, 0.f, 0.f, 0.f), h = in ? ghi[g] : l;
+        nearest_first(in, gap2(l, h, ql, qh), [&](int j) { visit_group(c * 32 + j); });
     }
     if (active) out[sorted[me]] = __fdiv_rn(__fadd_rn(__fadd_rn(best[0], best[1]), best[2]), 3.0f);
 }
@@ -276,16 +336,17 @@ int rg_knn_mean_dist(const float* points, int64_t n, float* mean_dist, void* wor
     KnnWs w = carve(workspace, n);
     const unsigned blocks = (unsigned)((n + 255) / 256);
     k_knn_init_bounds<<<1, 32, 0, s>>>(w.bounds);
-    k_knn_bounds<<<blocks, 256, 0, s>>>(n, points, w.bounds);
+    k_knn_bounds<<<blocks < 592u ? blocks : 592u, 256, 0, s>>>(n, points, w.bounds);
     k_knn_morton<<<blocks, 256, 0, s>>>(n, points, w.bounds, w.keys_in, w.vals_in);
     size_t bytes = w.sort_bytes;
     if (cub::DeviceRadixSort::SortPairs(w.sort_temp, bytes, w.keys_in, w.keys_out, w.vals_in, w.vals_out, (int)n, 0,
-                                        30, s) != cudaSuccess)
+                                        3 * kMortonBits, s) != cudaSuccess)
         return RG_ERR_CUDA;
-    const long long nb = (n + kBox - 1) / kBox;
-    k_knn_boxes<<<(unsigned)nb, kBox, 0, s>>>(n, points, w.vals_out, w.box_lo, w.box_hi);
+    k_knn_boxes<<<(unsigned)n_groups(n), 256, 0, s>>>(n, points, w.vals_out, w.pts, w.box_lo, w.box_hi, w.group_lo,
+                                                      w.group_hi);
     const long long warps = (n + 31) / 32;
-    k_knn_query<<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(n, points, w.vals_out, w.box_lo, w.box_hi, mean_dist);
+    k_knn_query<<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(n, w.pts, w.vals_out, w.box_lo, w.box_hi, w.group_lo,
+                                                            w.group_hi, mean_dist);
     return cudaGetLastError() == cudaSuccess ? RG_OK : RG_ERR_CUDA;
 }
 
