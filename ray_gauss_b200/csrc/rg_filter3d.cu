@@ -49,15 +49,17 @@ __global__ void __launch_bounds__(kFilterThreads) k_filter_depth(long long n, co
             for (int c = 0; c < nc; ++c) {
                 const float* k = cs + c * kCamFloats;
                 // xyz_cam = xyz @ R + T (row vector times R)
+                const float zr = __fadd_rn(__fmaf_rn(pz, k[8], __fmaf_rn(py, k[5], __fmul_rn(px, k[2]))), k[11]);
+                if (!(zr > 0.2f)) continue;
+                const float z = fmaxf(zr, 0.001f);
+                // a camera that is no nearer than one that sees the Gaussian already changes nothing: its
+                // window, two divisions, is not needed (100 cameras around a scene: one in five is)
+                if (seen && !(z < dist)) continue;
                 const float x = __fadd_rn(__fmaf_rn(pz, k[6], __fmaf_rn(py, k[3], __fmul_rn(px, k[0]))), k[9]);
                 const float y = __fadd_rn(__fmaf_rn(pz, k[7], __fmaf_rn(py, k[4], __fmul_rn(px, k[1]))), k[10]);
-                const float zr = __fadd_rn(__fmaf_rn(pz, k[8], __fmaf_rn(py, k[5], __fmul_rn(px, k[2]))), k[11]);
-                const bool front = zr > 0.2f;
-                const float z = fmaxf(zr, 0.001f);
                 const float sx = __fadd_rn(__fmul_rn(__fdiv_rn(x, z), k[12]), k[14]);
                 const float sy = __fadd_rn(__fmul_rn(__fdiv_rn(y, z), k[13]), k[15]);
-                const bool inside = sx >= k[16] && sx <= k[17] && sy >= k[18] && sy <= k[19];
-                if (front && inside) {
+                if (sx >= k[16] && sx <= k[17] && sy >= k[18] && sy <= k[19]) {
                     dist = fminf(dist, z);
                     seen = true;
                 }

@@ -28,21 +28,35 @@ def fov2focal(fov, pixels):
 def camera_table(cameras):
     """(n_cams, 20) float32 rows of rg_filter_camera and the largest focal length (a Python float,
     compared in double like the reference's loop)."""
-    rows, focal = [], 0.0
+    cameras = list(cameras)
+    if not cameras:
+        return np.zeros((0, 20), np.float32), 0.0
+    wvts = [cam.world_view_transform for cam in cameras]
+    try:
+        # one stack and one copy to the host for all cameras (each copy of its own costs a synchronisation)
+        wvt = torch.stack(wvts).detach().to("cpu", torch.float32).numpy()
+    except RuntimeError:      # matrices of several devices or shapes
+        wvt = np.stack([w.detach().to("cpu", torch.float32).numpy()[:4, :3] for w in wvts])
+    known = {}                # most cameras share their field of view and size
+    focals = []
     for cam in cameras:
-        wvt = cam.world_view_transform.detach().to("cpu", torch.float32).numpy()
-        W, H = cam.image_width, cam.image_height
-        fx, fy = fov2focal(cam.FoVx, W), fov2focal(cam.FoVy, H)
-        row = np.empty(20, np.float32)
-        row[0:9] = wvt[:3, :3].reshape(-1)
-        row[9:12] = wvt[3, :3]
-        row[12:20] = [fx, fy, W / 2.0, H / 2.0, -0.15 * W, W * 1.15, -0.15 * H, 1.15 * H]
-        rows.append(row)
-        if focal < fx:
-            focal = fx
-        if focal < fy:
-            focal = fy
-    return np.stack(rows) if rows else np.zeros((0, 20), np.float32), focal
+        key = (cam.FoVx, cam.FoVy, cam.image_width, cam.image_height)
+        f = known.get(key)
+        if f is None:
+            f = known[key] = (fov2focal(key[0], key[2]), fov2focal(key[1], key[3]), key[2], key[3])
+        focals.append(f)
+    fx, fy, W, H = np.array(focals, np.float64).T
+    table = np.empty((len(cameras), 20), np.float32)
+    table[:, 0:9] = wvt[:, :3, :3].reshape(-1, 9)
+    table[:, 9:12] = wvt[:, 3, :3]
+    for i, col in enumerate((fx, fy, W / 2.0, H / 2.0, -0.15 * W, W * 1.15, -0.15 * H, 1.15 * H)):
+        table[:, 12 + i] = col
+    focal = 0.0
+    for f in known.values():
+        for v in f[:2]:
+            if focal < v:
+                focal = v
+    return table, focal
 
 
 def compute_3D_filter(positions: torch.Tensor, cameras) -> torch.Tensor:
