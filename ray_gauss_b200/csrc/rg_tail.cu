@@ -13,11 +13,15 @@
 // Adam per element, as torch.optim.Adam:  m += (1 - beta1) (g - m);  v = beta2 v + (1 - beta2) g^2;
 // p -= (lr / (1 - beta1^t)) * m / (sqrt(v) / sqrt(1 - beta2^t) + eps).
 //
-// Layout: a block owns kTailGaussians consecutive Gaussians.  For each tensor it streams the block's
-// contiguous element range [g0 * width, g1 * width) with coalesced float4 accesses (scalar when a
-// pointer is not 16-byte aligned), then, after a block barrier, one thread per Gaussian applies the
-// statistics and the clamps to the values the block has just written.  Every byte is read and
-// written once: HBM-bound at 28 bytes per parameter float (param, m, v read and written, grad read).
+// Layout: k_tail_stream gives every tensor blocks of its own.  A thread takes whole rows with float4
+// accesses: a quaternion, four positions or lobe axes (12 floats), or four elements of a tensor whose
+// clamp is elementwise, so the clamp and the statistics work on the values in registers.  Every byte is
+// read and written once: HBM-bound at 28 bytes per parameter float (param, m, v read and written, grad
+// read).  1M Gaussians, 115 floats each, 3.25 GB: 548 us (91 % of a copy's rate), against 805 us when a block took 256
+// Gaussians through all tensors in turn (few loads in flight at a time, threads idle at the narrow
+// tensors, the clamps on parameters read again behind a barrier).  That form, k_train_tail, still does
+// what has no 16-byte alignment, and the last n % 4 Gaussians.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -76,23 +80,163 @@ __device__ void adam_range(const rg_adam_tensor& t, const AdamStep& s, long long
     }
 }
 
-__global__ void __launch_bounds__(kTailThreads) k_train_tail(const TailArgs args) {
+// The step of tensor i (false: it does not step).
+__device__ __forceinline__ bool adam_step(const rg_train_tail& d, int i, AdamStep& s) {
+    const rg_adam_tensor& t = d.tensors[i];
+    if (!t.active || !t.grad || !t.param || t.width <= 0) return false;
+    float lr = t.lr, bias1 = t.bias1, bias2_sqrt = t.bias2_sqrt;
+    if (d.step_scalars) {
+        const float* sc = d.step_scalars + 4 * i;
+        if (sc[0] == 0.f) return false;
+        lr = sc[1];
+        bias1 = sc[2];
+        bias2_sqrt = sc[3];
+    }
+    s = AdamStep{t.one_minus_beta1, t.one_minus_beta2, t.beta2, t.eps, lr / bias1, bias2_sqrt};
+    return true;
+}
+
+// Densification statistics of Gaussian g from its position gradient.
+__device__ __forceinline__ void tail_stats(const rg_train_tail& d, long long g, float gx, float gy, float gz) {
+    const float gn = sqrtf(gx * gx + gy * gy + gz * gz);
+    if (d.grad_norm_accum) d.grad_norm_accum[g] += gn;
+    if (d.num_accum && gn > 0.f) d.num_accum[g] += 1.f;
+    if (d.num_accum_gnv && gn > 0.f) d.num_accum_gnv[g] += 1.f;
+}
+__device__ __forceinline__ float4 unit_quaternion(float4 q) {
+    float nn = sqrtf(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w);
+    if (nn == 0.f) { q = make_float4(1.f, 0.f, 0.f, 0.f); nn = 1.f; }
+    return make_float4(q.x / nn, q.y / nn, q.z / nn, q.w / nn);
+}
+__device__ __forceinline__ void unit_axis(float* ax) {
+    float nn = sqrtf(ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2]);
+    if (nn == 0.f) { ax[0] = 0.f; ax[1] = 0.f; ax[2] = 1.f; nn = 1.f; }
+    for (int k = 0; k < 3; ++k) ax[k] /= nn;
+}
+__device__ __forceinline__ float clamp_scale(const rg_train_tail& d, float v, long long g) {
+    const float lo = d.min_scale ? d.min_scale[g] : -INFINITY;
+    if (v < lo) v = lo;
+    if (v > d.max_scale) v = d.max_scale;
+    return v;
+}
+
+// Blocks of the tensors: those of segment k end at block_end[k].
+struct TailSegments {
+    int count, iters;
+    int tensor[kTailMaxTensors];
+    unsigned block_end[kTailMaxTensors];
+};
+// float4 units of a thread at a time (loads first), and at most so many such steps of a block: 598 us with
+// 2 x 4, 564 with 2 x 8, 548 with 4 x 4, 949 with 1 x 1 (short blocks), 1M Gaussians.  Fewer steps where
+// they would leave the chip without four blocks per SM.
+constexpr int kTailUnroll = 4, kTailMaxIters = 4;
+
+// NV float4 of a tensor, `stride` float4 apart from number `first` on, those before `end`: stepped when
+// `steps`, then clamped by f(values of one, its number).  All loads come first.
+template <int NV, typename F>
+__device__ __forceinline__ void tail_unit(const rg_adam_tensor& t, const AdamStep& s, bool steps, long long first, int stride,
+                                          long long end, F f) {
+    float4 p[NV], g[NV], m[NV], v[NV];
+    float4* const P = reinterpret_cast<float4*>(t.param) + first;
+    const float4* const G = reinterpret_cast<const float4*>(t.grad) + first;
+    float4* const M = reinterpret_cast<float4*>(t.exp_avg) + first;
+    float4* const V = reinterpret_cast<float4*>(t.exp_avg_sq) + first;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        if (first + k * stride >= end) continue;
+        p[k] = __ldcs(P + k * stride);
+        if (steps) {
+            g[k] = __ldcs(G + k * stride);
+            m[k] = __ldcs(M + k * stride);
+            v[k] = __ldcs(V + k * stride);
+        }
+    }
+    if (steps) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            if (first + k * stride >= end) continue;
+            adam1(p[k].x, g[k].x, m[k].x, v[k].x, s);
+            adam1(p[k].y, g[k].y, m[k].y, v[k].y, s);
+            adam1(p[k].z, g[k].z, m[k].z, v[k].z, s);
+            adam1(p[k].w, g[k].w, m[k].w, v[k].w, s);
+            __stcs(M + k * stride, m[k]);
+            __stcs(V + k * stride, v[k]);
+        }
+    }
+    f(p);
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+        if (first + k * stride < end) __stcs(P + k * stride, p[k]);
+}
+
+// Gaussians [0, n4), n4 a multiple of 4; every tensor 16-byte aligned.
+__global__ void __launch_bounds__(kTailThreads) k_tail_stream(const TailArgs args, const TailSegments seg, long long n4) {
     const rg_train_tail& d = args.d;
-    const long long g0 = (long long)blockIdx.x * kTailGaussians;
+    int k = 0;
+    while (blockIdx.x >= seg.block_end[k]) ++k;
+    const int i = seg.tensor[k];
+    const rg_adam_tensor& t = d.tensors[i];
+    const long long block = blockIdx.x - (k ? seg.block_end[k - 1] : 0u);
+    AdamStep s;
+    const bool steps = adam_step(d, i, s);
+    const bool stats = i == d.idx_positions && t.grad && (d.grad_norm_accum || d.num_accum || d.num_accum_gnv);
+    const bool axis = i == d.idx_lobe_axis && d.normalize_lobe_axis;
+    if (stats || axis) {
+#pragma unroll 1
+        for (int it = 0; it < seg.iters; ++it) {
+            const long long u = (block * seg.iters + it) * kTailThreads + threadIdx.x;
+            if (u >= n4 * t.width / 12) return;
+            if (stats) {
+                const float4* G = reinterpret_cast<const float4*>(t.grad) + 3 * u;
+                const float4 a = G[0], b = G[1], c = G[2];
+                tail_stats(d, 4 * u, a.x, a.y, a.z);
+                tail_stats(d, 4 * u + 1, a.w, b.x, b.y);
+                tail_stats(d, 4 * u + 2, b.z, b.w, c.x);
+                tail_stats(d, 4 * u + 3, c.y, c.z, c.w);
+            }
+            if (steps || axis)
+                tail_unit<3>(t, s, steps, 3 * u, 1, 3 * u + 3, [&](float4* p) {
+                    if (axis)
+                        for (int j = 0; j < 4; ++j) unit_axis(reinterpret_cast<float*>(p) + 3 * j);
+                });
+        }
+        return;
+    }
+    const bool dens = i == d.idx_densities, quat = i == d.idx_quaternions && d.normalize_quaternions,
+               scale = i == d.idx_scales;
+    if (!steps && !dens && !quat && !scale) return;
+    const long long units = n4 * t.width / 4;
+#pragma unroll 1
+    for (int it = 0; it < seg.iters; ++it) {
+        const long long first = (block * seg.iters + it) * kTailUnroll * kTailThreads + threadIdx.x;
+        if (first >= units) return;
+        tail_unit<kTailUnroll>(t, s, steps, first, kTailThreads, units, [&](float4* p) {
+#pragma unroll
+            for (int k = 0; k < kTailUnroll; ++k) {
+                float* const e = reinterpret_cast<float*>(p + k);
+                const long long at = 4 * (first + k * kTailThreads);
+                if (at >= 4 * units) continue;
+                if (dens) {
+                    for (int c = 0; c < 4; ++c)
+                        if (e[c] < 0.f) e[c] = 0.f;
+                } else if (quat) {
+                    p[k] = unit_quaternion(p[k]);
+                } else if (scale) {
+                    for (int c = 0; c < 4; ++c) e[c] = clamp_scale(d, e[c], (at + c) / 3);
+                }
+            }
+        });
+    }
+}
+
+// The Gaussians from `first`.
+__global__ void __launch_bounds__(kTailThreads) k_train_tail(const TailArgs args, long long first) {
+    const rg_train_tail& d = args.d;
+    const long long g0 = first + (long long)blockIdx.x * kTailGaussians;
     const long long g1 = g0 + kTailGaussians < d.n ? g0 + kTailGaussians : d.n;
     for (int i = 0; i < d.n_tensors && i < kTailMaxTensors; ++i) {
-        const rg_adam_tensor& t = d.tensors[i];
-        if (!t.active || !t.grad || !t.param || t.width <= 0) continue;
-        float lr = t.lr, bias1 = t.bias1, bias2_sqrt = t.bias2_sqrt;
-        if (d.step_scalars) {
-            const float* sc = d.step_scalars + 4 * i;
-            if (sc[0] == 0.f) continue;
-            lr = sc[1];
-            bias1 = sc[2];
-            bias2_sqrt = sc[3];
-        }
-        const AdamStep s{t.one_minus_beta1, t.one_minus_beta2, t.beta2, t.eps, lr / bias1, bias2_sqrt};
-        adam_range(t, s, g0 * t.width, g1 * t.width);
+        AdamStep s;
+        if (adam_step(d, i, s)) adam_range(d.tensors[i], s, g0 * d.tensors[i].width, g1 * d.tensors[i].width);
     }
     __syncthreads();  // the clamps below read parameters that other threads of the block stepped
     const long long g = g0 + threadIdx.x;
@@ -101,10 +245,7 @@ __global__ void __launch_bounds__(kTailThreads) k_train_tail(const TailArgs args
     if (d.idx_positions >= 0 && d.tensors[d.idx_positions].grad &&
         (d.grad_norm_accum || d.num_accum || d.num_accum_gnv)) {
         const float* gp = d.tensors[d.idx_positions].grad + 3 * g;
-        const float gn = sqrtf(gp[0] * gp[0] + gp[1] * gp[1] + gp[2] * gp[2]);
-        if (d.grad_norm_accum) d.grad_norm_accum[g] += gn;
-        if (d.num_accum && gn > 0.f) d.num_accum[g] += 1.f;
-        if (d.num_accum_gnv && gn > 0.f) d.num_accum_gnv[g] += 1.f;
+        tail_stats(d, g, gp[0], gp[1], gp[2]);
     }
     // clamps after the step
     if (d.idx_densities >= 0) {
@@ -113,29 +254,15 @@ __global__ void __launch_bounds__(kTailThreads) k_train_tail(const TailArgs args
     }
     if (d.normalize_quaternions && d.idx_quaternions >= 0) {
         float4* qp = reinterpret_cast<float4*>(d.tensors[d.idx_quaternions].param) + g;
-        float4 q = *qp;
-        float nn = sqrtf(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w);
-        if (nn == 0.f) { q = make_float4(1.f, 0.f, 0.f, 0.f); nn = 1.f; }
-        *qp = make_float4(q.x / nn, q.y / nn, q.z / nn, q.w / nn);
+        *qp = unit_quaternion(*qp);
     }
     if (d.normalize_lobe_axis && d.idx_lobe_axis >= 0 && d.tensors[d.idx_lobe_axis].width > 0) {
         const rg_adam_tensor& t = d.tensors[d.idx_lobe_axis];
-        for (int l = 0; l < t.width / 3; ++l) {
-            float* ax = t.param + g * t.width + 3 * l;
-            float nn = sqrtf(ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2]);
-            if (nn == 0.f) { ax[0] = 0.f; ax[1] = 0.f; ax[2] = 1.f; nn = 1.f; }
-            for (int k = 0; k < 3; ++k) ax[k] /= nn;
-        }
+        for (int l = 0; l < t.width / 3; ++l) unit_axis(t.param + g * t.width + 3 * l);
     }
     if (d.idx_scales >= 0) {
         float* s = d.tensors[d.idx_scales].param + 3 * g;
-        const float lo = d.min_scale ? d.min_scale[g] : -INFINITY;
-        for (int k = 0; k < 3; ++k) {
-            float v = s[k];
-            if (v < lo) v = lo;
-            if (v > d.max_scale) v = d.max_scale;
-            s[k] = v;
-        }
+        for (int k = 0; k < 3; ++k) s[k] = clamp_scale(d, s[k], g);
     }
 }
 
@@ -176,8 +303,29 @@ int rg_train_tail_step(const rg_train_tail* d, void* stream) {
     if (d->n == 0) return RG_OK;
     TailArgs a;
     std::memcpy(&a.d, d, sizeof(rg_train_tail));
-    const long long blocks = (d->n + kTailGaussians - 1) / kTailGaussians;
-    k_train_tail<<<(unsigned)blocks, kTailThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(a);
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    // the streaming form takes every tensor that steps, is clamped or gives the statistics
+    TailSegments seg{};
+    long long n4 = d->n & ~3ll, blocks = 0, floats_all = 0;
+    for (int i = 0; i < d->n_tensors; ++i) floats_all += n4 * d->tensors[i].width;
+    seg.iters = (int)std::min<long long>(kTailMaxIters, std::max(1ll, floats_all / (4ll * kTailThreads * kTailUnroll * 592)));
+    for (int i = 0; i < d->n_tensors && n4; ++i) {
+        const rg_adam_tensor& t = d->tensors[i];
+        if (!t.param || t.width <= 0) continue;
+        if (((uintptr_t)t.param | (uintptr_t)t.grad | (uintptr_t)t.exp_avg | (uintptr_t)t.exp_avg_sq) & 15) n4 = 0;
+        // a thread takes 12 floats where k_tail_stream works on rows of 3, else kTailUnroll float4
+        const bool rows = (i == d->idx_positions && t.grad && (d->grad_norm_accum || d->num_accum || d->num_accum_gnv)) ||
+                          (i == d->idx_lobe_axis && d->normalize_lobe_axis);
+        const long long per_block = kTailThreads * seg.iters * (rows ? 12ll : 4ll * kTailUnroll);
+        const long long floats = n4 * t.width;
+        blocks += (floats + per_block - 1) / per_block;
+        seg.tensor[seg.count] = i;
+        seg.block_end[seg.count++] = (unsigned)blocks;
+    }
+    if (blocks > 0x7fffffffll) n4 = 0;
+    if (n4) k_tail_stream<<<(unsigned)blocks, kTailThreads, 0, st>>>(a, seg, n4);
+    if (n4 < d->n)
+        k_train_tail<<<(unsigned)((d->n - n4 + kTailGaussians - 1) / kTailGaussians), kTailThreads, 0, st>>>(a, n4);
     return cudaGetLastError() == cudaSuccess ? RG_OK : RG_ERR_CUDA;
 }
 
