@@ -235,16 +235,11 @@ __device__ float split_offset(const GatherArgs& a, int s, int copy, int c) {
     return __fmaf_rn(R2, v2, __fmaf_rn(R1, v1, __fmul_rn(R0, v0)));
 }
 
-// One output element of a tensor of kind K: copy, zero, or the role's transform.
-template <int K, typename Idx>
-__device__ __forceinline__ float dens_value(const GatherArgs& a, const rg_densify_tensor& t, Idx e, Idx w) {
-    if (K == RG_DENSIFY_ZERO) return 0.f;
-    const Idx o = e / w;
-    const int c = (int)(e - o * w);
-    const int2 m = a.w.map[o];
-    const long long si = (long long)m.x * w + c;
-    if (K == RG_DENSIFY_OLD_ONLY) return m.y == 0 ? t.src[si] : 0.f;
-    float v = t.src[si];
+// Element c of the output row that comes from m = (source row, kind): copy, zero, or the role's transform.
+template <int K>
+__device__ __forceinline__ float dens_value(const GatherArgs& a, const rg_densify_tensor& t, int2 m, int c) {
+    if (K == RG_DENSIFY_OLD_ONLY && m.y != 0) return 0.f;
+    float v = t.src[(long long)m.x * t.width + c];
     if (K == RG_DENSIFY_DENSITIES) {
         if (m.y != 0 || (a.w.flags[m.x] & F_CLONE)) v = __fmul_rn(v, 0.5f);
     } else if (K == RG_DENSIFY_LOG_SCALES) {
@@ -255,26 +250,49 @@ __device__ __forceinline__ float dens_value(const GatherArgs& a, const rg_densif
     return v;
 }
 
-// Grid-stride over the tensor's output floats, kUnroll independent elements per thread per pass so
-// that several loads are in flight before the first store.
-constexpr int kUnroll = 4;
-
+// Four consecutive output floats from e on: one division and, inside a row, one map entry for the four
+// (with a division and a map entry each the call took 453 us on 300k Gaussians of 115 floats, 328 so).
 template <int K, typename Idx>
-__device__ __forceinline__ void dens_gather_tensor(const GatherArgs& a, const rg_densify_tensor& t) {
-    const Idx w = (Idx)t.width;
-    const Idx total = (Idx)a.n_out * w;
-    const Idx stride = (Idx)gridDim.x * blockDim.x;
-    for (Idx base = (Idx)blockIdx.x * blockDim.x + threadIdx.x; base < total; base += kUnroll * stride) {
-        float v[kUnroll];
-#pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            const Idx e = base + u * stride;
-            v[u] = e < total ? dens_value<K>(a, t, e, w) : 0.f;
+__device__ __forceinline__ float4 dens_quad(const GatherArgs& a, const rg_densify_tensor& t, Idx e, Idx total) {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (K != RG_DENSIFY_ZERO) {
+        const Idx w = (Idx)t.width;
+        Idx o = e / w;
+        int c = (int)(e - o * w);
+        int2 m = a.w.map[o];
+        if ((K == RG_DENSIFY_COPY || K == RG_DENSIFY_OLD_ONLY) && (w & 3) == 0 && ((uintptr_t)t.src & 15) == 0) {
+            if (K == RG_DENSIFY_OLD_ONLY && m.y != 0) return make_float4(0.f, 0.f, 0.f, 0.f);
+            return __ldcs(reinterpret_cast<const float4*>(t.src + (long long)m.x * w + c));
         }
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            const Idx e = base + u * stride;
-            if (e < total) t.dst[e] = v[u];
+        for (int j = 0; j < 4; ++j) {
+            if (e + j >= total) break;
+            v[j] = dens_value<K>(a, t, m, c);
+            if (++c == (int)w) {
+                c = 0;
+                ++o;
+                if (e + j + 1 < total) m = a.w.map[o];
+            }
+        }
+    }
+    return make_float4(v[0], v[1], v[2], v[3]);
+}
+
+// Grid-stride over the tensor's output floats, a quad at a time (two in flight were slower: 359 us a whole
+// call on 300k Gaussians, 328 with one).
+template <int K, typename Idx>
+__device__ __forceinline__ void dens_gather_tensor(const GatherArgs& a, const rg_densify_tensor& t) {
+    const Idx total = (Idx)a.n_out * (Idx)t.width;
+    const Idx stride = 4 * (Idx)gridDim.x * blockDim.x;
+    const bool vec = ((uintptr_t)t.dst & 15) == 0;
+    for (Idx e = 4 * ((Idx)blockIdx.x * blockDim.x + threadIdx.x); e < total; e += stride) {
+        const float4 v = dens_quad<K, Idx>(a, t, e, total);
+        if (vec && e + 4 <= total) {
+            __stcs(reinterpret_cast<float4*>(t.dst + e), v);
+        } else {
+            const float f[4] = {v.x, v.y, v.z, v.w};
+            for (int j = 0; j < 4; ++j)
+                if (e + j < total) t.dst[e + j] = f[j];
         }
     }
 }
@@ -383,10 +401,10 @@ int rg_densify_apply(const rg_densify* d, const float* split_normals, const rg_d
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     long long maxw = 1;
     for (int i = 0; i < n_tensors; ++i) maxw = tensors[i].width > maxw ? tensors[i].width : maxw;
-    long long want = (d->n_out * maxw + 255) / 256;
+    long long want = (d->n_out * maxw + 1023) / 1024;   // blocks of 256 quads
     const long long cap = (long long)sms * 8;
     const unsigned gx = (unsigned)(want < cap ? (want > 0 ? want : 1) : cap);
-    if (d->n_out * maxw + (long long)kUnroll * gx * 256 < (long long)UINT32_MAX)
+    if (d->n_out * maxw + 2048ll * gx < (long long)UINT32_MAX)   // no index above it wraps
         k_dens_gather<unsigned><<<dim3(gx, (unsigned)n_tensors), 256, 0, s>>>(a);
     else
         k_dens_gather<unsigned long long><<<dim3(gx, (unsigned)n_tensors), 256, 0, s>>>(a);
