@@ -39,7 +39,7 @@ struct rg_engine {
     const rg_camera* rec_cams = nullptr;
     int rec_n_cams = 0;
     rg_settings rec_settings{};
-    int rec_split = 1;               // the split of its tiles
+    rg::SplitPair rec_split{1, 1};   // the splits of its tiles
     long long expect_rays = 0;       // rays of the launches that follow (rg_expect_rays; 0: unknown)
     rg_tuning tuning{64, 0, 64, 1, 0};
     unsigned long long launches = 0;
@@ -199,8 +199,8 @@ int kernel_mode(const rg_settings* s) {
 }
 
 // Slabs of a ray side by side: more in launches of fewer rays.
-int launch_split(const rg_engine* e, const rg_settings* s) {
-    return rg::render_split(s->mode, s->rnd_sample, e->tuning.list_capacity, e->n_built, e->expect_rays);
+rg::SplitPair launch_split(const rg_engine* e, const rg_settings* s, int n_views) {
+    return rg::render_split(s->mode, s->rnd_sample, e->tuning.list_capacity, e->n_built, n_views, e->expect_rays);
 }
 
 int render_grid(rg_engine* e, bool bwd, int mode, int split) {
@@ -208,6 +208,20 @@ int render_grid(rg_engine* e, bool bwd, int mode, int split) {
     int occ = rg::render_occupancy(bwd, mode, e->tuning.list_capacity, split);
     if (per_sm <= 0 || per_sm > occ) per_sm = occ > 0 ? occ : 1;
     return e->num_sms * per_sm;
+}
+
+// The render launch after launch_setup_views.  Where the splits differ, both kernels are launched and the
+// one that the scene box did not choose returns at once.
+cudaError_t launch_splits(rg_engine* e, bool bwd, const rg_settings* s, rg::SplitPair split, const rg::RenderArgs& a,
+                          cudaStream_t st) {
+    const int cap = e->tuning.list_capacity, mode = kernel_mode(s);
+    cudaError_t err = rg::launch_render(bwd, s->mode, cap, split.near, render_grid(e, bwd, mode, split.near), a, st);
+    e->launches += 1;
+    if (err == cudaSuccess && split.far != split.near) {
+        err = rg::launch_render(bwd, s->mode, cap, split.far, render_grid(e, bwd, mode, split.far), a, st);
+        e->launches += 1;
+    }
+    return err;
 }
 
 int fill_args(rg_engine* e, const rg_camera* cams, const rg_settings* s, rg::RenderArgs& a) {
@@ -433,8 +447,8 @@ int rg_launch_forward(rg_engine* e, const rg_camera* cams, int32_t n_cams, const
     if (e->n_built <= 0 || e->colors_views < n_cams) return RG_ERR_STATE;
     DeviceScope dev_scope;
     if ((rc = dev_scope.enter(e))) return rc;
-    const int split = launch_split(e, s);
-    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->vt, e->work_counter, S(stream)), "setup views");
+    const rg::SplitPair split = launch_split(e, s, n_cams);
+    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->scene_ord, e->vt, e->work_counter, S(stream)), "setup views");
     rg::RenderArgs a;
     fill_args(e, cams, s, a);
     a.ray_colors = ray_colors;
@@ -447,11 +461,10 @@ int rg_launch_forward(rg_engine* e, const rg_camera* cams, int32_t n_cams, const
         a.rec_top = e->rec_top;
         a.rec_cap = e->rec_cap;
         a.rec_tile = e->rec_tile;
-        a.rec_tiles = (int)record_heads(e->rec_tiles, split);
+        a.rec_tiles = (int)record_heads(e->rec_tiles, std::max(split.near, split.far));
     }
-    int grid = render_grid(e, false, kernel_mode(s), split);
-    RG_CUDA(rg::launch_render(false, s->mode, e->tuning.list_capacity, split, grid, a, S(stream)), "render forward");
-    e->launches += 2;
+    RG_CUDA(launch_splits(e, false, s, split, a, S(stream)), "render forward");
+    e->launches += 1;
     if (record) {
         e->rec_valid = true;
         e->rec_cams = cams;
@@ -474,16 +487,15 @@ int rg_launch_inference(rg_engine* e, const rg_camera* cams, int32_t n_cams, con
     rg_settings si = *s;
     si.jitter = 0;
     si.rnd_sample = 0;
-    const int split = launch_split(e, &si);
-    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->vt, e->work_counter, S(stream)), "setup views");
+    const rg::SplitPair split = launch_split(e, &si, n_cams);
+    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->scene_ord, e->vt, e->work_counter, S(stream)), "setup views");
     rg::RenderArgs a;
     fill_args(e, cams, &si, a);
     a.ray_colors = ray_colors;
     a.infer = 1;
     a.counts = gaussians_per_ray;
-    int grid = render_grid(e, false, kernel_mode(&si), split);
-    RG_CUDA(rg::launch_render(false, si.mode, e->tuning.list_capacity, split, grid, a, S(stream)), "render inference");
-    e->launches += 2;
+    RG_CUDA(launch_splits(e, false, &si, split, a, S(stream)), "render inference");
+    e->launches += 1;
     return RG_OK;
 }
 
@@ -515,8 +527,8 @@ int rg_launch_backward(rg_engine* e, const rg_camera* cams, int32_t n_cams, cons
     // camera table, view count and settings: the chunk sequence is then the forward's, over its tiles.
     const bool replay = e->rec_valid && e->tuning.record_hits == 1 && e->rec_cams == cams && e->rec_n_cams == n_cams &&
                         std::memcmp(&e->rec_settings, s, sizeof(rg_settings)) == 0;
-    const int split = replay ? e->rec_split : launch_split(e, s);
-    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->vt, e->work_counter, S(stream)), "setup views");
+    const rg::SplitPair split = replay ? e->rec_split : launch_split(e, s, n_cams);
+    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->scene_ord, e->vt, e->work_counter, S(stream)), "setup views");
     rg::RenderArgs a;
     fill_args(e, cams, s, a);
     a.ray_colors_in = ray_colors;
@@ -528,13 +540,12 @@ int rg_launch_backward(rg_engine* e, const rg_camera* cams, int32_t n_cams, cons
         a.rec_arena = e->rec_arena;
         a.rec_cap = e->rec_cap;
         a.rec_tile = e->rec_tile;
-        a.rec_tiles = (int)record_heads(e->rec_tiles, split);
+        a.rec_tiles = (int)record_heads(e->rec_tiles, std::max(split.near, split.far));
         a.replay = 1;
     }
-    int grid = render_grid(e, true, kernel_mode(s), split);
-    RG_CUDA(rg::launch_render(true, s->mode, e->tuning.list_capacity, split, grid, a, S(stream)), "render backward");
+    RG_CUDA(launch_splits(e, true, s, split, a, S(stream)), "render backward");
     RG_CUDA(rg::launch_moment_grads((int)N, e->bvh.leaf_rec, e->bvh.leaf_ext, e->gacc_geo, S(stream)), "moments");
-    e->launches += 3;
+    e->launches += 2;
     return RG_OK;
 }
 

@@ -42,9 +42,20 @@ __device__ __forceinline__ void sh_basis(float x, float y, float z, int deg, flo
     B[15] = cSH3[6] * x * (xx - 3.f * yy);
 }
 
-__global__ void k_setup_views(const rg_camera* __restrict__ cams, int n, int tile_w, int tile_h, ViewTable* vt,
-                              int* work_counter) {
+__global__ void k_setup_views(const rg_camera* __restrict__ cams, int n, SplitPair pair, const int* __restrict__ scene_ord,
+                              ViewTable* vt, int* work_counter) {
     if (threadIdx.x != 0) return;
+    int split = pair.near;
+    if (pair.far != pair.near) {
+        float d2 = 0.f;
+        for (int a = 0; a < 3; ++a) {
+            const float e = ord2f(scene_ord[3 + a]) - ord2f(scene_ord[a]);
+            d2 += e * e;
+        }
+        if (!(d2 <= kFarBox * kFarBox)) split = pair.far;
+    }
+    const int tile_w = rg::tile_w(split), tile_h = rg::tile_h(split);
+    vt->split = split;
     int tiles = 0;
     long long rays = 0;
     for (int v = 0; v < n; ++v) {
@@ -278,9 +289,9 @@ __global__ void __launch_bounds__(128) k_color_bwd_sg(long long n, const float* 
     out.positions[3 * g + 2] += dpos[2];
 }
 
-cudaError_t launch_setup_views(const rg_camera* cams, int n_cams, int split, ViewTable* vt, int* work_counter,
-                               cudaStream_t s) {
-    k_setup_views<<<1, 32, 0, s>>>(cams, n_cams, tile_w(split), tile_h(split), vt, work_counter);
+cudaError_t launch_setup_views(const rg_camera* cams, int n_cams, SplitPair split, const int* scene_ord, ViewTable* vt,
+                               int* work_counter, cudaStream_t s) {
+    k_setup_views<<<1, 32, 0, s>>>(cams, n_cams, split, scene_ord, vt, work_counter);
     return cudaGetLastError();
 }
 

@@ -22,6 +22,11 @@ constexpr int kTileH = 4;
 // ... or, with two or four slabs of a ray side by side (split), a 4x4 or 4x2 one
 __host__ __device__ constexpr int tile_w(int split) { return split == 1 ? kTileW : 4; }
 __host__ __device__ constexpr int tile_h(int split) { return split == 4 ? 2 : 4; }
+// The splits of a launch, for scenes whose box is short and long (render_split).
+struct SplitPair {
+    int near, far;
+};
+constexpr float kFarBox = 20.f;         // diagonal of a long box: 1000 slabs
 constexpr int kMaxChunk = 255;          // slabs per traversal chunk (slab ranges are bytes)
 constexpr int kStack = 256;             // warp traversal stack depth (up to 31 pushes per wide node on the path)
 
@@ -48,6 +53,7 @@ struct DevStatus {
 // Per-launch view table computed on the device from the camera array (no host sync).
 struct ViewTable {
     int n_views;
+    int split;              // slabs side by side (1, 2 or 4): the kernels of another split return at once
     int total_tiles;
     long long total_rays;
     int tile_prefix[65];

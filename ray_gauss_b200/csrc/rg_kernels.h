@@ -81,9 +81,9 @@ cudaError_t launch_refit(long long n, const float* aabb, const GaussRec* rec, co
                          BvhBuffers& b, cudaStream_t s);
 
 cudaError_t launch_moment_grads(int n, const LeafRec* rec, const float4* ext, float4* acc, cudaStream_t s);
-// split: slabs side by side in the render launch that follows (render_split): its tiles are smaller
-cudaError_t launch_setup_views(const rg_camera* cams, int n_cams, int split, ViewTable* vt, int* work_counter,
-                               cudaStream_t s);
+// split: slabs side by side in the render launches that follow (render_split); their tiles are smaller
+cudaError_t launch_setup_views(const rg_camera* cams, int n_cams, SplitPair split, const int* scene_ord, ViewTable* vt,
+                               int* work_counter, cudaStream_t s);
 cudaError_t launch_color_forward(const rg_gaussians* g, const rg_camera* cams, int n_cams, const int* rank,
                                  float4* rgb_leaf, float* rgb_out, cudaStream_t s);
 cudaError_t launch_color_backward(const rg_gaussians* g, const rg_camera* cams, int n_cams, const int* rank,
@@ -93,8 +93,8 @@ cudaError_t launch_color_backward(const rg_gaussians* g, const rg_camera* cams, 
 // mode: RG_MODE_PARITY / RG_MODE_FAST; cap: 64/128; split: 1, 2 or 4 slabs of a ray side by side
 cudaError_t launch_render(bool backward, int mode, int cap, int split, int grid, const RenderArgs& a, cudaStream_t s);
 int render_occupancy(bool backward, int mode, int cap, int split);
-// The split of a launch of n_rays rays (0: unknown, which is 1) over n Gaussians.
-int render_split(int mode, int rnd_sample, int cap, long long n, long long n_rays);
+// The splits of a launch of n_rays rays (0: unknown, which is 1) in n_views views over n Gaussians.
+SplitPair render_split(int mode, int rnd_sample, int cap, long long n, int n_views, long long n_rays);
 
 // Copies a device status block read back to the host into the public struct (record_words is left
 // to the caller).

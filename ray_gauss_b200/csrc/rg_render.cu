@@ -35,6 +35,7 @@
 // arithmetic.  RG_MODE_FAST evaluates the 8 samples of a slab from the quadratic form of the
 // Mahalanobis distance along the ray with the SFU exponential and accumulates the adjoint in
 // moment form.
+#include <algorithm>
 #include <cstddef>
 
 #include "rg_common.cuh"
@@ -1537,6 +1538,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
     const int lane = threadIdx.x & 31;
     WarpSmem<FAST, SUB, CAP>& sm = smem[threadIdx.x >> 5];
     const ViewTable* vt = a.views;
+    if (vt->split != SUB) return;
     const float bg = a.white_bg ? 1.f : 0.f;
     if (lane == 0) {
 #pragma unroll
@@ -2001,28 +2003,27 @@ int render_occupancy(bool backward, int mode, int cap, int split) {
     return nb;
 }
 
-// Slabs side by side, by the launch's number of 8x4-pixel tiles.  Forward + backward in ms with 4 / 2 / 1
-// slabs, one view of SH-1 Gaussians:
-//   fast     1536 tiles:  300k on shells  9.2 / 18.3 / 41.0   1M in a ball with a far field  7.9 /  9.3 / 15.6
-//            7350         300k shells     7.8 / 10.1 / 18.2   1M ball                       19.0 / 14.8 / 14.8
-//           15000         50k shells      2.0 /  1.6 /  2.0   1M ball                       35.0 / 26.0 / 21.5
-//           28359         50k shells      3.3 /  2.3 /  2.2   1M ball                       62.1 / 45.1 / 34.1
-//   parity   7350         300k shells    12.8 / 19.8 / 35.6   50k shells                     2.9 /  2.6 /  3.9
-//           15000         300k shells    18.3 / 22.6 / 34.9   50k shells                     5.1 /  3.7 /  4.2
-//           28359         300k shells    27.4 / 26.7 / 41.5   50k shells                     8.9 /  5.8 /  5.1
-// Few tiles wait for the slowest one, which the split shortens; many share the traversal better when
-// they are whole.  The parity kernels' lists hold fewer entries of a whole tile, so that dense tiles
-// (many Gaussians per tile) gain from the split for longer.  The lines lie where the geometric means
-// over these scenes and some of several views cross.  Whole steps: 10k Gaussians at 200x200, drop-in,
-// 1.56 ms whole and 0.86 split; 300k on shells at 797x801, drop-in, 35.2 and 19.0; three uneven views of
-// 60k on shells, fast, 8.9 and 2.4.
-int render_split(int mode, int rnd_sample, int cap, long long n, long long n_rays) {
+// Slabs side by side.  Few tiles wait for the slowest one, which the split shortens, the more the more
+// Gaussians a tile sees; many share the traversal better when they are whole, above all where rays are
+// long (an unbounded scene's far field: chunk after chunk with few Gaussians).  With T the launch's
+// 8x4-pixel tiles and x = Gaussians * views / T / (T / 1000), the lines below are where forward +
+// backward cross over 144 launches of 300 to 200,000 tiles, 1 to 12 views and 5k to 1M Gaussians in
+// boxes, on shells (3 to 5 units across) and in a ball with a far field (200); they lose 0.1 to 2 % on
+// the best choice for each.  In ms with 4 / 2 / 1 slabs:
+//   fast, short    300k, 1536 tiles  9.2 / 18.3 / 51.6    300k, 15000 tiles  10.0 / 10.3 / 16.9
+//                  50k, 28359        3.3 /  2.3 /  2.3    325k, 56328, 10 views  48.8 / 49.1 / 92.9
+//   fast, long     1M, 1536          7.9 /  9.3 / 15.6    1M, 28359          62.1 / 45.1 / 34.1
+//   parity, short  300k, 15000      18.3 / 22.6 / 34.9    50k, 28359          8.9 /  5.8 /  5.1
+// Whole steps: 10k Gaussians at 200x200, drop-in, 1.56 ms whole and 0.86 split; 300k on shells at
+// 797x801, drop-in, 35.2 and 19.0; three uneven views of 60k on shells, fast, 8.9 and 2.4.
+SplitPair render_split(int mode, int rnd_sample, int cap, long long n, int n_views, long long n_rays) {
     const bool fast = mode == RG_MODE_FAST && rnd_sample == 0;
     // random offsets draw slab after slab; long lists are whole tiles' (the autotuner's choice)
-    if (rnd_sample == 1 || cap > 64 || n_rays <= 0) return 1;
-    const long long tiles = n_rays / (kTileW * kTileH);
-    if (tiles <= (fast ? 8000 : 5000) || (!fast && tiles <= 30000 && tiles <= n / 10)) return 4;
-    return tiles <= (fast ? 22000 : 40000) ? 2 : 1;
+    if (rnd_sample == 1 || cap > 64 || n_rays <= 0) return {1, 1};
+    const double t = (double)std::max(1ll, n_rays / (kTileW * kTileH));
+    const double x = 1000.0 * (double)n * n_views / (t * t);
+    auto pick = [&](double four, double two) { return x >= four ? 4 : x >= two ? 2 : 1; };
+    return {fast ? pick(1.0, 0.1) : pick(0.7, 0.2), pick(32.0, 6.0)};
 }
 
 cudaError_t launch_render(bool backward, int mode, int cap, int split, int grid, const RenderArgs& args, cudaStream_t s) {

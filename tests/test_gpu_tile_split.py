@@ -28,7 +28,7 @@ class _Rays:
 
 
 @pytest.mark.parametrize("record", [1, -1])
-@pytest.mark.parametrize("split", [1, 2, 4])
+@pytest.mark.parametrize("split", [1, 2, 4, "far"])
 @pytest.mark.parametrize("mode", ["parity", "fast"])
 def test_layouts_against_oracle(cuda, oracle, mode, split, record):
     from ray_gauss_b200 import synthetic as S
@@ -36,6 +36,8 @@ def test_layouts_against_oracle(cuda, oracle, mode, split, record):
     from ray_gauss_b200.engine import Engine, make_gaussians
     p, _, white = S.workload("small_object", n=1500, seed=2)
     p["scales"] = p["scales"] * 3.0
+    if split == "far":        # a long scene box: of the two kernels that are launched, the other one runs
+        p["positions"][:3] = p["positions"][:3] * 25.0
     cams = [S.look_at_camera(e, [0.0, 0.0, 0.0], W + 5 * i, H, fovx=math.radians(40.0), device=cuda)
             for i, e in enumerate(([2.5, 1.0, 0.6], [0.3, -2.8, 0.2]))]
     P = {k: v.to(cuda).contiguous() for k, v in p.items()}
@@ -43,7 +45,7 @@ def test_layouts_against_oracle(cuda, oracle, mode, split, record):
     views = BatchedViews(cams, mode=mode)
     eng = Engine()
     eng.set_tuning(record_hits=record)
-    eng.lib = _Rays(eng.lib, {1: 0, 2: 10_000 * 32, 4: views.n_rays}[split])
+    eng.lib = _Rays(eng.lib, {1: 0, 2: 3000 * 32, 4: views.n_rays, "far": 3000 * 32}[split])
     g = make_gaussians(P["positions"], P["scales"], P["quaternions"], P["densities"], P["color_features"])
     cams_t, _, _ = eng.cameras(cams)
     img, _ = eng.render_forward(g, cams_t, 2, views.n_rays, _st(views))
