@@ -41,7 +41,11 @@ def camera_table(cameras):
     focals = []
     for cam in cameras:
         key = (cam.FoVx, cam.FoVy, cam.image_width, cam.image_height)
-        f = known.get(key)
+        try:
+            f = known.get(key)
+        except TypeError:     # values without a hash, such as zero-dimensional arrays
+            key = tuple(float(v) for v in key)
+            f = known.get(key)
         if f is None:
             f = known[key] = (fov2focal(key[0], key[2]), fov2focal(key[1], key[3]), key[2], key[3])
         focals.append(f)
