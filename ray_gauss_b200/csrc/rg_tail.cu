@@ -17,10 +17,10 @@
 // accesses: a quaternion, four positions or lobe axes (12 floats), or four elements of a tensor whose
 // clamp is elementwise, so the clamp and the statistics work on the values in registers.  Every byte is
 // read and written once: HBM-bound at 28 bytes per parameter float (param, m, v read and written, grad
-// read).  1M Gaussians, 115 floats each, 3.25 GB: 548 us (91 % of a copy's rate), against 805 us when a block took 256
+// read).  1M Gaussians, 115 floats each, 3.25 GB: 553 us (90 % of a copy's rate), against 805 us when a block took 256
 // Gaussians through all tensors in turn (few loads in flight at a time, threads idle at the narrow
 // tensors, the clamps on parameters read again behind a barrier).  That form, k_train_tail, still does
-// what has no 16-byte alignment, and the last n % 4 Gaussians.
+// what has no 16-byte alignment and what l2_resident names.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -120,6 +120,24 @@ __device__ __forceinline__ float clamp_scale(const rg_train_tail& d, float v, lo
     return v;
 }
 
+// The statistics or the clamp of tensor i for Gaussian g, from memory.
+__device__ void tail_row(const rg_train_tail& d, int i, long long g) {
+    const rg_adam_tensor& t = d.tensors[i];
+    if (i == d.idx_positions && t.grad && (d.grad_norm_accum || d.num_accum || d.num_accum_gnv)) {
+        const float* gp = t.grad + 3 * g;
+        tail_stats(d, g, gp[0], gp[1], gp[2]);
+    }
+    if (i == d.idx_densities && t.param[g] < 0.f) t.param[g] = 0.f;
+    if (i == d.idx_quaternions && d.normalize_quaternions) {
+        float4* qp = reinterpret_cast<float4*>(t.param) + g;
+        *qp = unit_quaternion(*qp);
+    }
+    if (i == d.idx_lobe_axis && d.normalize_lobe_axis)
+        for (int l = 0; l < t.width / 3; ++l) unit_axis(t.param + g * t.width + 3 * l);
+    if (i == d.idx_scales)
+        for (int k = 0; k < 3; ++k) t.param[3 * g + k] = clamp_scale(d, t.param[3 * g + k], g);
+}
+
 // Blocks of the tensors: those of segment k end at block_end[k].
 struct TailSegments {
     int count, iters;
@@ -144,11 +162,11 @@ __device__ __forceinline__ void tail_unit(const rg_adam_tensor& t, const AdamSte
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         if (first + k * stride >= end) continue;
-        p[k] = __ldcs(P + k * stride);
+        p[k] = P[k * stride];
         if (steps) {
             g[k] = __ldcs(G + k * stride);
-            m[k] = __ldcs(M + k * stride);
-            v[k] = __ldcs(V + k * stride);
+            m[k] = M[k * stride];
+            v[k] = V[k * stride];
         }
     }
     if (steps) {
@@ -159,19 +177,30 @@ __device__ __forceinline__ void tail_unit(const rg_adam_tensor& t, const AdamSte
             adam1(p[k].y, g[k].y, m[k].y, v[k].y, s);
             adam1(p[k].z, g[k].z, m[k].z, v[k].z, s);
             adam1(p[k].w, g[k].w, m[k].w, v[k].w, s);
-            __stcs(M + k * stride, m[k]);
-            __stcs(V + k * stride, v[k]);
+            M[k * stride] = m[k];
+            V[k * stride] = v[k];
         }
     }
     f(p);
 #pragma unroll
     for (int k = 0; k < NV; ++k)
-        if (first + k * stride < end) __stcs(P + k * stride, p[k]);
+        if (first + k * stride < end) P[k * stride] = p[k];
 }
 
-// Gaussians [0, n4), n4 a multiple of 4; every tensor 16-byte aligned.
-__global__ void __launch_bounds__(kTailThreads) k_tail_stream(const TailArgs args, const TailSegments seg, long long n4) {
+// Gaussians [0, n4), n4 a multiple of 4; every tensor 16-byte aligned.  Where n4 < n a last block per tensor
+// takes the rest (10k Gaussians: 41 us a call with a launch of its own for them, 33 without).
+__global__ void __launch_bounds__(kTailThreads, 2) k_tail_stream(const TailArgs args, const TailSegments seg, long long n4) {
     const rg_train_tail& d = args.d;
+    const unsigned whole = seg.block_end[seg.count - 1];
+    if (blockIdx.x >= whole) {
+        const int i = seg.tensor[blockIdx.x - whole];
+        const rg_adam_tensor& t = d.tensors[i];
+        AdamStep s;
+        if (adam_step(d, i, s)) adam_range(t, s, n4 * t.width, d.n * t.width);
+        __syncthreads();  // the clamp reads parameters that other threads stepped
+        if (n4 + threadIdx.x < d.n) tail_row(d, i, n4 + threadIdx.x);
+        return;
+    }
     int k = 0;
     while (blockIdx.x >= seg.block_end[k]) ++k;
     const int i = seg.tensor[k];
@@ -222,48 +251,27 @@ __global__ void __launch_bounds__(kTailThreads) k_tail_stream(const TailArgs arg
                 } else if (quat) {
                     p[k] = unit_quaternion(p[k]);
                 } else if (scale) {
-                    for (int c = 0; c < 4; ++c) e[c] = clamp_scale(d, e[c], (at + c) / 3);
+                    const long long g = at / 3;
+                    const int r = (int)(at - 3 * g);
+                    for (int c = 0; c < 4; ++c) e[c] = clamp_scale(d, e[c], g + (r + c >= 3));
                 }
             }
         });
     }
 }
 
-// The Gaussians from `first`.
-__global__ void __launch_bounds__(kTailThreads) k_train_tail(const TailArgs args, long long first) {
+__global__ void __launch_bounds__(kTailThreads) k_train_tail(const TailArgs args) {
     const rg_train_tail& d = args.d;
-    const long long g0 = first + (long long)blockIdx.x * kTailGaussians;
+    const long long g0 = (long long)blockIdx.x * kTailGaussians;
     const long long g1 = g0 + kTailGaussians < d.n ? g0 + kTailGaussians : d.n;
-    for (int i = 0; i < d.n_tensors && i < kTailMaxTensors; ++i) {
+    for (int i = 0; i < d.n_tensors; ++i) {
         AdamStep s;
         if (adam_step(d, i, s)) adam_range(d.tensors[i], s, g0 * d.tensors[i].width, g1 * d.tensors[i].width);
     }
     __syncthreads();  // the clamps below read parameters that other threads of the block stepped
     const long long g = g0 + threadIdx.x;
     if (g >= g1) return;
-    // densification statistics from the position gradient
-    if (d.idx_positions >= 0 && d.tensors[d.idx_positions].grad &&
-        (d.grad_norm_accum || d.num_accum || d.num_accum_gnv)) {
-        const float* gp = d.tensors[d.idx_positions].grad + 3 * g;
-        tail_stats(d, g, gp[0], gp[1], gp[2]);
-    }
-    // clamps after the step
-    if (d.idx_densities >= 0) {
-        float* p = d.tensors[d.idx_densities].param + g;
-        if (*p < 0.f) *p = 0.f;
-    }
-    if (d.normalize_quaternions && d.idx_quaternions >= 0) {
-        float4* qp = reinterpret_cast<float4*>(d.tensors[d.idx_quaternions].param) + g;
-        *qp = unit_quaternion(*qp);
-    }
-    if (d.normalize_lobe_axis && d.idx_lobe_axis >= 0 && d.tensors[d.idx_lobe_axis].width > 0) {
-        const rg_adam_tensor& t = d.tensors[d.idx_lobe_axis];
-        for (int l = 0; l < t.width / 3; ++l) unit_axis(t.param + g * t.width + 3 * l);
-    }
-    if (d.idx_scales >= 0) {
-        float* s = d.tensors[d.idx_scales].param + 3 * g;
-        for (int k = 0; k < 3; ++k) s[k] = clamp_scale(d, s[k], g);
-    }
+    for (int i = 0; i < d.n_tensors; ++i) tail_row(d, i, g);
 }
 
 int check_tail(const rg_train_tail* d) {
@@ -291,6 +299,18 @@ int check_tail(const rg_train_tail* d) {
         if (!d->step_scalars && (!(t.bias1 > 0.f) || !(t.bias2_sqrt > 0.f))) return RG_ERR_INVALID_ARG;
     }
     return RG_OK;
+}
+
+// Clouds of narrow rows whose tensors (with the gradients) about fit L2 go to k_train_tail: most of what it
+// reads hits there, and its blocks, with half the registers, are all resident at once, while k_tail_stream's
+// come in waves.  k_train_tail / k_tail_stream, us: 23 floats per Gaussian: 14 / 14 at 40k, 16 / 21 at 80k, 35 / 41
+// at 250k, 62 / 62 at 400k; 44 floats: 23 / 21 at 40k, 27 / 35 at 80k, 43 / 51 at 160k, 80 / 71 at 250k; 59
+// floats: 23 / 21 at 40k, 25 / 29 at 60k, 53 / 58 at 160k; 79 floats: 51 / 45 at 60k, 92 / 61 at 120k; 115
+// floats: 52 / 43 at 40k, 113 / 84 at 120k (it takes the tensors in turn: long chains).
+bool l2_resident(const rg_train_tail& d) {
+    long long width = 0;
+    for (int i = 0; i < d.n_tensors; ++i) width += d.tensors[i].width;
+    return width <= 64 && d.n >= 50000 && 16 * d.n * width <= 150000000;
 }
 
 }  // namespace
@@ -322,10 +342,12 @@ int rg_train_tail_step(const rg_train_tail* d, void* stream) {
         seg.tensor[seg.count] = i;
         seg.block_end[seg.count++] = (unsigned)blocks;
     }
-    if (blocks > 0x7fffffffll) n4 = 0;
-    if (n4) k_tail_stream<<<(unsigned)blocks, kTailThreads, 0, st>>>(a, seg, n4);
-    if (n4 < d->n)
-        k_train_tail<<<(unsigned)((d->n - n4 + kTailGaussians - 1) / kTailGaussians), kTailThreads, 0, st>>>(a, n4);
+    if (n4 < d->n) blocks += seg.count;
+    if (blocks > 0x7fffffffll || !seg.count || l2_resident(*d)) n4 = 0;
+    if (n4)
+        k_tail_stream<<<(unsigned)blocks, kTailThreads, 0, st>>>(a, seg, n4);
+    else
+        k_train_tail<<<(unsigned)((d->n + kTailGaussians - 1) / kTailGaussians), kTailThreads, 0, st>>>(a);
     return cudaGetLastError() == cudaSuccess ? RG_OK : RG_ERR_CUDA;
 }
 

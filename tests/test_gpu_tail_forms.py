@@ -9,11 +9,14 @@ WIDTHS = dict(positions=(3,), densities=(), scales=(3,), quaternions=(4,), rgb=(
               bandwidth=(5,), axis=(5, 3))
 
 
-def _tensors(n, offset, dev):
+NARROW = {k: WIDTHS[k] for k in ("positions", "densities", "scales", "quaternions", "rgb", "axis")}
+
+
+def _tensors(n, offset, dev, widths):
     """Random tensors whose storage starts `offset` floats after a 16-byte boundary."""
     gen = torch.Generator(device="cpu").manual_seed(n)
     out = {}
-    for k, sh in WIDTHS.items():
+    for k, sh in widths.items():
         flat = torch.empty(offset + n * int(torch.Size(sh).numel()), device=dev)
         t = flat[offset:].view((n,) + sh)
         t.copy_(torch.randn((n,) + sh, generator=gen))
@@ -21,12 +24,13 @@ def _tensors(n, offset, dev):
     return out
 
 
-@pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 4096, 5003])
-def test_streaming_form_equals_the_unaligned_form(cuda, n):
+@pytest.mark.parametrize("n,widths", [(n, WIDTHS) for n in (1, 3, 4, 5, 1023, 4096, 5003)] +
+                         [(n, NARROW) for n in (49_999, 50_000, 50_001)])   # narrow rows: whole blocks from 50k on
+def test_streaming_form_equals_the_unaligned_form(cuda, n, widths):
     from ray_gauss_b200.train_tail import FusedTrainTail, LrSchedule
     got = []
     for offset in (0, 1):
-        p, g = _tensors(n, offset, cuda), _tensors(n, 0, cuda)
+        p, g = _tensors(n, offset, cuda, widths), _tensors(n, 0, cuda, widths)
         g["positions"][::2] = 0.0
         if offset == 0:
             p["quaternions"][0] = 0.0
