@@ -182,7 +182,7 @@ RG_API int rg_destroy(rg_engine* e);
  * hit-list record (96 B per ray); without it the backward traverses the BVH again. */
 RG_API int rg_reserve(rg_engine* e, int64_t n, int32_t n_views, int64_t n_rays);
 /* The number of rays of the render launches that follow (the cameras are read on the device, so the
- * engine does not know it otherwise; 0, the default: unknown).  It chooses between two tile layouts of
+ * engine does not know it otherwise; 0, the default: unknown).  It chooses between the tile layouts of
  * the render kernels, not what they compute: a small launch ends with its slowest tile and runs on
  * smaller ones.  A backward that replays its forward's hit lists keeps the forward's layout. */
 RG_API int rg_expect_rays(rg_engine* e, int64_t n_rays);

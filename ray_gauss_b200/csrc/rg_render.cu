@@ -10,20 +10,19 @@
 //   sample buffers            :437-498, compositing :500-519
 //   adjoint                   optix_raycasting/cuda_train/backward/gaussians_aabb.cu:505-775
 //
-// Design.  A warp owns an 8x4 pixel tile (tiles of all views are pulled from one atomic work
-// counter).  Each lane marches its own ray with the reference's slab sequence (tb += 0.02 in
-// FP32); the warp advances in chunks of K slabs per lane (K adapts between 1 and 255: it grows
-// while hits are sparse and halves when the hit list overflows).  For a chunk the warp traverses
-// the wide BVH once for the packet of its lanes' segments (one child slot per lane, tested with
-// interval arithmetic over the lanes' directions) with a warp-uniform stack, runs the exact
-// ellipsoid test per lane at the leaves
-// and appends every leaf that any lane hits to a shared hit
-// list with, per lane, the range of the chunk's slabs its interval covers (exact for K <= 8; one
-// slab of margin on each side for longer chunks, where the extra slabs' samples fall outside the
-// threshold ellipsoid and are masked out).  The list is consumed slab by slab: each lane evaluates
-// only entries whose range holds the slab, reading the leaf record with a warp-uniform (broadcast)
-// load.  A full list for a single slab is consumed in several passes (a leaf-index cursor skips
-// the leaves already taken; DFS order visits leaves in increasing index), so no hit is dropped.
+// Design.  A warp owns an 8x4 pixel tile, or a part of one where it takes several slabs of a ray at a time
+// (TileShape); tiles of all views are pulled from one atomic work counter.  Each ray marches with the
+// reference's slab sequence (tb += 0.02 in FP32); the warp advances in chunks of K slabs per ray (K adapts
+// between 1 and 255: it grows while hits are sparse and shrinks in place when the hit list overflows).  For a
+// chunk the warp traverses the wide BVH once for the packet of its rays' segments (one child slot per lane,
+// tested with interval arithmetic over the rays' directions) with a warp-uniform stack.  Leaves wait until
+// there are 32, are culled one per lane against the tile's ray cone, and the candidates take the exact
+// ellipsoid test, all rays at a time.  A leaf that any ray hits is appended to a shared hit list with, per
+// ray, the range of the chunk's slabs its interval covers (settled with the exact test where it decides).
+// The list is consumed slab by slab: each lane evaluates only entries whose range holds its slab, reading the
+// leaf record with a warp-uniform (broadcast) load.  A full list for a single slab is consumed in several
+// passes (a leaf-index cursor skips the leaves already taken; DFS order visits leaves in increasing index),
+// so no hit is dropped.
 // The adjoint recomputes each slab's sample buffers, folds the compositing adjoint into three
 // scalars per sample, evaluates each Gaussian's gradient per lane, reduces it across the warp with
 // a transposed shuffle reduction (16 shuffles for 14 values) and issues one atomic per value.
@@ -50,16 +49,16 @@ constexpr float kNegHalfLog2e = -0.72134752044448170f;
 constexpr float kLog2SigThr = -3.3219280948873623f;   // log2(0.1): per-sample density threshold
 constexpr float kInvSlab = 50.0f;          // 1 / 0.02
 constexpr int kExactChunk = 8;             // chunks up to this length use exact slab ranges
-constexpr int kCounters = 9;
+constexpr int kCounters = 9;               // per-warp counters: the WarpStats fields, hit pairs, slabs
+#ifndef RG_DIRECT_ATOMIC_LANES
+#define RG_DIRECT_ATOMIC_LANES 24  // up to this many contributing lanes add with float4 atomics directly
+#endif
 #ifndef RG_SPLIT_DIRECT_ATOMIC_LANES
 // ... and on split tiles, whose lanes are few rays' slabs: a Gaussian near the camera gets 10^5 and more of
 // them, and what is added alone to its large sum is lost below the sum's last bit (24 here: 3e-3 off on 4
 // views at 1920x1080; 4: as exact as whole tiles at the sizes that are split)
 #define RG_SPLIT_DIRECT_ATOMIC_LANES 4
 #endif
-#ifndef RG_DIRECT_ATOMIC_LANES
-#define RG_DIRECT_ATOMIC_LANES 24  // up to this many contributing lanes add with float4 atomics directly
-#endif               // per-warp counters: the WarpStats fields, hit pairs, slabs
 constexpr unsigned kNoRecord = 0xffffffffu;     // hit-list record: no (next) chunk record
 constexpr unsigned kRecordMulti = 0x80000000u;  // chunk consumed in several traversal passes
 constexpr unsigned kRecordFailed = 0xfffffffeu; // the tile's last chunk did not fit the arena
@@ -1496,7 +1495,9 @@ __device__ __forceinline__ float group_transmittance(RayState& r, const f2* alph
 // fit the shared memory of the 64-entry tuning (256-entry fast lists) and were measured best on
 // 1M Gaussians x 16 views.  The parity kernels want registers for the slab's points and sums rather
 // than warps (300k-Gaussian object, forward / backward: 12.8 / 24.7 ms at 4 blocks, 128 registers and
-// 400 B of spills; 12.3 / 22.5 at 3; 13.4 / 22.2 at 2, without spills).
+// 400 B of spills; 12.3 / 22.5 at 3; 13.4 / 22.2 at 2, without spills).  Split tiles come in launches whose
+// warps do not fill the chip, so registers cost nothing (three views of 60k Gaussians on whole tiles, fast,
+// per step: 8.9 ms at 7 blocks, 7.8 at 4, 7.7 at 3).
 #ifndef RG_FAST_FWD_MIN_BLOCKS
 #define RG_FAST_FWD_MIN_BLOCKS 7
 #endif
