@@ -260,6 +260,8 @@ __global__ void __launch_bounds__(kTailThreads, 2) k_tail_stream(const TailArgs 
     }
 }
 
+// The clamps are written out: through tail_row they take registers that cost a block per SM (160k x 44
+// floats 43 -> 60 us).
 __global__ void __launch_bounds__(kTailThreads) k_train_tail(const TailArgs args) {
     const rg_train_tail& d = args.d;
     const long long g0 = (long long)blockIdx.x * kTailGaussians;
@@ -271,7 +273,29 @@ __global__ void __launch_bounds__(kTailThreads) k_train_tail(const TailArgs args
     __syncthreads();  // the clamps below read parameters that other threads of the block stepped
     const long long g = g0 + threadIdx.x;
     if (g >= g1) return;
-    for (int i = 0; i < d.n_tensors; ++i) tail_row(d, i, g);
+    // densification statistics from the position gradient
+    if (d.idx_positions >= 0 && d.tensors[d.idx_positions].grad &&
+        (d.grad_norm_accum || d.num_accum || d.num_accum_gnv)) {
+        const float* gp = d.tensors[d.idx_positions].grad + 3 * g;
+        tail_stats(d, g, gp[0], gp[1], gp[2]);
+    }
+    // clamps after the step
+    if (d.idx_densities >= 0) {
+        float* p = d.tensors[d.idx_densities].param + g;
+        if (*p < 0.f) *p = 0.f;
+    }
+    if (d.normalize_quaternions && d.idx_quaternions >= 0) {
+        float4* qp = reinterpret_cast<float4*>(d.tensors[d.idx_quaternions].param) + g;
+        *qp = unit_quaternion(*qp);
+    }
+    if (d.normalize_lobe_axis && d.idx_lobe_axis >= 0 && d.tensors[d.idx_lobe_axis].width > 0) {
+        const rg_adam_tensor& t = d.tensors[d.idx_lobe_axis];
+        for (int l = 0; l < t.width / 3; ++l) unit_axis(t.param + g * t.width + 3 * l);
+    }
+    if (d.idx_scales >= 0) {
+        float* s = d.tensors[d.idx_scales].param + 3 * g;
+        for (int k = 0; k < 3; ++k) s[k] = clamp_scale(d, s[k], g);
+    }
 }
 
 int check_tail(const rg_train_tail* d) {
