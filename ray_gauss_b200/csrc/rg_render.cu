@@ -614,12 +614,13 @@ __device__ __forceinline__ void chunk_extent(const RayState& r, bool on, int K, 
 // Gaussians x 16 views 214M exact tests instead of 581M (122M entries used), forward 214.7 -> 196.8
 // ms; 3M x 4 x 1080p: 118.4 -> 98.3 ms.
 //
-// A chunk with too many Gaussians is shortened in place (K, nv and seg_hi): when the candidates or the
-// list fill up, K is halved until there is room, what starts at slab K or later is dropped (it holds
-// no slab of the shorter chunk), entries of the list that stay get the exact test again, and the
-// traversal goes on from its stack with the smaller packet.  The list is the one that a traversal
-// started with the shorter chunk builds, and nothing is visited twice.  `ovf` is set when the list
-// filled up for a single slab before the traversal finished.
+// A chunk with too many Gaussians is shortened in place (K, nv and seg_hi): when the list fills up, K is
+// halved, entries that start at slab K or later are dropped, those that stay get the exact test again,
+// and the traversal goes on from its stack with the smaller packet.  The list is the one that a
+// traversal started with the shorter chunk builds, and nothing is visited twice.  Only entries count: a
+// chunk's length decides which samples at slab edges the fast arithmetic evaluates, so it must not depend
+// on how many leaves pass may_hit.  When these fill their buffer they get the exact test at once and the
+// walk goes on.  `ovf` is set when the list filled up for a single slab before the traversal finished.
 template <bool FAST, int SUB, int CAP, bool DIAG>
 __device__ int traverse(WarpSmem<FAST, SUB, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float t_end,
                         float& seg_hi, int& K, int& nv, int cursor, bool& ovf, int lane, WarpStats& ws, bool infer) {
@@ -716,35 +717,6 @@ __device__ int traverse(WarpSmem<FAST, SUB, CAP>& sm, const RenderArgs& a, const
             __syncwarp();
             if (sp == 0) walk = false;
             else cur = sm.stack[--sp];
-        } else if (walk && nc > NC - 64 && K > 1 && rt >= rn && done == 0) {
-            // the candidates are many: shorten the chunk and drop those beyond it
-            unsigned halvings = 0;
-            int kept;
-            do {
-                K >>= 1;
-                ++halvings;
-                kept = 0;
-                for (int e = 0; e < nc; e += 32)
-                    kept += __popc(__ballot_sync(kFull, e + lane < nc && 2 * (int)(cand[e + lane] >> 25) < K));
-            } while (K > 1 && kept > NC - 64);
-            if (lane == 0) atomicAdd(&a.st->chunk_splits, (unsigned long long)halvings);
-            chunk_extent(r, on, K, t_end, nv, seg_hi);
-            set_packet<FAST, SUB, CAP>(sm, r, on, seg_hi, lane);
-            int to = 0;
-            for (int e = 0; e < nc; e += 32) {
-                const unsigned c = e + lane < nc ? cand[e + lane] : 0u;
-                const unsigned km = __ballot_sync(kFull, e + lane < nc && 2 * (int)(c >> 25) < K);
-                if ((km >> lane) & 1u) cand[to + __popc(km & ((1u << lane) - 1u))] = c;
-                to += __popc(km);
-                __syncwarp();
-            }
-            // the waiting leaves move up behind the candidates
-            const unsigned w0 = lane < nr ? cand[nc + lane] : 0u, w1 = 32 + lane < nr ? cand[nc + 32 + lane] : 0u;
-            __syncwarp();
-            if (lane < nr) cand[to + lane] = w0;
-            if (32 + lane < nr) cand[to + 32 + lane] = w1;
-            nc = to;
-            __syncwarp();
         } else {
             // exact tests, in order: the list's entries again after a chunk was shortened, else candidates
             const bool again = rt < rn;
@@ -759,7 +731,7 @@ __device__ int traverse(WarpSmem<FAST, SUB, CAP>& sm, const RenderArgs& a, const
             } else {
                 if (done >= nc) {
                     if (!walk) break;
-                    // a single slab: its candidates are in the list, the tree goes on (under 32 leaves wait)
+                    // the candidates were many: they are in the list, the tree goes on (under 32 leaves wait)
                     const unsigned w = lane < nr ? cand[nc + lane] : 0u;
                     __syncwarp();
                     if (lane < nr) cand[lane] = w;
@@ -788,16 +760,8 @@ __device__ int traverse(WarpSmem<FAST, SUB, CAP>& sm, const RenderArgs& a, const
                 }
                 // the list is full: shorten the chunk, test its entries again, then come back to this leaf
                 __syncwarp();
-                unsigned halvings = 0;
-                int kept;
-                do {
-                    K >>= 1;
-                    ++halvings;
-                    kept = 0;
-                    for (int e = lane; e < CAP; e += 32)
-                        kept += __popc(__ballot_sync(kFull, (int)(sm.urng[e] & 0xffffu) < K));
-                } while (K > 1 && kept >= CAP);
-                if (lane == 0) atomicAdd(&a.st->chunk_splits, (unsigned long long)halvings);
+                K >>= 1;
+                if (lane == 0) atomicAdd(&a.st->chunk_splits, 1ull);
                 chunk_extent(r, on, K, t_end, nv, seg_hi);
                 set_packet<FAST, SUB, CAP>(sm, r, on, seg_hi, lane);
                 rt = 0;
