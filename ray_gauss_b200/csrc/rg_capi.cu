@@ -448,7 +448,8 @@ int rg_launch_forward(rg_engine* e, const rg_camera* cams, int32_t n_cams, const
     DeviceScope dev_scope;
     if ((rc = dev_scope.enter(e))) return rc;
     const rg::SplitPair split = launch_split(e, s, n_cams);
-    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->scene_ord, e->vt, e->work_counter, S(stream)), "setup views");
+    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, kernel_mode(s) == RG_MODE_FAST, e->scene_ord, e->vt,
+                                   e->work_counter, S(stream)), "setup views");
     rg::RenderArgs a;
     fill_args(e, cams, s, a);
     a.ray_colors = ray_colors;
@@ -488,7 +489,8 @@ int rg_launch_inference(rg_engine* e, const rg_camera* cams, int32_t n_cams, con
     si.jitter = 0;
     si.rnd_sample = 0;
     const rg::SplitPair split = launch_split(e, &si, n_cams);
-    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->scene_ord, e->vt, e->work_counter, S(stream)), "setup views");
+    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, kernel_mode(&si) == RG_MODE_FAST, e->scene_ord, e->vt,
+                                   e->work_counter, S(stream)), "setup views");
     rg::RenderArgs a;
     fill_args(e, cams, &si, a);
     a.ray_colors = ray_colors;
@@ -528,7 +530,8 @@ int rg_launch_backward(rg_engine* e, const rg_camera* cams, int32_t n_cams, cons
     const bool replay = e->rec_valid && e->tuning.record_hits == 1 && e->rec_cams == cams && e->rec_n_cams == n_cams &&
                         std::memcmp(&e->rec_settings, s, sizeof(rg_settings)) == 0;
     const rg::SplitPair split = replay ? e->rec_split : launch_split(e, s, n_cams);
-    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, e->scene_ord, e->vt, e->work_counter, S(stream)), "setup views");
+    RG_CUDA(rg::launch_setup_views(cams, n_cams, split, kernel_mode(s) == RG_MODE_FAST, e->scene_ord, e->vt,
+                                   e->work_counter, S(stream)), "setup views");
     rg::RenderArgs a;
     fill_args(e, cams, s, a);
     a.ray_colors_in = ray_colors;

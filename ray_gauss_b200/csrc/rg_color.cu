@@ -42,8 +42,8 @@ __device__ __forceinline__ void sh_basis(float x, float y, float z, int deg, flo
     B[15] = cSH3[6] * x * (xx - 3.f * yy);
 }
 
-__global__ void k_setup_views(const rg_camera* __restrict__ cams, int n, SplitPair pair, const int* __restrict__ scene_ord,
-                              ViewTable* vt, int* work_counter) {
+__global__ void k_setup_views(const rg_camera* __restrict__ cams, int n, SplitPair pair, bool whole_tiles,
+                              const int* __restrict__ scene_ord, ViewTable* vt, int* work_counter) {
     if (threadIdx.x != 0) return;
     int split = pair.near;
     if (pair.far != pair.near) {
@@ -54,7 +54,7 @@ __global__ void k_setup_views(const rg_camera* __restrict__ cams, int n, SplitPa
         }
         if (!(d2 <= kFarBox * kFarBox)) split = pair.far;
     }
-    const int tile_w = rg::tile_w(split), tile_h = rg::tile_h(split);
+    const int tile_w = rg::tile_w(whole_tiles ? 1 : split), tile_h = rg::tile_h(whole_tiles ? 1 : split);
     vt->split = split;
     int tiles = 0;
     long long rays = 0;
@@ -289,9 +289,9 @@ __global__ void __launch_bounds__(128) k_color_bwd_sg(long long n, const float* 
     out.positions[3 * g + 2] += dpos[2];
 }
 
-cudaError_t launch_setup_views(const rg_camera* cams, int n_cams, SplitPair split, const int* scene_ord, ViewTable* vt,
-                               int* work_counter, cudaStream_t s) {
-    k_setup_views<<<1, 32, 0, s>>>(cams, n_cams, split, scene_ord, vt, work_counter);
+cudaError_t launch_setup_views(const rg_camera* cams, int n_cams, SplitPair split, bool whole_tiles, const int* scene_ord,
+                               ViewTable* vt, int* work_counter, cudaStream_t s) {
+    k_setup_views<<<1, 32, 0, s>>>(cams, n_cams, split, whole_tiles, scene_ord, vt, work_counter);
     return cudaGetLastError();
 }
 

@@ -19,7 +19,7 @@ constexpr float kSigThr = 0.1f;         // per-sample density threshold
 constexpr int kWarp = 32;
 constexpr int kTileW = 8;               // a warp renders an 8x4 pixel tile
 constexpr int kTileH = 4;
-// ... or, with two or four slabs of a ray side by side (split), a 4x4 or 4x2 one
+// ... or, with two or four slabs of a ray side by side (split; parity arithmetic), a 4x4 or 4x2 one
 __host__ __device__ constexpr int tile_w(int split) { return split == 1 ? kTileW : 4; }
 __host__ __device__ constexpr int tile_h(int split) { return split == 4 ? 2 : 4; }
 // The splits of a launch, for scenes whose box is short and long (render_split).

@@ -81,9 +81,10 @@ cudaError_t launch_refit(long long n, const float* aabb, const GaussRec* rec, co
                          BvhBuffers& b, cudaStream_t s);
 
 cudaError_t launch_moment_grads(int n, const LeafRec* rec, const float4* ext, float4* acc, cudaStream_t s);
-// split: slabs side by side in the render launches that follow (render_split); their tiles are smaller
-cudaError_t launch_setup_views(const rg_camera* cams, int n_cams, SplitPair split, const int* scene_ord, ViewTable* vt,
-                               int* work_counter, cudaStream_t s);
+// split: slabs side by side in the render launches that follow (render_split); their tiles are smaller unless
+// whole_tiles (fast arithmetic: teams of warps)
+cudaError_t launch_setup_views(const rg_camera* cams, int n_cams, SplitPair split, bool whole_tiles, const int* scene_ord,
+                               ViewTable* vt, int* work_counter, cudaStream_t s);
 cudaError_t launch_color_forward(const rg_gaussians* g, const rg_camera* cams, int n_cams, const int* rank,
                                  float4* rgb_leaf, float* rgb_out, cudaStream_t s);
 cudaError_t launch_color_backward(const rg_gaussians* g, const rg_camera* cams, int n_cams, const int* rank,

@@ -183,7 +183,7 @@ extern "C" RG_API int rg_render_forward_noalloc(const rg_gaussians* g, const rg_
     if (rg::launch_prepass(g, rec, aabb, scene_ord, status, st) != cudaSuccess) return RG_ERR_CUDA;
     if (rg::launch_build(n, aabb, scene_ord, rec, g, bvh, st) != cudaSuccess) return RG_ERR_CUDA;
     if (rg::launch_color_forward(g, cams, n_cams, bvh.rank, rgb_leaf, nullptr, st) != cudaSuccess) return RG_ERR_CUDA;
-    if (rg::launch_setup_views(cams, n_cams, rg::SplitPair{1, 1}, scene_ord, vt, work, st) != cudaSuccess) return RG_ERR_CUDA;
+    if (rg::launch_setup_views(cams, n_cams, rg::SplitPair{1, 1}, true, scene_ord, vt, work, st) != cudaSuccess) return RG_ERR_CUDA;
 
     rg::RenderArgs a;
     std::memset(&a, 0, sizeof(a));

@@ -11,7 +11,7 @@
 //   adjoint                   optix_raycasting/cuda_train/backward/gaussians_aabb.cu:505-775
 //
 // Design.  A warp owns an 8x4 pixel tile, or a part of one where it takes several slabs of a ray at a time
-// (TileShape); tiles of all views are pulled from one atomic work counter.  Each ray marches with the
+// (TileShape; in the fast arithmetic the warps of a tile then share its list); tiles of all views are pulled from one atomic work counter.  Each ray marches with the
 // reference's slab sequence (tb += 0.02 in FP32); the warp advances in chunks of K slabs per ray (K adapts
 // between 1 and 255: it grows while hits are sparse and shrinks in place when the hit list overflows).  For a
 // chunk the warp traverses the wide BVH once for the packet of its rays' segments (one child slot per lane,
@@ -65,18 +65,21 @@ constexpr unsigned kRecordFailed = 0xfffffffeu; // the tile's last chunk did not
 
 // Rays and slabs of a warp.  SUB == 1: 32 rays (8x4 pixels), a slab at a time.  SUB == 2 or 4: 16 (4x4) or 8
 // (4x2) rays, the lanes SUB r .. SUB r + SUB - 1 holding ray r's slabs k .. k + SUB - 1.  Their sums are
-// independent; only the transmittance runs through them in turn, by the same operations as slab after
-// slab.  A Gaussian spans a few slabs, so a list entry is evaluated once for them all, by a tile that is
-// smaller: not many more evaluations in all, but a fraction of them in one tile's chain, and a launch
-// of few tiles lasts as long as its slowest one.  Leaves are tested SUB at a time.  render_split has the
-// lines between them.
+// independent; only transmittance and colour (in the adjoint: g . R) run through them in turn, by the same
+// operations as slab after slab.  A Gaussian spans a few slabs, so a list entry is evaluated once for them
+// all, for fewer rays: not many more evaluations in all, but a fraction of them in one tile's chain, and a
+// launch of few tiles lasts as long as its slowest one.  render_split has the lines between them.
+//   Parity arithmetic: a list holds each ray's exact slabs, so it does not matter which rays share it.  A warp
+// is by itself, with a smaller tile; leaves are tested SUB at a time.
+//   Fast arithmetic: a ray evaluates the slabs that any ray of its list covers, up to the chunk's end, and at
+// a slab's edge a sample can round above the threshold outside the ray's own interval.  So the rays that
+// share a list and a chunk stay those of the 8x4 tile: SUB warps are a team, which builds the tile's list
+// together (TeamSmem) and then marches a part of its rays each.
 template <int SUB>
 struct TileShape {
     static constexpr int rays = 32 / SUB;
     static constexpr int w = tile_w(SUB), h = tile_h(SUB);
     static_assert(w * h == rays, "a ray per pixel");
-    // the lanes of sub-slab 0
-    static constexpr unsigned lanes = SUB == 1 ? 0xffffffffu : SUB == 2 ? 0x55555555u : 0x11111111u;
 };
 
 // Warp hit-list layout.  Parity arithmetic keeps, per entry and ray, the exact range of the chunk's
@@ -86,12 +89,15 @@ struct TileShape {
 // are masked out), which allows longer lists and so longer chunks in dense regions.
 template <bool FAST, int SUB, int CAP>
 struct WarpSmem {
+    using Store = WarpSmem;                              // what lies in shared memory: one per warp
+    static constexpr int kStores = kWarpsPerBlock;
+    __device__ static WarpSmem& of(Store* s, int warp, int) { return s[warp]; }
     static constexpr int MB = FAST || SUB > 1 ? 4 : 2;   // slabs per entry-mask block (a multiple of SUB)
     static constexpr int NB = 64;                        // entry-mask blocks
     static constexpr int KM = MB == 4 ? 255 : 128;       // longest chunk (MB * NB, slab ranges are bytes)
     int ids[CAP];
     unsigned urng[CAP];                              // union of the lanes' slab ranges: lo | hi << 16
-    unsigned lmask[FAST ? CAP : 1];                  // fast: rays (sub-slab 0 lanes) whose interval overlaps the chunk
+    unsigned lmask[FAST ? CAP : 1];                  // fast: rays whose interval overlaps the chunk
     unsigned short lrng[FAST ? 1 : CAP][32 / SUB];   // parity: per ray lo | hi << 8 (lo > hi: no hit)
     unsigned smask[NB][CAP / 32];                    // entries whose union range meets block k / MB
     unsigned long long occ[4];                       // slabs holding any entry (union occupancy)
@@ -102,6 +108,67 @@ struct WarpSmem {
     unsigned rec_first, rec_prev;                    // forward: first / last chunk record
     unsigned rec_cur;                                // backward: next chunk record to replay
     unsigned long long cnt[kCounters];               // activity counters of the warp (lane 0)
+};
+
+// A team's part of shared memory: the list of its 8x4 tile and, per warp, the entry masks of the warp's rays.
+template <int SUB, int CAP>
+struct TeamSmem {
+    struct Warp {
+        unsigned smask[64][CAP / 32];
+        unsigned long long occ[4], cnt[kCounters];
+    };
+    int ids[CAP];
+    unsigned urng[CAP], lmask[CAP];                  // over the tile's 32 rays
+    unsigned leaves[2 * CAP], cand[2 * CAP];         // leaves of the walk, and those that pass the cone test
+    __align__(16) float packet[24];
+    __align__(16) float cone[12];
+    int stack[kStack];
+    unsigned rec_first, rec_prev;
+    int tile[2];
+    unsigned hits[2][SUB];                           // leaves that each warp found hit
+    unsigned walked;                                 // leaves of the walk | tree not through << 31
+    unsigned char live[32];                          // rays that go on
+    Warp warp[SUB];
+};
+// A warp of a team: names of what it uses in the team's part.
+template <int SUB, int CAP>
+struct TeamWarp {
+    using Store = TeamSmem<SUB, CAP>;
+    static constexpr int kStores = kWarpsPerBlock / SUB;
+    static constexpr int MB = 4, NB = 64, KM = 255;
+    Store& t;
+    const int w;                                     // the warp's number in the team; 0 leads
+    const int slot;                                  // the list lane (pixel of the 8x4 tile) of this lane's ray
+    const unsigned own;                              // the list lanes of the warp's rays
+    int flip = 0, tile_flip = 0;                     // which of the two buffers is next
+    int (&ids)[CAP];
+    unsigned (&urng)[CAP], (&lmask)[CAP];
+    unsigned (&smask)[64][CAP / 32];
+    unsigned long long (&occ)[4], (&cnt)[kCounters];
+    float (&packet)[24], (&cone)[12];
+    int (&stack)[kStack];
+    // the warp's rays: the tile's left or right half (SUB == 2), or one of its quarters
+    __device__ static int first(int w) { return SUB == 2 ? 4 * w : 4 * (w & 1) + 16 * (w >> 1); }
+    __device__ TeamWarp(Store& s, int w_, int lane)
+        : t(s), w(w_), slot(first(w_) + lane / SUB % 4 + 8 * (lane / SUB / 4)),
+          own((SUB == 2 ? 0x0f0f0f0fu : 0x00000f0fu) << first(w_)), ids(s.ids), urng(s.urng), lmask(s.lmask),
+          smask(s.warp[w_].smask), occ(s.warp[w_].occ), cnt(s.warp[w_].cnt), packet(s.packet), cone(s.cone),
+          stack(s.stack) {}
+    // Waits for the team's warps (what they wrote to shared memory is then visible).
+    __device__ void sync() const {
+        __syncwarp();
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)(threadIdx.x >> 5) / SUB), "n"(32 * SUB) : "memory");
+    }
+};
+template <int CAP>
+struct WarpSmem<true, 2, CAP> : TeamWarp<2, CAP> {
+    using TeamWarp<2, CAP>::TeamWarp;
+    __device__ static WarpSmem of(TeamSmem<2, CAP>* s, int warp, int lane) { return WarpSmem(s[warp / 2], warp % 2, lane); }
+};
+template <int CAP>
+struct WarpSmem<true, 4, CAP> : TeamWarp<4, CAP> {
+    using TeamWarp<4, CAP>::TeamWarp;
+    __device__ static WarpSmem of(TeamSmem<4, CAP>* s, int warp, int lane) { return WarpSmem(s[warp / 4], warp % 4, lane); }
 };
 
 // Warp-uniform activity counters of one tile (32-bit; added to the warp's shared-memory totals at
@@ -433,6 +500,13 @@ __device__ __forceinline__ int occ_next(const unsigned long long* occ, int k, in
     return K;
 }
 
+// Where the chunk records of a tile are kept: with the warp, or with the team.
+template <bool FAST, int SUB, int CAP>
+__device__ __forceinline__ auto& record_of(WarpSmem<FAST, SUB, CAP>& sm) {
+    if constexpr (FAST && SUB > 1) return sm.t;
+    else return sm;
+}
+
 // Adds the tile's counters to the warp's totals and resets them.
 template <bool FAST, int SUB, int CAP, bool DIAG>
 __device__ __forceinline__ void flush_stats(WarpSmem<FAST, SUB, CAP>& sm, WarpStats& ws, unsigned hits, unsigned slabs,
@@ -458,6 +532,24 @@ __device__ __forceinline__ void flush_stats(WarpSmem<FAST, SUB, CAP>& sm, WarpSt
     ws = WarpStats();
 }
 
+// The slabs [lo, hi] of the chunk in which a ray meets a leaf (exact test; lo > hi: none).
+template <bool FAST>
+__device__ __forceinline__ void leaf_slabs(const RenderArgs& a, const RayState& r, float seg_hi, int K, int nv, int leaf,
+                                           bool infer, int& lo, int& hi) {
+    float root1, root2;
+    bool ok;
+    if (FAST) {
+        ok = roots_fast(load_rec(a.rec, leaf), r, root1, root2);
+    } else {
+        float4 m4 = __ldg(reinterpret_cast<const float4*>(a.rec + leaf));
+        ok = roots_exact(load_is(a.is_rec, leaf), f3(m4.x, m4.y, m4.z), r, root1, root2);
+    }
+    // the slab query ends at the box exit in training launches and at the slab end in
+    // inference launches (cuda_test/gaussians_aabb.cu:408-409)
+    const float tclip = infer ? INFINITY : r.texit;
+    if (ok) slab_range<FAST>(r, K, nv, seg_hi, tclip, root1, root2, lo, hi);
+}
+
 // Exact test of SUB leaves at a time, each by the 32 / SUB rays of the tile (`leaf`: the one of the
 // lane's sub-slab, < 0 for none).  Leaves that any ray hits are appended to the list, in order.  Returns
 // how many leaves were dealt with: SUB, or the number of those before the one that found the list full.
@@ -467,20 +559,7 @@ __device__ __forceinline__ int leaf_batch(WarpSmem<FAST, SUB, CAP>& sm, const Re
                                           WarpStats& ws, bool infer) {
     if (DIAG) ws.leaf_tests += __popc(__ballot_sync(kFull, lane < SUB && leaf >= 0));
     int lo = 255, hi = -1;
-    if (on && (SUB == 1 || leaf >= 0)) {
-        float root1, root2;
-        bool ok;
-        if (FAST) {
-            ok = roots_fast(load_rec(a.rec, leaf), r, root1, root2);
-        } else {
-            float4 m4 = __ldg(reinterpret_cast<const float4*>(a.rec + leaf));
-            ok = roots_exact(load_is(a.is_rec, leaf), f3(m4.x, m4.y, m4.z), r, root1, root2);
-        }
-        // the slab query ends at the box exit in training launches and at the slab end in
-        // inference launches (cuda_test/gaussians_aabb.cu:408-409)
-        const float tclip = infer ? INFINITY : r.texit;
-        if (ok) slab_range<FAST>(r, K, nv, seg_hi, tclip, root1, root2, lo, hi);
-    }
+    if (on && (SUB == 1 || leaf >= 0)) leaf_slabs<FAST>(a, r, seg_hi, K, nv, leaf, infer, lo, hi);
     const unsigned any = __ballot_sync(kFull, lo <= hi);
     if (!any) return SUB;
     if constexpr (SUB == 1) {
@@ -499,6 +578,7 @@ __device__ __forceinline__ int leaf_batch(WarpSmem<FAST, SUB, CAP>& sm, const Re
         ++count;
         return 1;
     } else {
+        static_assert(!FAST, "teams test their leaves with team_batch");
         const int sub = lane % SUB;
         int ulo = lo, uhi = hi;
         unsigned hit = any;          // bit q: some ray hits the leaf of sub-slab q
@@ -511,9 +591,8 @@ __device__ __forceinline__ int leaf_batch(WarpSmem<FAST, SUB, CAP>& sm, const Re
         hit &= (1u << SUB) - 1u;
         const int at = count + __popc(hit & ((1u << sub) - 1u)), n = __popc(hit);
         if (((hit >> sub) & 1u) && at < CAP) {
-            if (!FAST) sm.lrng[at][lane / SUB] = (unsigned short)((lo & 0xff) | ((hi & 0xff) << 8));
+            sm.lrng[at][lane / SUB] = (unsigned short)((lo & 0xff) | ((hi & 0xff) << 8));
             if (lane < SUB) {
-                if (FAST) sm.lmask[at] = (any >> sub) & TileShape<SUB>::lanes;
                 sm.ids[at] = leaf;
                 sm.urng[at] = (unsigned)ulo | ((unsigned)uhi << 16);
             }
@@ -549,8 +628,13 @@ __device__ __forceinline__ unsigned long long range_bits(int lo, int hi, int w) 
 // serial walk of all entries per block and, for the occupancy, by lane 0 as entries were appended.
 template <bool FAST, int SUB, int CAP, bool DIAG>
 __device__ __forceinline__ void finish_list(WarpSmem<FAST, SUB, CAP>& sm, int count, int K, int lane, WarpStats& ws) {
+    constexpr bool TEAM = FAST && SUB > 1;   // a team's warp takes the entries that its rays hit
     __syncwarp();
-    if (DIAG) ws.entries += count;
+    if constexpr (TEAM) {
+        if (DIAG && sm.w == 0) ws.entries += count;
+    } else {
+        if (DIAG) ws.entries += count;
+    }
     constexpr int MB = WarpSmem<FAST, SUB, CAP>::MB;
     const int nblk = (K + MB - 1) / MB, nocc = (K + 63) >> 6;
     const int nw = nwords(count);
@@ -559,7 +643,9 @@ __device__ __forceinline__ void finish_list(WarpSmem<FAST, SUB, CAP>& sm, int co
 #pragma unroll 1
     for (int w = 0; w < nw; ++w) {
         const int e = 32 * w + lane;
-        const unsigned u = e < count ? sm.urng[e] : 0xffffu;   // no entry: lo 65535 > hi 0
+        bool in = e < count;
+        if constexpr (TEAM) in = in && (sm.lmask[e] & sm.own);
+        const unsigned u = in ? sm.urng[e] : 0xffffu;   // no entry: lo 65535 > hi 0
         const int lo = (int)(u & 0xffffu), hi = (int)(u >> 16);
         // entry e meets block bk iff b0 <= bk <= b1
         const int b0 = lo / MB, b1 = hi / MB;
@@ -602,6 +688,125 @@ __device__ __forceinline__ void chunk_extent(const RayState& r, bool on, int K, 
     }
 }
 
+// A walk through the wide tree (warp-uniform).  Candidates [0, nc), then leaves still waiting for may_hit
+// [nc, nc + nr).  A candidate is leaf | (first slab / 2) << 25.
+struct Walk {
+    int nc = 0, nr = 0;
+    int sp = 0, cur = ~0;    // one Gaussian: the root is a leaf
+    bool more = true;        // cur is still to be visited
+    unsigned guard = 0, visits = 0;
+};
+constexpr unsigned kLeafMask = (1u << 25) - 1u;
+static_assert(kMaxGaussians == 1ll << 25, "25 bits of a candidate hold the leaf");
+
+__device__ __forceinline__ Walk walk_start(const RenderArgs& a) {
+    Walk s;
+    if (a.n_leaves > 1) {
+        const int2 root = __ldg(a.wide_tab);
+        s.cur = wide_pack(root.x, root.y);
+    }
+    return s;
+}
+
+// may_hit for a leaf of the lane's own.  A ray of the tile may meet it in the chunk: `first` is the first slab
+// where.  [t0, t1]: where the tile's chunks start; t_last: where they end.
+struct ChunkSpan {
+    float t0, t1, t_last;
+};
+__device__ __forceinline__ ChunkSpan chunk_span(const RayState& r, bool on, float seg_hi) {
+    return {__uint_as_float(__reduce_min_sync(kFull, on ? __float_as_uint(r.tb) : 0x7f800000u)),
+            __uint_as_float(__reduce_max_sync(kFull, on ? __float_as_uint(r.tb) : 0u)),
+            __uint_as_float(__reduce_max_sync(kFull, on ? __float_as_uint(seg_hi) : 0u))};
+}
+template <bool FAST, int SUB, int CAP>
+__device__ __forceinline__ bool cull(const WarpSmem<FAST, SUB, CAP>& sm, const RenderArgs& a, float3 o, const ChunkSpan& c,
+                                     int K, int leaf, int& first) {
+    float t;
+    const bool may = may_hit<FAST, SUB, CAP>(sm, load_rec(a.rec, leaf), o, c.t0 * 0.99999f, c.t_last * 1.00001f, t);
+    // slab s of a lane starts at tb + 0.02 s up to the drift of the repeated addition
+    const float drift = (float)(K + 1) * (c.t1 + (float)K * kSlab) * (kInvSlab * 2.4e-7f);
+    first = min(255, max(0, (int)((t - c.t1) * kInvSlab - 1.f - drift)));
+    return may && first < K;
+}
+
+// Goes on until the buffer (2 CAP words) is nearly full or the tree is through.  CULL: the leaves take may_hit
+// on the way; else every leaf is a candidate.
+template <bool CULL, bool FAST, int SUB, int CAP, bool DIAG>
+__device__ __forceinline__ void walk_tree(WarpSmem<FAST, SUB, CAP>& sm, unsigned* cand, const RenderArgs& a,
+                                          const RayState& r, bool on, float seg_hi, int K, int cursor, Walk& s,
+                                          int lane) {
+    constexpr int NC = 2 * CAP;
+    const unsigned guard_max = 2u * (unsigned)a.n_leaves + 64u;
+    while (true) {
+        if constexpr (!CULL) {
+            s.nc += s.nr;
+            s.nr = 0;
+        }
+        if (CULL && (s.nr >= 32 || (s.nr > 0 && !s.more))) {
+            // may_hit for up to 32 waiting leaves; the rest moves up behind the candidates
+            const int m = min(s.nr, 32);
+            const unsigned leaf = lane < m ? cand[s.nc + lane] : 0u;
+            const unsigned next = 32 + lane < s.nr ? cand[s.nc + 32 + lane] : 0u;
+            const ChunkSpan c = chunk_span(r, on, seg_hi);
+            int first = 0;
+            const bool may = lane < m && (int)leaf > cursor && cull<FAST, SUB, CAP>(sm, a, r.o, c, K, (int)leaf, first);
+            const unsigned mm = __ballot_sync(kFull, may);
+            if (may) cand[s.nc + __popc(mm & ((1u << lane) - 1u))] = leaf | ((unsigned)(first >> 1) << 25);
+            s.nc += __popc(mm);
+            s.nr -= m;
+            __syncwarp();
+            if (lane < s.nr) cand[s.nc + lane] = next;
+            __syncwarp();
+        } else if (s.more && s.nc <= NC - 64) {
+            if (++s.guard > guard_max) {
+                if (lane == 0) atomicAdd(&a.st->watchdog_trips, 1ull);
+                s.more = false;
+                continue;
+            }
+            if (s.cur >= 0) {
+                if (DIAG) ++s.visits;
+                const int first = s.cur & ((1 << kWideCountShift) - 1), n = (s.cur >> kWideCountShift) + 1;
+                bool hit = false;
+                int cid = 0;
+                if (lane < n) {
+                    float3 lo, hi;
+                    int range_hi;
+                    load_slot(a.slots + first + lane, lo, hi, cid, range_hi);
+                    hit = (range_hi > cursor) && packet_hit(sm.packet, lo, hi);
+                }
+                const unsigned hm = __ballot_sync(kFull, hit), im = __ballot_sync(kFull, hit && cid >= 0);
+                const unsigned lead = hm & ((im & (0u - im)) - 1u);   // leaves before the first node (all: no node)
+                if ((lead >> lane) & 1u) cand[s.nc + s.nr + __popc(lead & ((1u << lane) - 1u))] = (unsigned)~cid;
+                s.nr += __popc(lead);
+                unsigned rest = hm & ~lead;
+                if (rest) {
+                    // a hit lane's place on the stack is the number of hit children above it
+                    const int f = __ffs(rest) - 1;
+                    rest &= rest - 1u;
+                    const int more = __popc(rest);
+                    if (s.sp + more <= kStack) {
+                        if ((rest >> lane) & 1u) sm.stack[s.sp + __popc(rest >> lane) - 1] = cid;
+                        s.sp += more;
+                    } else if (lane == 0) {
+                        atomicAdd(&a.st->stack_overflows, 1ull);
+                    }
+                    s.cur = __shfl_sync(kFull, cid, f);
+                    __syncwarp();
+                    continue;
+                }
+            } else {
+                if (lane == 0) cand[s.nc + s.nr] = (unsigned)~s.cur;
+                ++s.nr;
+            }
+            __syncwarp();
+            if (s.sp == 0) s.more = false;
+            else s.cur = sm.stack[--s.sp];
+        } else {
+            break;
+        }
+    }
+}
+
 // Warp-cooperative traversal for the chunk [tb, seg_hi] of every active lane (the packet set by
 // set_packet).  At a wide node lane k tests child slot k against the packet.  Hit leaves wait in a
 // buffer (the leading ones of a node are taken all at once); the first hit child that is a node is
@@ -627,152 +832,199 @@ __device__ int traverse(WarpSmem<FAST, SUB, CAP>& sm, const RenderArgs& a, const
     int count = 0;
     ++ws.traversals;
     ovf = false;
-    // Candidates [0, nc), then leaves still waiting for may_hit [nc, nc + nr): the entry masks' space,
-    // which finish_list writes only afterwards.  A candidate is leaf | (first slab / 2) << 25.
+    // the candidates lie in the entry masks' space, which finish_list writes only afterwards
     unsigned* const cand = &sm.smask[0][0];
-    constexpr int NC = 2 * CAP;
-    static_assert(sizeof(sm.smask) >= NC * sizeof(unsigned) && NC >= 256, "candidate buffer");
-    static_assert(kMaxGaussians == 1ll << 25, "25 bits of a candidate hold the leaf");
-    constexpr unsigned kLeafMask = (1u << 25) - 1u;
-    int nc = 0, nr = 0;
+    static_assert(sizeof(sm.smask) >= 2 * CAP * sizeof(unsigned) && 2 * CAP >= 256, "candidate buffer");
     int done = 0;            // candidates that had the exact test
     int rt = 0, rn = 0;      // entries of the shortened chunk's old list still to test again: [rt, rn)
-    int sp = 0;
-    int cur = ~0;            // one Gaussian: the root is a leaf
-    bool walk = true;        // cur is still to be visited
-    if (a.n_leaves > 1) {
-        const int2 root = __ldg(a.wide_tab);
-        cur = wide_pack(root.x, root.y);
-    }
-    unsigned guard = 0, visits = 0;
-    const unsigned guard_max = 2u * (unsigned)a.n_leaves + 64u;
+    Walk s = walk_start(a);
     while (true) {
-        if (rt >= rn && done == 0 && (nr >= 32 || (nr > 0 && !walk))) {
-            // may_hit for up to 32 waiting leaves; the rest moves up behind the candidates
-            const int m = min(nr, 32);
-            const unsigned leaf = lane < m ? cand[nc + lane] : 0u;
-            const unsigned next = 32 + lane < nr ? cand[nc + 32 + lane] : 0u;
-            // slab s of a lane starts at tb + 0.02 s up to the drift of the repeated addition
-            const float tb0 = __uint_as_float(__reduce_min_sync(kFull, on ? __float_as_uint(r.tb) : 0x7f800000u));
-            const float tb1 = __uint_as_float(__reduce_max_sync(kFull, on ? __float_as_uint(r.tb) : 0u));
-            const float t1 = __uint_as_float(__reduce_max_sync(kFull, on ? __float_as_uint(seg_hi) : 0u));
-            bool may = lane < m && (int)leaf > cursor;
-            int first = 0;
-            if (may) {
-                float t;
-                may = may_hit<FAST, SUB, CAP>(sm, load_rec(a.rec, (int)leaf), r.o, tb0 * 0.99999f, t1 * 1.00001f, t);
-                const float drift = (float)(K + 1) * (tb1 + (float)K * kSlab) * (kInvSlab * 2.4e-7f);
-                first = min(255, max(0, (int)((t - tb1) * kInvSlab - 1.f - drift)));
-                may = may && first < K;
-            }
-            const unsigned mm = __ballot_sync(kFull, may);
-            if (may) cand[nc + __popc(mm & ((1u << lane) - 1u))] = leaf | ((unsigned)(first >> 1) << 25);
-            nc += __popc(mm);
-            nr -= m;
-            __syncwarp();
-            if (lane < nr) cand[nc + lane] = next;
-            __syncwarp();
-        } else if (walk && nc <= NC - 64 && rt >= rn && done == 0) {
-            if (++guard > guard_max) {
-                if (lane == 0) atomicAdd(&a.st->watchdog_trips, 1ull);
-                walk = false;
+        if (rt >= rn && done == 0) walk_tree<true, FAST, SUB, CAP, DIAG>(sm, cand, a, r, on, seg_hi, K, cursor, s, lane);
+        // exact tests, in order: the list's entries again after a chunk was shortened, else candidates
+        const bool again = rt < rn;
+        unsigned todo;
+        unsigned mine = 0u;
+        if (again) {
+            // in registers before its places are written again (an entry never moves up)
+            const bool in = rt + lane < rn;
+            if (in) mine = (unsigned)sm.ids[rt + lane];
+            todo = __ballot_sync(kFull, in && (int)(sm.urng[rt + lane] & 0xffffu) < K);
+            rt += 32;
+        } else {
+            if (done >= s.nc) {
+                if (!s.more) break;
+                // the candidates were many: they are in the list, the tree goes on (under 32 leaves wait)
+                const unsigned w = lane < s.nr ? cand[s.nc + lane] : 0u;
+                __syncwarp();
+                if (lane < s.nr) cand[lane] = w;
+                s.nc = done = 0;
+                __syncwarp();
                 continue;
             }
-            unsigned rest = 0u;
-            if (cur >= 0) {
-                if (DIAG) ++visits;
-                const int first = cur & ((1 << kWideCountShift) - 1), n = (cur >> kWideCountShift) + 1;
-                bool hit = false;
-                int cid = 0;
-                if (lane < n) {
-                    float3 lo, hi;
-                    int range_hi;
-                    load_slot(a.slots + first + lane, lo, hi, cid, range_hi);
-                    hit = (range_hi > cursor) && packet_hit(sm.packet, lo, hi);
-                }
-                const unsigned hm = __ballot_sync(kFull, hit), im = __ballot_sync(kFull, hit && cid >= 0);
-                const unsigned lead = hm & ((im & (0u - im)) - 1u);   // leaves before the first node (all: no node)
-                if ((lead >> lane) & 1u) cand[nc + nr + __popc(lead & ((1u << lane) - 1u))] = (unsigned)~cid;
-                nr += __popc(lead);
-                rest = hm & ~lead;
-                if (rest) {
-                    // a hit lane's place on the stack is the number of hit children above it
-                    const int f = __ffs(rest) - 1;
-                    rest &= rest - 1u;
-                    const int more = __popc(rest);
-                    if (sp + more <= kStack) {
-                        if ((rest >> lane) & 1u) sm.stack[sp + __popc(rest >> lane) - 1] = cid;
-                        sp += more;
-                    } else if (lane == 0) {
-                        atomicAdd(&a.st->stack_overflows, 1ull);
-                    }
-                    cur = __shfl_sync(kFull, cid, f);
-                    __syncwarp();
-                    continue;
-                }
-            } else {
-                if (lane == 0) cand[nc + nr] = (unsigned)~cur;
-                ++nr;
-            }
-            __syncwarp();
-            if (sp == 0) walk = false;
-            else cur = sm.stack[--sp];
-        } else {
-            // exact tests, in order: the list's entries again after a chunk was shortened, else candidates
-            const bool again = rt < rn;
-            unsigned todo;
-            unsigned mine = 0u;
-            if (again) {
-                // in registers before its places are written again (an entry never moves up)
-                const bool in = rt + lane < rn;
-                if (in) mine = (unsigned)sm.ids[rt + lane];
-                todo = __ballot_sync(kFull, in && (int)(sm.urng[rt + lane] & 0xffffu) < K);
-                rt += 32;
-            } else {
-                if (done >= nc) {
-                    if (!walk) break;
-                    // the candidates were many: they are in the list, the tree goes on (under 32 leaves wait)
-                    const unsigned w = lane < nr ? cand[nc + lane] : 0u;
-                    __syncwarp();
-                    if (lane < nr) cand[lane] = w;
-                    nc = done = 0;
-                    __syncwarp();
-                    continue;
-                }
-                const bool in = done + lane < nc;
-                const unsigned c = in ? cand[done + lane] : 0u;
-                mine = c & kLeafMask;
-                todo = __ballot_sync(kFull, in && 2 * (int)(c >> 25) < K);
-            }
-            while (todo) {
-                const int leaf = next_leaf<SUB>(todo, mine, lane);
-                const int n = leaf_batch<FAST, SUB, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, leaf, count, lane, ws, infer);
+            const bool in = done + lane < s.nc;
+            const unsigned c = in ? cand[done + lane] : 0u;
+            mine = c & kLeafMask;
+            todo = __ballot_sync(kFull, in && 2 * (int)(c >> 25) < K);
+        }
+        while (todo) {
+            const int leaf = next_leaf<SUB>(todo, mine, lane);
+            const int n = leaf_batch<FAST, SUB, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, leaf, count, lane, ws, infer);
 #pragma unroll
-                for (int i = 0; i < SUB; ++i)
-                    if (i < n) todo &= todo - 1u;
-                if (n < SUB) break;
+            for (int i = 0; i < SUB; ++i)
+                if (i < n) todo &= todo - 1u;
+            if (n < SUB) break;
+        }
+        if (!again) done = min(s.nc, done + (todo ? __ffs(todo) - 1 : 32));
+        if (todo) {
+            if (K == 1) {
+                ovf = true;
+                break;
             }
-            if (!again) done = min(nc, done + (todo ? __ffs(todo) - 1 : 32));
-            if (todo) {
-                if (K == 1) {
-                    ovf = true;
-                    break;
-                }
-                // the list is full: shorten the chunk, test its entries again, then come back to this leaf
-                __syncwarp();
-                K >>= 1;
-                if (lane == 0) atomicAdd(&a.st->chunk_splits, 1ull);
-                chunk_extent(r, on, K, t_end, nv, seg_hi);
-                set_packet<FAST, SUB, CAP>(sm, r, on, seg_hi, lane);
-                rt = 0;
-                rn = count;
-                count = 0;
-            }
+            // the list is full: shorten the chunk, test its entries again, then come back to this leaf
             __syncwarp();
+            K >>= 1;
+            if (lane == 0) atomicAdd(&a.st->chunk_splits, 1ull);
+            chunk_extent(r, on, K, t_end, nv, seg_hi);
+            set_packet<FAST, SUB, CAP>(sm, r, on, seg_hi, lane);
+            rt = 0;
+            rn = count;
+            count = 0;
+        }
+        __syncwarp();
+    }
+    if (DIAG) ws.node_visits += s.visits;
+    finish_list<FAST, SUB, CAP, DIAG>(sm, count, K, lane, ws);
+    return count;
+}
+
+// Exact tests of a team: the leaves of `todo` (bits of lanes whose `mine` holds a leaf, the same in every warp)
+// are dealt out to its warps, a lane per ray of the tile (r: the list lane's ray), and those that any ray
+// hits are appended to the list, in order.  Returns what is left of `todo` when the list is full, else 0.
+// One barrier: the buffers alternate, and an entry's place is at or before the one its leaf was read from.
+template <int SUB, int CAP, bool DIAG>
+__device__ __forceinline__ unsigned team_batch(WarpSmem<true, SUB, CAP>& sm, const RenderArgs& a, const RayState& r,
+                                               bool on, float seg_hi, int K, int nv, unsigned todo, unsigned mine,
+                                               int& count, int lane, WarpStats& ws, bool infer) {
+    constexpr int kShare = 32 / SUB;
+    unsigned hits = 0u, rays = 0u, range = 0u;   // lane i keeps the warp's i-th leaf
+#pragma unroll 2
+    for (int i = 0; i < kShare; ++i) {
+        const int b = i * SUB + sm.w;
+        const int leaf = (int)__shfl_sync(kFull, mine, b);
+        if (!((todo >> b) & 1u)) continue;
+        int lo = 255, hi = -1;
+        if (on) leaf_slabs<true>(a, r, seg_hi, K, nv, leaf, infer, lo, hi);
+        const unsigned any = __ballot_sync(kFull, lo <= hi);
+        if (!any) continue;
+        const unsigned ulo = __reduce_min_sync(kFull, (unsigned)lo);
+        const unsigned uhi = __reduce_max_sync(kFull, (unsigned)(hi + 1)) - 1u;
+        hits |= 1u << b;
+        if (lane == i) {
+            rays = any;
+            range = ulo | (uhi << 16);
         }
     }
-    if (DIAG) ws.node_visits += visits;
-    finish_list<FAST, SUB, CAP, DIAG>(sm, count, K, lane, ws);
+    if (DIAG) ws.leaf_tests += sm.w == 0 ? __popc(todo) : 0;
+    if (lane == 0) sm.t.hits[sm.flip][sm.w] = hits;
+    sm.sync();
+    unsigned all = 0u;
+#pragma unroll
+    for (int q = 0; q < SUB; ++q) all |= sm.t.hits[sm.flip][q];
+    sm.flip ^= 1;
+    const int b = lane % kShare * SUB + sm.w;
+    const int leaf = (int)__shfl_sync(kFull, mine, b);
+    const int at = count + __popc(all & ((1u << b) - 1u)), n = __popc(all), room = CAP - count;
+    if (rays && at < CAP) {
+        sm.ids[at] = leaf;
+        sm.urng[at] = range;
+        sm.lmask[at] = rays;
+    }
+    count += min(n, room);
+    if (n <= room) return 0u;
+    for (int i = 0; i < room; ++i) all &= all - 1u;   // the first leaf without room
+    return todo & ~((all & (0u - all)) - 1u);
+}
+
+// traverse by a team: the same list, from the rays of its 8x4 tile.  The team's first warp walks, all of them
+// cull and test.  Every warp takes the same way through here.
+template <int SUB, int CAP, bool DIAG>
+__device__ int team_traverse(WarpSmem<true, SUB, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float t_end,
+                             float& seg_hi, int& K, int& nv, int cursor, bool& ovf, int lane, WarpStats& ws, bool infer) {
+    unsigned* const cand = sm.t.cand;
+    int count = 0;
+    ovf = false;
+    Walk s = walk_start(a);
+    if (sm.w == 0) {
+        ++ws.traversals;
+        set_packet<true, SUB, CAP>(sm, r, on, seg_hi, lane);
+    }
+    sm.sync();               // the last chunk's list has been read
+    while (true) {
+        if (sm.w == 0) {
+            walk_tree<false, true, SUB, CAP, DIAG>(sm, sm.t.leaves, a, r, on, seg_hi, K, cursor, s, lane);
+            if (lane == 0) sm.t.walked = (unsigned)s.nc | (s.more ? 1u << 31 : 0u);
+        }
+        sm.sync();
+        const int nl = (int)(sm.t.walked & 0xffffu);
+        const bool more = sm.t.walked >> 31;
+        // the cone test, 32 leaves per warp
+        const ChunkSpan span = chunk_span(r, on, seg_hi);
+        int nc = 0;
+        for (int base = 0; base < nl; base += 32 * SUB) {
+            const int l = base + 32 * sm.w + lane;
+            const unsigned leaf = l < nl ? sm.t.leaves[l] : 0u;
+            int first = 0;
+            const bool may = l < nl && (int)leaf > cursor && cull<true, SUB, CAP>(sm, a, r.o, span, K, (int)leaf, first);
+            const unsigned mm = __ballot_sync(kFull, may);
+            if (lane == 0) sm.t.hits[sm.flip][sm.w] = mm;
+            sm.sync();
+            int at = nc;
+#pragma unroll
+            for (int q = 0; q < SUB; ++q) {
+                const int n = __popc(sm.t.hits[sm.flip][q]);
+                if (q < sm.w) at += n;
+                nc += n;
+            }
+            sm.flip ^= 1;
+            if (may) cand[at + __popc(mm & ((1u << lane) - 1u))] = leaf | ((unsigned)(first >> 1) << 25);
+        }
+        sm.sync();
+        for (int done = 0; done < nc;) {
+            const bool in = done + lane < nc;
+            const unsigned c = in ? cand[done + lane] : 0u;
+            const unsigned todo = __ballot_sync(kFull, in && 2 * (int)(c >> 25) < K);
+            const unsigned left = team_batch<SUB, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, todo, c & kLeafMask, count, lane,
+                                                             ws, infer);
+            done += left ? __ffs(left) - 1 : 32;
+            if (!left) continue;
+            if (K == 1) {
+                ovf = true;
+                break;
+            }
+            // the list is full: shorten the chunk, test its entries again, then come back to this leaf
+            K >>= 1;
+            chunk_extent(r, on, K, t_end, nv, seg_hi);
+            if (sm.w == 0) {
+                if (lane == 0) atomicAdd(&a.st->chunk_splits, 1ull);
+                set_packet<true, SUB, CAP>(sm, r, on, seg_hi, lane);
+            }
+            sm.sync();
+            const int n = count;
+            count = 0;
+            for (int e = 0; e < n; e += 32) {
+                const bool old = e + lane < n;
+                const unsigned leaf = old ? (unsigned)sm.ids[e + lane] : 0u;
+                const unsigned stay = __ballot_sync(kFull, old && (int)(sm.urng[e + lane] & 0xffffu) < K);
+                team_batch<SUB, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, stay, leaf, count, lane, ws, infer);
+            }
+        }
+        if (ovf || !more) break;
+        // the leaves were many: those hit are in the list, the tree goes on
+        s.nc = 0;
+    }
+    sm.sync();
+    if (DIAG) ws.node_visits += s.visits;
+    finish_list<true, SUB, CAP, DIAG>(sm, count, K, lane, ws);
     return count;
 }
 
@@ -794,6 +1046,23 @@ __device__ int replay_list(WarpSmem<FAST, SUB, CAP>& sm, const RenderArgs& a, co
         }
     }
     finish_list<FAST, SUB, CAP, DIAG>(sm, count, K, lane, ws);
+    return count;
+}
+
+// replay_list by a team.
+template <int SUB, int CAP, bool DIAG>
+__device__ int team_replay(WarpSmem<true, SUB, CAP>& sm, const RenderArgs& a, const RayState& r, bool on, float seg_hi,
+                           int K, int nv, const unsigned* ids, int n, int lane, WarpStats& ws) {
+    int count = 0;
+    n = min(n, CAP);
+    sm.sync();               // the last chunk's list has been read
+    for (int base = 0; base < n; base += 32) {
+        const int mine = base + lane < n ? (int)ids[base + lane] : -1;
+        const unsigned todo = __ballot_sync(kFull, mine >= 0 && mine < a.n_leaves);
+        team_batch<SUB, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, todo, (unsigned)mine, count, lane, ws, false);
+    }
+    sm.sync();
+    finish_list<true, SUB, CAP, DIAG>(sm, count, K, lane, ws);
     return count;
 }
 
@@ -887,9 +1156,13 @@ __device__ __forceinline__ bool in_urange(unsigned u, int k) {
 // meets the chunk, the parity lists each ray's exact slab range.
 template <bool FAST, int SUB, int CAP>
 __device__ __forceinline__ bool lane_has_entry(const WarpSmem<FAST, SUB, CAP>& sm, int e, int kl, int lane) {
-    if (FAST) return ((sm.lmask[e] >> (lane / SUB * SUB)) & 1u) && (SUB == 1 || in_urange(sm.urng[e], kl));
-    const unsigned short rg = sm.lrng[e][lane / SUB];
-    return kl >= (int)(rg & 0xff) && kl <= (int)(rg >> 8);
+    if constexpr (FAST) {
+        if constexpr (SUB == 1) return (sm.lmask[e] >> lane) & 1u;
+        else return ((sm.lmask[e] >> sm.slot) & 1u) && in_urange(sm.urng[e], kl);
+    } else {
+        const unsigned short rg = sm.lrng[e][lane / SUB];
+        return kl >= (int)(rg & 0xff) && kl <= (int)(rg >> 8);
+    }
 }
 // Whether an entry's union range meets the slabs k .. k + SUB - 1.
 template <int SUB>
@@ -1230,16 +1503,6 @@ struct AdjBuf<false> {
     f2 H[kPairs], F[kPairs];
 };
 
-// Adds the same value to every H.
-__device__ __forceinline__ void add_start(AdjBuf<true>& ad, float x) {
-#pragma unroll
-    for (int i = 0; i < kBuf; ++i) ad.H[i] += x;
-}
-__device__ __forceinline__ void add_start(AdjBuf<false>& ad, float x) {
-#pragma unroll
-    for (int p = 0; p < kPairs; ++p) ad.H[p] = add2(ad.H[p], dup2(x));
-}
-
 // Adjoint of slab k for all list entries: per-lane gradient of each hit Gaussian, warp reduction,
 // one atomic per value.  Value order: ddens, S1.xyz, M2 (xx yy zz xy xz yz), 0, drgb.xyz.
 template <bool FAST, int SUB, int CAP, bool DIAG>
@@ -1455,6 +1718,124 @@ __device__ __forceinline__ float group_transmittance(RayState& r, const f2* alph
     return mine;
 }
 
+// composite for the slabs of a group: the terms of a lane's samples side by side, then added to the ray's
+// colour in turn.  `act`: the lane's slab counts; r.T is the transmittance at its start.
+template <bool FAST, int SUB>
+__device__ __forceinline__ void group_colour(RayState& r, const SlabBuf<FAST, false>& sb, const f2* alpha, bool act, int lane,
+                                             f2 nz) {
+    float w[kBuf];                       // fast: weight of a sample's colour sum
+    f2 cx[kPairs], cy[kPairs], cz[kPairs];   // parity: the terms
+    float T = r.T;
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) {
+        const f2 om = fma2(alpha[p], dup2(-1.f), dup2(1.f));
+        if constexpr (FAST) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = 2 * p + h;
+                w[i] = sb.sig[i] > 0.f ? __fdividef(T * half2(alpha[p], h), sb.sig[i]) : 0.f;
+                T *= half2(om, h);
+            }
+        } else {
+            const float s0 = lo2(sb.sig[p]), s1 = hi2(sb.sig[p]);
+            const f2 inv = pk(s0 > 0.f ? __frcp_rn(s0) : 0.f, s1 > 0.f ? __frcp_rn(s1) : 0.f);
+            const float T1 = __fmul_rn(T, lo2(om));
+            const f2 ta = mul2_rn(pk(T, T1), alpha[p], nz);
+            cx[p] = mul2_rn(mul2(sb.cx[p], inv), ta, nz);
+            cy[p] = mul2_rn(mul2(sb.cy[p], inv), ta, nz);
+            cz[p] = mul2_rn(mul2(sb.cz[p], inv), ta, nz);
+            T = __fmul_rn(T1, hi2(om));
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < SUB; ++q) {
+        if (lane % SUB == q && act) {
+            if constexpr (FAST) {
+#pragma unroll
+                for (int i = 0; i < kBuf; ++i)
+                    r.C = f3(fmaf(sb.C[i].x, w[i], r.C.x), fmaf(sb.C[i].y, w[i], r.C.y), fmaf(sb.C[i].z, w[i], r.C.z));
+            } else {
+#pragma unroll
+                for (int p = 0; p < kPairs; ++p)
+                    r.C = f3(__fadd_rn(__fadd_rn(r.C.x, lo2(cx[p])), hi2(cx[p])),
+                             __fadd_rn(__fadd_rn(r.C.y, lo2(cy[p])), hi2(cy[p])),
+                             __fadd_rn(__fadd_rn(r.C.z, lo2(cz[p])), hi2(cz[p])));
+            }
+        }
+        const int from = lane / SUB * SUB + q;
+        r.C = f3(__shfl_sync(kFull, r.C.x, from), __shfl_sync(kFull, r.C.y, from), __shfl_sync(kFull, r.C.z, from));
+    }
+}
+
+// slab_adjoint_scalars for the slabs of a group: what does not hold g . R side by side, then g . R through
+// them in turn.  Returns it at the group's end.
+template <bool FAST, int SUB>
+__device__ __forceinline__ float group_adjoint_scalars(const RayState& r, const SlabBuf<FAST, true>& sb, const f2* alpha,
+                                                       bool act, AdjBuf<FAST>& ad, int lane) {
+    float g[kBuf], x[kBuf];             // -g.C / sigma; T alpha, then g . R at the sample
+    float T = r.T;
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) {
+        const f2 om = fma2(alpha[p], dup2(-1.f), dup2(1.f));
+        if constexpr (FAST) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = 2 * p + h;
+                const float cd = sb.sig[i];
+                float inv = 0.f;
+                if (cd > 0.f) inv = __fdividef(1.f, cd);
+                g[i] = -(sb.gC[i] * inv);
+                x[i] = T * half2(alpha[p], h);
+                ad.F[i] = x[i] * inv;
+                T = T * half2(om, h);
+            }
+        } else {
+            const float s0 = lo2(sb.sig[p]), s1 = hi2(sb.sig[p]);
+            const f2 inv = pk(s0 > 0.f ? __frcp_rn(s0) : 0.f, s1 > 0.f ? __frcp_rn(s1) : 0.f);
+            const float T1 = __fmul_rn(T, lo2(om));
+            const f2 ngc = mul2(sb.ng[p], inv), ta = mul2(pk(T, T1), alpha[p]);
+            ad.F[p] = mul2(ta, inv);
+            g[2 * p] = lo2(ngc);
+            g[2 * p + 1] = hi2(ngc);
+            x[2 * p] = lo2(ta);
+            x[2 * p + 1] = hi2(ta);
+            T = __fmul_rn(T1, hi2(om));
+        }
+    }
+    float run = r.gR;
+#pragma unroll
+    for (int q = 0; q < SUB; ++q) {
+        if (lane % SUB == q && act) {
+#pragma unroll
+            for (int i = 0; i < kBuf; ++i) {
+                const float at = run;
+                run = fmaf(g[i], x[i], run);
+                x[i] = at;
+            }
+        }
+        run = __shfl_sync(kFull, run, lane / SUB * SUB + q);
+    }
+    T = r.T;
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) {
+        const f2 om = fma2(alpha[p], dup2(-1.f), dup2(1.f));
+        if constexpr (FAST) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = 2 * p + h;
+                ad.H[i] = ad.F[i] * g[i] - kDt * (T * g[i] + x[i]);
+                T = T * half2(om, h);
+            }
+        } else {
+            const float T1 = __fmul_rn(T, lo2(om));
+            const f2 ngc = pk(g[2 * p], g[2 * p + 1]), gR = pk(x[2 * p], x[2 * p + 1]);
+            ad.H[p] = fma2(ad.F[p], ngc, mul2(fma2(pk(T, T1), ngc, gR), dup2(-kDt)));
+            T = __fmul_rn(T1, hi2(om));
+        }
+    }
+    return run;
+}
+
 // Resident blocks per SM each kernel is compiled for (0: the compiler's choice).  The fast defaults
 // fit the shared memory of the 64-entry tuning (256-entry fast lists) and were measured best on
 // 1M Gaussians x 16 views.  The parity kernels want registers for the slab's points and sums rather
@@ -1499,9 +1880,11 @@ constexpr int min_blocks() {
 // without it those counters compile away and the kernel holds fewer live registers.
 template <bool BWD, bool FAST, int SUB, int CAP, bool DIAG>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB>()) k_render(RenderArgs a) {
-    __shared__ WarpSmem<FAST, SUB, CAP> smem[kWarpsPerBlock];
+    using SM = WarpSmem<FAST, SUB, CAP>;
+    constexpr bool TEAM = FAST && SUB > 1;   // the list is the one of a whole tile's rays, shared by SUB warps
+    __shared__ typename SM::Store smem[SM::kStores];
     const int lane = threadIdx.x & 31;
-    WarpSmem<FAST, SUB, CAP>& sm = smem[threadIdx.x >> 5];
+    decltype(auto) sm = SM::of(smem, threadIdx.x >> 5, lane);
     const ViewTable* vt = a.views;
     if (vt->split != SUB) return;
     const float bg = a.white_bg ? 1.f : 0.f;
@@ -1514,8 +1897,16 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
 
     while (true) {
         int tile = 0;
-        if (lane == 0) tile = atomicAdd(a.work_counter, 1);
-        tile = __shfl_sync(kFull, tile, 0);
+        if constexpr (TEAM) {
+            // (a team may pass a tile without a barrier: the two places alternate)
+            if (sm.w == 0 && lane == 0) sm.t.tile[sm.tile_flip] = atomicAdd(a.work_counter, 1);
+            sm.sync();
+            tile = sm.t.tile[sm.tile_flip];
+            sm.tile_flip ^= 1;
+        } else {
+            if (lane == 0) tile = atomicAdd(a.work_counter, 1);
+            tile = __shfl_sync(kFull, tile, 0);
+        }
         if (tile >= vt->total_tiles) break;
         // view of this tile (binary search over the tile prefix)
         int lo = 0, hi = vt->n_views - 1;
@@ -1526,14 +1917,15 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
         const int view = lo;
         const rg_camera cam = a.cams[view];
         const int W = cam.width, H = cam.height;
-        using TS = TileShape<SUB>;
+        using TS = TileShape<TEAM ? 1 : SUB>;
         const int tiles_x = (W + TS::w - 1) / TS::w;
         const int local = tile - vt->tile_prefix[view];
         const int ray = lane / SUB, sub = lane % SUB;
-        const int px = (local % tiles_x) * TS::w + ray % TS::w;
-        const int py = (local / tiles_x) * TS::h + ray / TS::w;
-        const bool valid = px < W && py < H;
-        const unsigned ray_l = (unsigned)(py * W + px);
+        const int pixel = TEAM ? lane : ray;
+        const int px = (local % tiles_x) * TS::w + pixel % TS::w;
+        const int py = (local / tiles_x) * TS::h + pixel / TS::w;
+        bool valid = px < W && py < H;
+        unsigned ray_l = (unsigned)(py * W + px);
         const int rgb_base = view * a.n_leaves;   // views x leaves < 2^31 (checked by the host)
 
         RayState r;
@@ -1574,6 +1966,17 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
         }
         r.alive = valid && (r.tenter < r.texit);
         r.tb = r.tenter;
+        // a team's warp: the list lane's ray of the whole tile, whose lists all warps build, and the ray it marches
+        RayState lr = r;
+        unsigned live = 0u;
+        if constexpr (TEAM) {
+            live = __ballot_sync(kFull, r.alive);
+            r.d = f3(__shfl_sync(kFull, lr.d.x, sm.slot), __shfl_sync(kFull, lr.d.y, sm.slot),
+                     __shfl_sync(kFull, lr.d.z, sm.slot));
+            r.texit = __shfl_sync(kFull, lr.texit, sm.slot);
+            valid = __shfl_sync(kFull, (int)valid, sm.slot);
+            ray_l = __shfl_sync(kFull, ray_l, sm.slot);
+        }
         r.T = 1.f;
         r.C = f3(0.f, 0.f, 0.f);
         r.g = f3(0.f, 0.f, 0.f);
@@ -1589,24 +1992,32 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
         int rounds = 0;
         // end of the searched range: an inference launch queries the last slab in full
         const bool infer = !BWD && a.infer;
-        const float t_end = infer ? r.texit + kSlab : r.texit;
+        const float l_texit = TEAM ? lr.texit : r.texit;
+        const float t_end = infer ? l_texit + kSlab : l_texit;
         // hit-list record of this tile: the forward appends chunk records, the backward replays them
         const bool rec_here = a.rec_arena != nullptr && tile < a.rec_tiles;
-        if (lane == 0) {
+        const bool leads = TEAM ? threadIdx.x / 32 % SUB == 0 : true;
+        unsigned team_rec = kNoRecord;   // backward: a team's next chunk record to replay
+        if constexpr (TEAM) {
+            if (BWD && rec_here && a.replay) team_rec = a.rec_tile[tile];
+            if (leads && lane == 0) sm.t.rec_first = sm.t.rec_prev = kNoRecord;
+        } else if (lane == 0) {
             sm.rec_first = kNoRecord;
             sm.rec_prev = kNoRecord;
             sm.rec_cur = (BWD && rec_here && a.replay) ? a.rec_tile[tile] : kNoRecord;
         }
         __syncwarp();
         while (true) {
-            bool on = r.alive;
+            bool on = TEAM ? live != 0u : r.alive;
             if (!__any_sync(kFull, on)) break;
             if (++rounds > kMaxRounds) {
-                if (lane == 0) atomicAdd(&a.st->watchdog_trips, 1ull);
+                if (leads && lane == 0) atomicAdd(&a.st->watchdog_trips, 1ull);
                 break;
             }
             unsigned rec_hdr = 0u;
-            unsigned rec_cur = BWD ? sm.rec_cur : kNoRecord;
+            unsigned rec_cur = kNoRecord;
+            if constexpr (TEAM) rec_cur = team_rec;
+            else if (BWD) rec_cur = sm.rec_cur;
             if (BWD && rec_cur != kNoRecord) {
                 if (rec_cur + 2u > a.rec_cap) {
                     rec_cur = kNoRecord;   // malformed link: traverse from here on
@@ -1618,22 +2029,45 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
             int nv;
             float seg_hi;
             // a slab step that no longer changes tb (|t| beyond ~2^19) would march forever
-            if (on && (!(r.tb < r.texit) || r.tb + kSlab == r.tb)) r.alive = on = false;
-            chunk_extent(r, on, K, t_end, nv, seg_hi);
+            bool l_on = false;   // a team: the list lane's ray
+            if constexpr (TEAM) {
+                l_on = ((live >> lane) & 1u) && lr.tb < lr.texit && lr.tb + kSlab != lr.tb;
+                live = __ballot_sync(kFull, l_on);
+                on = (live >> sm.slot) & 1u;
+                r.tb = __shfl_sync(kFull, lr.tb, sm.slot);
+                chunk_extent(lr, l_on, K, t_end, nv, seg_hi);
+            } else {
+                if (on && (!(r.tb < r.texit) || r.tb + kSlab == r.tb)) r.alive = on = false;
+                chunk_extent(r, on, K, t_end, nv, seg_hi);
+            }
             bool ovf = false;
             int count;
             const bool replayed = BWD && rec_cur != kNoRecord && !(rec_hdr & kRecordMulti);
-            if (!replayed) set_packet<FAST, SUB, CAP>(sm, r, on, seg_hi, lane);
+            // the hits after leaf `cursor`: entries (over: more than the list holds)
+            auto search = [&](int cursor, bool& over) {
+                if constexpr (TEAM)
+                    return team_traverse<SUB, CAP, DIAG>(sm, a, lr, l_on, t_end, seg_hi, K, nv, cursor, over, lane, ws,
+                                                         infer);
+                else
+                    return traverse<FAST, SUB, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, over, lane, ws,
+                                                          infer);
+            };
             if (replayed) {
                 const unsigned n_ids = min(rec_hdr & 0xffffu, a.rec_cap - rec_cur - 2u);
-                count = replay_list<FAST, SUB, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, a.rec_arena + rec_cur + 2, (int)n_ids,
-                                               lane, ws);
-                ++ws.replays;
+                const unsigned* ids = a.rec_arena + rec_cur + 2;
+                if constexpr (TEAM)
+                    count = team_replay<SUB, CAP, DIAG>(sm, a, lr, l_on, seg_hi, K, nv, ids, (int)n_ids, lane, ws);
+                else
+                    count = replay_list<FAST, SUB, CAP, DIAG>(sm, a, r, on, seg_hi, K, nv, ids, (int)n_ids, lane, ws);
+                if (leads) ++ws.replays;
             } else {
-                count = traverse<FAST, SUB, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, -1, ovf, lane, ws, infer);
+                if constexpr (!TEAM) set_packet<FAST, SUB, CAP>(sm, r, on, seg_hi, lane);
+                count = search(-1, ovf);
             }
+            const int K_now = K;
             const unsigned long long* occ = sm.occ;
-            if (!BWD && rec_here && sm.rec_prev != kRecordFailed) {
+            auto& rec = record_of(sm);
+            if (!BWD && rec_here && leads && rec.rec_prev != kRecordFailed) {
                 // chunk record: header (multi-pass flag | K << 16 | id count), next record, ids
                 const unsigned n_ids = ovf ? 0u : (unsigned)count;
                 const unsigned words = 2u + n_ids;
@@ -1644,11 +2078,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
                         off = (unsigned)o;
                         a.rec_arena[off] = (ovf ? kRecordMulti : 0u) | ((unsigned)K << 16) | n_ids;
                         a.rec_arena[off + 1] = kNoRecord;
-                        if (sm.rec_prev != kNoRecord) a.rec_arena[sm.rec_prev + 1] = off;
-                        if (sm.rec_first == kNoRecord) sm.rec_first = off;
-                        sm.rec_prev = off;
+                        if (rec.rec_prev != kNoRecord) a.rec_arena[rec.rec_prev + 1] = off;
+                        if (rec.rec_first == kNoRecord) rec.rec_first = off;
+                        rec.rec_prev = off;
                     } else {
-                        sm.rec_prev = kRecordFailed;   // the chunks so far stay: the backward traverses after them
+                        rec.rec_prev = kRecordFailed;   // the chunks so far stay: the backward traverses after them
                         atomicAdd(&a.st->record_overflows, 1ull);
                     }
                 }
@@ -1754,28 +2188,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
                             if (nh > a.max_prim_slice) atomicAdd(&a.st->slab_cap_exceeded, 1ull);
                         }
                         if constexpr (!BWD) {
-                            // each lane keeps the colour of its own slabs
-                            if (has && dense) composite<FAST>(r, sb, alpha, a.neg_zero);
+                            group_colour<FAST, SUB>(r, sb, alpha, has && dense, lane, a.neg_zero);
                         } else {
-                            // g . R is linear through the scalars: from 0 first, then the lane's start, which
-                            // is the group's less what the slabs before the lane's took
                             AdjBuf<FAST> ad;
-                            float Ta, took;
-                            const float gR0 = r.gR;
-                            r.gR = 0.f;
-                            slab_adjoint_scalars<FAST>(r, sb, alpha, ad, Ta, took, a.neg_zero);
-                            if (!(has && dense)) took = 0.f;
-                            float upto = took;
-#pragma unroll
-                            for (int o = 1; o < SUB; o <<= 1) {
-                                const float v = __shfl_up_sync(kFull, upto, o);
-                                if (sub >= o) upto += v;
-                            }
-                            const float all = __shfl_sync(kFull, upto, ray * SUB + SUB - 1);
-                            add_start(ad, -kDt * (gR0 + (upto - took)));
+                            const float gR_end = group_adjoint_scalars<FAST, SUB>(r, sb, alpha, has && dense, ad, lane);
                             slab_adjoint<FAST, SUB, CAP, DIAG>(sm, k, K, has && dense, r, a, rgb_base, roff, ad,
                                                                nwords(count), lane, ws, view);
-                            r.gR = gR0 + all;
+                            r.gR = gR_end;
                         }
                         r.T = T_end;
                         // on to the next group (or the end of the chunk)
@@ -1790,7 +2209,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
                 }
             } else {
                 // K == 1 and more hits than the list holds: consume the slab in several passes
-                const bool has_ray = on && nv > 0 && r.T > kTeps, has = has_ray && sub == 0;
+                const bool has_ray = on && r.tb < r.texit && r.T > kTeps, has = has_ray && sub == 0;
                 float roff[kBuf];
                 unsigned seed_next = slab_offsets(a.rnd_sample, r.seed, roff);
                 SlabBuf<FAST, BWD> sb;
@@ -1801,8 +2220,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
                 while (more) {
                     int cursor = sm.ids[count - 1];
                     __syncwarp();
-                    if (lane == 0) atomicAdd(&a.st->list_passes, 1ull);
-                    count = traverse<FAST, SUB, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, more, lane, ws, infer);
+                    if (leads && lane == 0) atomicAdd(&a.st->list_passes, 1ull);
+                    count = search(cursor, more);
                     nh += slab_buffers<FAST, SUB, CAP, BWD, DIAG>(sm, 0, 1, has, r, a, rgb_base, roff, sb, nwords(count), lane,
                                                              ws);
                 }
@@ -1828,7 +2247,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
                     int cursor = -1;
                     bool more2 = true;
                     while (more2) {
-                        count = traverse<FAST, SUB, CAP, DIAG>(sm, a, r, on, t_end, seg_hi, K, nv, cursor, more2, lane, ws, infer);
+                        count = search(cursor, more2);
                         slab_adjoint<FAST, SUB, CAP, DIAG>(sm, 0, 1, act, r, a, rgb_base, roff, ad, nwords(count), lane, ws,
                                                       view);
                         if (more2) cursor = sm.ids[count - 1];
@@ -1843,23 +2262,30 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
                 if constexpr (SUB > 1) {
                     r.T = __shfl_sync(kFull, r.T, ray * SUB);
                     r.gR = __shfl_sync(kFull, r.gR, ray * SUB);
+                    r.C = f3(__shfl_sync(kFull, r.C.x, ray * SUB), __shfl_sync(kFull, r.C.y, ray * SUB),
+                             __shfl_sync(kFull, r.C.z, ray * SUB));
                 }
                 if (has_ray) r.tb = r.tb + kSlab;
             }
-            if (on) r.alive = r.alive && (r.T > kTeps) && (r.tb < r.texit);
-            if (BWD && lane == 0) sm.rec_cur = (rec_cur != kNoRecord) ? a.rec_arena[rec_cur + 1] : kNoRecord;
-            __syncwarp();
+            if constexpr (TEAM) {
+                if (l_on)
+                    for (int j = 0; j < K_now && lr.tb < lr.texit; ++j) lr.tb = lr.tb + kSlab;
+                if (sub == 0) sm.t.live[sm.slot] = on && r.T > kTeps && r.tb < r.texit;
+                if (BWD) team_rec = (rec_cur != kNoRecord) ? a.rec_arena[rec_cur + 1] : kNoRecord;
+                sm.sync();
+                live = __ballot_sync(kFull, sm.t.live[lane] != 0);
+            } else {
+                if (on) r.alive = r.alive && (r.T > kTeps) && (r.tb < r.texit);
+                if (BWD && lane == 0) sm.rec_cur = (rec_cur != kNoRecord) ? a.rec_arena[rec_cur + 1] : kNoRecord;
+                __syncwarp();
+            }
         }
-        if (!BWD && rec_here && lane == 0)
-            a.rec_tile[tile] = sm.rec_first;
+        if (!BWD && rec_here && leads && lane == 0)
+            a.rec_tile[tile] = record_of(sm).rec_first;
         flush_stats<FAST, SUB, CAP, DIAG>(sm, ws, hits_acc, slabs_acc, lane);
         if constexpr (!BWD && SUB > 1) {
 #pragma unroll
-            for (int o = 1; o < SUB; o <<= 1) {
-                r.C = f3(r.C.x + __shfl_xor_sync(kFull, r.C.x, o), r.C.y + __shfl_xor_sync(kFull, r.C.y, o),
-                         r.C.z + __shfl_xor_sync(kFull, r.C.z, o));
-                hits_acc += __shfl_xor_sync(kFull, hits_acc, o);
-            }
+            for (int o = 1; o < SUB; o <<= 1) hits_acc += __shfl_xor_sync(kFull, hits_acc, o);
         }
         if (!BWD && valid && sub == 0) {
             const long long ray_g = vt->ray_prefix[view] + (long long)ray_l;
@@ -1925,24 +2351,24 @@ cudaError_t launch_moment_grads(int n, const LeafRec* rec, const float4* ext, fl
 
 // List capacity per arithmetic: 4x the tuning value (64 or 128) for the fast lists; 128 for the
 // parity lists of whole tiles at either value (their slab ranges make an entry 72 B; shorter lists turn
-// dense slabs into multi-pass traversals, which the backward cannot replay).  The split tiles hold 256
-// entries in either arithmetic.
+// dense slabs into multi-pass traversals, which the backward cannot replay).  The parity lists of split tiles
+// hold 192 or 256 entries; a team's list has the length of the whole tile's, for the same chunks.
 using ParitySmem = WarpSmem<false, 1, 128>;
 using FastSmem256 = WarpSmem<true, 1, 256>;
 using FastSmem512 = WarpSmem<true, 1, 512>;
 using ParitySplit2Smem = WarpSmem<false, 2, 192>;
 using ParitySplitSmem = WarpSmem<false, 4, 256>;
-using FastSplit2Smem = WarpSmem<true, 2, 256>;
-using FastSplitSmem = WarpSmem<true, 4, 256>;
+using FastTeam2Smem = TeamSmem<2, 256>;
+using FastTeamSmem = TeamSmem<4, 256>;
 // packet and cone are read as float4: 16-byte aligned in every warp's slice of the block's array
-template <typename S>
+template <typename S, int WARPS = 1>
 constexpr bool smem_fits() {
     return offsetof(S, packet) % 16 == 0 && offsetof(S, cone) % 16 == 0 && sizeof(S) % 16 == 0 &&
-           sizeof(S) * kWarpsPerBlock <= 48 * 1024;
+           sizeof(S) * kWarpsPerBlock / WARPS <= 48 * 1024;
 }
 static_assert(smem_fits<ParitySmem>() && smem_fits<FastSmem256>() && smem_fits<FastSmem512>() &&
-                  smem_fits<ParitySplit2Smem>() && smem_fits<FastSplit2Smem>() && smem_fits<ParitySplitSmem>() &&
-                  smem_fits<FastSplitSmem>(),
+                  smem_fits<ParitySplit2Smem>() && smem_fits<FastTeam2Smem, 2>() && smem_fits<ParitySplitSmem>() &&
+                  smem_fits<FastTeamSmem, 4>(),
               "alignment, static shared memory limit");
 
 // The kernel of a launch: calls f(kernel).
@@ -1970,17 +2396,15 @@ int render_occupancy(bool backward, int mode, int cap, int split) {
 
 // Slabs side by side.  Few tiles wait for the slowest one, which the split shortens, the more the more
 // Gaussians a tile sees; many share the traversal better when they are whole, above all where rays are
-// long (an unbounded scene's far field: chunk after chunk with few Gaussians).  With T the launch's
-// 8x4-pixel tiles and x = Gaussians * views / T / (T / 1000), the lines below are where forward +
-// backward cross over 144 launches of 300 to 200,000 tiles, 1 to 12 views and 5k to 1M Gaussians in
-// boxes, on shells (3 to 5 units across) and in a ball with a far field (200); they lose 0.1 to 2 % on
-// the best choice for each.  In ms with 4 / 2 / 1 slabs:
-//   fast, short    300k, 1536 tiles  9.2 / 18.3 / 51.6    300k, 15000 tiles  10.0 / 10.3 / 16.9
-//                  50k, 28359        3.3 /  2.3 /  2.3    325k, 56328, 10 views  48.8 / 49.1 / 92.9
-//   fast, long     1M, 1536          7.9 /  9.3 / 15.6    1M, 28359          62.1 / 45.1 / 34.1
-//   parity, short  300k, 15000      18.3 / 22.6 / 34.9    50k, 28359          8.9 /  5.8 /  5.1
-// Whole steps: 10k Gaussians at 200x200, drop-in, 1.56 ms whole and 0.86 split; 300k on shells at
-// 797x801, drop-in, 35.2 and 19.0; three uneven views of 60k on shells, fast, 8.9 and 2.4.
+// long (an unbounded scene's far field: chunk after chunk with few Gaussians).  The results are the same.
+// With T the launch's 8x4-pixel tiles and x = Gaussians * views / T / (T / 1000), the lines below are where
+// forward + backward cross: fast over 117 launches of 300 to 147,000 tiles, 1 to 8 views and 5k to 600k
+// Gaussians in boxes, on shells (3 to 5 units across) and in a ball with a far field (200), where they lose
+// 1 to 2 % on the best choice for each; parity over 30 such launches of one view.  In ms with 4 / 2 / 1 slabs:
+//   fast, short    200k, 1500 tiles, 2 views  63.3 / 94.0 / 181    20k, 34187, 4 views    4.8 /  3.3 /  2.7
+//                  200k, 17048, 4 views       19.8 / 24.6 / 43.0   600k, 34187, 4 views  77.5 / 74.1 / 86.0
+//   fast, long     200k, 1500, 2 views        14.3 / 22.7 / 43.3   200k, 17048, 4 views  46.9 / 35.7 / 26.7
+//   parity, short  200k, 15000                20.2 / 17.0 / 22.8   600k, 15000           47.1 / 53.2 / 84.6
 SplitPair render_split(int mode, int rnd_sample, int cap, long long n, int n_views, long long n_rays) {
     const bool fast = mode == RG_MODE_FAST && rnd_sample == 0;
     // random offsets draw slab after slab; long lists are whole tiles' (the autotuner's choice)
@@ -1988,7 +2412,7 @@ SplitPair render_split(int mode, int rnd_sample, int cap, long long n, int n_vie
     const double t = (double)std::max(1ll, n_rays / (kTileW * kTileH));
     const double x = 1000.0 * (double)n * n_views / (t * t);
     auto pick = [&](double four, double two) { return x >= four ? 4 : x >= two ? 2 : 1; };
-    return {fast ? pick(1.0, 0.1) : pick(0.7, 0.2), pick(32.0, 6.0)};
+    return fast ? SplitPair{pick(2.5, 0.3), pick(45.0, 4.0)} : SplitPair{pick(1.5, 0.2), pick(32.0, 6.0)};
 }
 
 cudaError_t launch_render(bool backward, int mode, int cap, int split, int grid, const RenderArgs& args, cudaStream_t s) {
