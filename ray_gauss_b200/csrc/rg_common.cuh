@@ -106,6 +106,11 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
     return d;
 }
 // SFU base-2 logarithm (x <= 0 gives -inf / NaN, which fail every threshold comparison)
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float y;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 __device__ __forceinline__ float lg2_approx(float x) {
     float y;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -321,9 +321,14 @@ __device__ __forceinline__ void set_cone(WarpSmem<FAST, SUB, CAP>& sm, const rg_
 // towards the rays until all of them lie under it: the tilt's tangent is tau = (|p.U| + |p.V|) /
 // (|C| - |e.U| - |e.V|), and the centre's height over the plane is (rho - b tau) / sqrt(1 + tau^2).
 // No ray reaches a sphere that lies over the plane.  Along e the sphere spans b -+ R and a ray moves
-// by (|C| -+ |e.U| -+ |e.V|) / |D| per unit of its parameter.  The margin, a thousandth of R and 1e-5
-// of |O|, is above the rounding of this test and of the exact one by a factor of ten.  NaN (a
-// Gaussian that is never hit, an overflow) keeps the leaf: the exact test decides.
+// by (|C| -+ |e.U| -+ |e.V|) / |D| per unit of its parameter.
+//   Rounding.  O, C, U, V and the exact test's images of the ray are products with M: each is off by up to
+// 2e-7 |M| times the vector that went in, which for a flat Gaussian is far more than 2e-7 times the result.
+// Carried to the sphere each moves a ray by 2e-7 |M| |mu - o|, all of them by less than 1e-6 of it (|M| the
+// Frobenius norm); the steps after the products add 1e-5 |O| at most: both widen R, with a thousandth of it.
+// What is left of b e in P would be multiplied by the long U and V: they enter the tilt without their parts
+// along e, with 4e-7 of their lengths for what that rounds off.  NaN (a Gaussian that is never hit, an
+// overflow) keeps the leaf: the exact test decides.
 template <bool FAST, int SUB, int CAP>
 __device__ __forceinline__ bool may_hit(const WarpSmem<FAST, SUB, CAP>& sm, const LeafRec& rec, float3 o, float t0, float t1,
                                         float& t_first) {
@@ -343,10 +348,13 @@ __device__ __forceinline__ bool may_hit(const WarpSmem<FAST, SUB, CAP>& sm, cons
     const float3 P = O - e * b;
     const float rho2 = dot3(P, P), ir = rsqrtf(rho2);
     const float rho = rho2 * ir;
-    const float width = (fabsf(dot3(P, U)) + fabsf(dot3(P, V))) * ir;
-    const float spread = fabsf(dot3(e, U)) + fabsf(dot3(e, V));
-    const float along = c1 - spread;
-    const float R = __fdividef(1.f, rec.r0.w) * 1.001f + 1e-5f * (rho + fabsf(b));
+    const float eu = dot3(e, U), ev = dot3(e, V);
+    const float width = (fabsf(dot3(P, U - e * eu)) + fabsf(dot3(P, V - e * ev))) * ir +
+                        4e-7f * (sqrt_approx(dot3(U, U)) + sqrt_approx(dot3(V, V)));
+    const float spread = fabsf(eu) + fabsf(ev);
+    const float along = c1 * 0.99999f - spread;
+    const float m2 = dot3(r0, r0) + dot3(r1, r1) + dot3(r2, r2);
+    const float R = __fdividef(1.f, rec.r0.w) * 1.001f + 1e-5f * (rho + fabsf(b)) + 1e-6f * sqrt_approx(m2 * dot3(v, v));
     const bool miss = along > 0.f && rho * along - b * width > R * sqrtf(along * along + width * width);
     t_first = __fdividef(fmaxf(b - R, 0.f) * q2.y, c1 + spread) * 0.99999f;
     const bool before = along > 0.f && (b + R) * q2.z * 1.00001f < t0 * along, after = t_first > t1;
