@@ -815,6 +815,17 @@ __device__ __forceinline__ void walk_tree(WarpSmem<FAST, SUB, CAP>& sm, unsigned
     }
 }
 
+// Marches up to n slabs by repeated addition; returns how many.  Its variables are its own: an empty far field is
+// nothing but this loop, and a ray's state that is spilled around it would be loaded and stored in every turn
+// (5000 Gaussians in a ball, two views at 610x442, forward / backward: 2.39 / 2.10 ms so, 2.12 / 1.77 now).
+__device__ __forceinline__ unsigned march(float& tb, float texit, int n) {
+    float t = tb;
+    int j = 0;
+    for (; j < n && t < texit; ++j) t = t + kSlab;
+    tb = t;
+    return (unsigned)j;
+}
+
 // Warp-cooperative traversal for the chunk [tb, seg_hi] of every active lane (the packet set by
 // set_packet).  At a wide node lane k tests child slot k against the packet.  Hit leaves wait in a
 // buffer (the leading ones of a node are taken all at once); the first hit child that is a node is
@@ -2107,12 +2118,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
                         if (!occ_test(occ, k)) {
                             // no lane has a hit in slabs [k, k2): march them (tb only; T is unchanged)
                             int k2 = occ_next(occ, k, K);
-                            if (has) {
-                                for (int j = k; j < k2 && r.tb < r.texit; ++j) {
-                                    r.tb = r.tb + kSlab;
-                                    ++slabs_acc;
-                                }
-                            }
+                            if (has) slabs_acc += march(r.tb, r.texit, k2 - k);
                             k = k2 - 1;
                             continue;
                         }
@@ -2161,10 +2167,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
                             // march the groups without a hit (tb only; T is unchanged)
                             const int k2 = occ_next(occ, k, K), stop = k2 < K ? k2 / SUB * SUB : K;
                             if (base) {
-                                for (int j = k; j < stop && r.tb < r.texit; ++j) {
-                                    r.tb = r.tb + kSlab;
-                                    if (sub == 0) ++slabs_acc;
-                                }
+                                const unsigned n_slabs = march(r.tb, r.texit, stop - k);
+                                if (sub == 0) slabs_acc += n_slabs;
                             }
                             k = stop - SUB;
                             if (stop == K) break;
@@ -2276,8 +2280,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks<BWD, FAST, SUB
                 if (has_ray) r.tb = r.tb + kSlab;
             }
             if constexpr (TEAM) {
-                if (l_on)
-                    for (int j = 0; j < K_now && lr.tb < lr.texit; ++j) lr.tb = lr.tb + kSlab;
+                if (l_on) march(lr.tb, lr.texit, K_now);
                 if (sub == 0) sm.t.live[sm.slot] = on && r.T > kTeps && r.tb < r.texit;
                 if (BWD) team_rec = (rec_cur != kNoRecord) ? a.rec_arena[rec_cur + 1] : kNoRecord;
                 sm.sync();
