@@ -32,34 +32,40 @@ def camera_table(cameras):
     if not cameras:
         return np.zeros((0, 20), np.float32), 0.0
     wvts = [cam.world_view_transform for cam in cameras]
-    try:
-        # one stack and one copy to the host for all cameras (each copy of its own costs a synchronisation)
-        wvt = torch.stack(wvts).detach().to("cpu", torch.float32).numpy()
-    except RuntimeError:      # matrices of several devices or shapes
-        wvt = np.stack([w.detach().to("cpu", torch.float32).numpy()[:4, :3] for w in wvts])
-    known = {}                # most cameras share their field of view and size
-    focals = []
-    for cam in cameras:
-        key = (cam.FoVx, cam.FoVy, cam.image_width, cam.image_height)
+    stacked = None
+    if len({w.dtype for w in wvts}) == 1:
         try:
-            f = known.get(key)
-        except TypeError:     # values without a hash, such as zero-dimensional arrays
-            key = tuple(float(v) for v in key)
-            f = known.get(key)
-        if f is None:
-            f = known[key] = (fov2focal(key[0], key[2]), fov2focal(key[1], key[3]), key[2], key[3])
-        focals.append(f)
-    fx, fy, W, H = np.array(focals, np.float64).T
+            stacked = torch.stack(wvts)
+        except RuntimeError:  # matrices of several devices or shapes
+            pass
+    if stacked is not None:   # one copy to the host for all cameras (each copy of its own costs a synchronisation)
+        wvt = stacked.detach().to("cpu", torch.float32).numpy()
+    else:
+        wvt = np.stack([w.detach().to("cpu", torch.float32).numpy()[:4, :3] for w in wvts])
+    known, numbers, which = {}, [], []      # most cameras share their field of view and size
+    focal = 0.0
+    for cam in cameras:
+        key = FoVx, FoVy, W, H = cam.FoVx, cam.FoVy, cam.image_width, cam.image_height
+        # other kinds of numbers can be equal and still multiply in another precision
+        plain = type(W) is int and type(H) is int and type(FoVx) is float and type(FoVy) is float
+        at = known.get(key) if plain else None
+        if at is None:
+            at = len(numbers)
+            if plain:
+                known[key] = at
+            fx, fy = fov2focal(FoVx, W), fov2focal(FoVy, H)
+            row = np.empty(8, np.float32)
+            row[:] = [fx, fy, W / 2.0, H / 2.0, -0.15 * W, W * 1.15, -0.15 * H, 1.15 * H]
+            numbers.append(row)
+            if focal < fx:
+                focal = fx
+            if focal < fy:
+                focal = fy
+        which.append(at)
     table = np.empty((len(cameras), 20), np.float32)
     table[:, 0:9] = wvt[:, :3, :3].reshape(-1, 9)
     table[:, 9:12] = wvt[:, 3, :3]
-    for i, col in enumerate((fx, fy, W / 2.0, H / 2.0, -0.15 * W, W * 1.15, -0.15 * H, 1.15 * H)):
-        table[:, 12 + i] = col
-    focal = 0.0
-    for f in known.values():
-        for v in f[:2]:
-            if focal < v:
-                focal = v
+    table[:, 12:20] = np.stack(numbers)[which]
     return table, focal
 
 
