@@ -42,30 +42,30 @@ def camera_table(cameras):
         wvt = stacked.detach().to("cpu", torch.float32).numpy()
     else:
         wvt = np.stack([w.detach().to("cpu", torch.float32).numpy()[:4, :3] for w in wvts])
-    known, numbers, which = {}, [], []      # most cameras share their field of view and size
+    known, plain, odd = {}, [], []          # many cameras share their field of view and size
     focal = 0.0
-    for cam in cameras:
+    for i, cam in enumerate(cameras):
         key = FoVx, FoVy, W, H = cam.FoVx, cam.FoVy, cam.image_width, cam.image_height
-        # other kinds of numbers can be equal and still multiply in another precision
-        plain = type(W) is int and type(H) is int and type(FoVx) is float and type(FoVy) is float
-        at = known.get(key) if plain else None
-        if at is None:
-            at = len(numbers)
-            if plain:
-                known[key] = at
-            fx, fy = fov2focal(FoVx, W), fov2focal(FoVy, H)
-            row = np.empty(8, np.float32)
-            row[:] = [fx, fy, W / 2.0, H / 2.0, -0.15 * W, W * 1.15, -0.15 * H, 1.15 * H]
-            numbers.append(row)
-            if focal < fx:
-                focal = fx
-            if focal < fy:
-                focal = fy
-        which.append(at)
+        if type(W) is int and type(H) is int and type(FoVx) is float and type(FoVy) is float:
+            f = known.get(key)
+            if f is None:
+                f = known[key] = (fov2focal(FoVx, W), fov2focal(FoVy, H), W, H)
+            plain.append(f)
+        else:                 # other kinds of numbers can be equal and still multiply in another precision
+            f = fov2focal(FoVx, W), fov2focal(FoVy, H)
+            plain.append((0.0, 0.0, 0, 0))
+            odd.append((i, [*f, W / 2.0, H / 2.0, -0.15 * W, W * 1.15, -0.15 * H, 1.15 * H]))
+        for v in f[:2]:
+            if focal < v:
+                focal = v
+    fx, fy, W, H = np.array(plain, np.float64).T
     table = np.empty((len(cameras), 20), np.float32)
     table[:, 0:9] = wvt[:, :3, :3].reshape(-1, 9)
     table[:, 9:12] = wvt[:, 3, :3]
-    table[:, 12:20] = np.stack(numbers)[which]
+    for i, col in enumerate((fx, fy, W / 2.0, H / 2.0, -0.15 * W, W * 1.15, -0.15 * H, 1.15 * H)):
+        table[:, 12 + i] = col
+    for i, row in odd:
+        table[i, 12:20] = row
     return table, focal
 
 
