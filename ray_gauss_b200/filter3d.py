@@ -44,20 +44,23 @@ def camera_table(cameras):
         wvt = np.stack([w.detach().to("cpu", torch.float32).numpy()[:4, :3] for w in wvts])
     known, plain, odd = {}, [], []          # many cameras share their field of view and size
     focal = 0.0
-    for i, cam in enumerate(cameras):
+    for cam in cameras:
         key = FoVx, FoVy, W, H = cam.FoVx, cam.FoVy, cam.image_width, cam.image_height
-        if type(W) is int and type(H) is int and type(FoVx) is float and type(FoVy) is float:
-            f = known.get(key)
-            if f is None:
-                f = known[key] = (fov2focal(FoVx, W), fov2focal(FoVy, H), W, H)
-            plain.append(f)
-        else:                 # other kinds of numbers can be equal and still multiply in another precision
-            f = fov2focal(FoVx, W), fov2focal(FoVy, H)
-            plain.append((0.0, 0.0, 0, 0))
-            odd.append((i, [*f, W / 2.0, H / 2.0, -0.15 * W, W * 1.15, -0.15 * H, 1.15 * H]))
-        for v in f[:2]:
-            if focal < v:
-                focal = v
+        # other kinds of numbers can be equal and still multiply in another precision
+        ordinary = type(W) is int and type(H) is int and type(FoVx) is float and type(FoVy) is float
+        f = known.get(key) if ordinary else None
+        if f is None:
+            fx, fy = fov2focal(FoVx, W), fov2focal(FoVy, H)
+            if focal < fx:
+                focal = fx
+            if focal < fy:
+                focal = fy
+            if ordinary:
+                f = known[key] = (fx, fy, W, H)
+            else:
+                f = (0.0, 0.0, 0, 0)
+                odd.append((len(plain), [fx, fy, W / 2.0, H / 2.0, -0.15 * W, W * 1.15, -0.15 * H, 1.15 * H]))
+        plain.append(f)
     fx, fy, W, H = np.array(plain, np.float64).T
     table = np.empty((len(cameras), 20), np.float32)
     table[:, 0:9] = wvt[:, :3, :3].reshape(-1, 9)
