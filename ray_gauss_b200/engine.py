@@ -231,14 +231,18 @@ class Engine:
                                      _stream(self.device)), self.h, "rg_forward_sh")
         self.generation += 1
 
+    def _expect_rays(self, ray_colors):
+        # three colours per ray, whatever the tensor's shape
+        self.lib.rg_expect_rays(self.h, 0 if ray_colors is None else ray_colors.numel() // 3)
+
     def launch_forward(self, cams_t, n_cams, settings, ray_colors, final_T=None):
-        self.lib.rg_expect_rays(self.h, ray_colors.shape[0])
+        self._expect_rays(ray_colors)
         with self._timed("launch_forward"):
                 check(self.lib.rg_launch_forward(self.h, _ptr(cams_t), int(n_cams), ctypes.byref(settings),
                                              _ptr(ray_colors), _ptr(final_T), _stream(self.device)), self.h, "rg_launch_forward")
 
     def launch_backward(self, cams_t, n_cams, settings, ray_colors, dL):
-        self.lib.rg_expect_rays(self.h, ray_colors.shape[0])
+        self._expect_rays(ray_colors)
         with self._timed("launch_backward"):
             check(self.lib.rg_launch_backward(self.h, _ptr(cams_t), int(n_cams), ctypes.byref(settings),
                                               _ptr(ray_colors), _ptr(dL), _stream(self.device)), self.h, "rg_launch_backward")
@@ -271,7 +275,7 @@ class Engine:
         return ray_colors, fT
 
     def launch_inference(self, cams_t, n_cams, settings, ray_colors, counts=None):
-        self.lib.rg_expect_rays(self.h, ray_colors.shape[0])
+        self._expect_rays(ray_colors)
         with self._timed("launch_inference"):
             check(self.lib.rg_launch_inference(self.h, _ptr(cams_t), int(n_cams), ctypes.byref(settings),
                                                _ptr(ray_colors), _ptr(counts), _stream(self.device)), self.h,
