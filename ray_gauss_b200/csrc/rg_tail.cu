@@ -20,7 +20,7 @@
 // read).  1M Gaussians, 115 floats each, 3.25 GB: 553 us (90 % of a copy's rate), against 805 us when a block took 256
 // Gaussians through all tensors in turn (few loads in flight at a time, threads idle at the narrow
 // tensors, the clamps on parameters read again behind a barrier).  That form, k_train_tail, still does
-// what has no 16-byte alignment and what l2_resident names.
+// what has no 16-byte alignment, tensors that are not separate, and what l2_resident names.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -337,6 +337,29 @@ bool l2_resident(const rg_train_tail& d) {
     return width <= 64 && d.n >= 50000 && 16 * d.n * width <= 150000000;
 }
 
+// Whether the tensors can be taken side by side: none is in two roles, and what one writes no other uses.
+bool separate(const rg_train_tail& d) {
+    const int role[5] = {d.idx_positions, d.idx_densities, d.idx_scales, d.idx_quaternions, d.idx_lobe_axis};
+    for (int i = 0; i < 5; ++i)
+        for (int j = 0; j < i; ++j)
+            if (role[i] >= 0 && role[i] == role[j]) return false;
+    for (int i = 0; i < d.n_tensors; ++i) {
+        const rg_adam_tensor& t = d.tensors[i];
+        const uintptr_t at[4] = {(uintptr_t)t.param, (uintptr_t)t.exp_avg, (uintptr_t)t.exp_avg_sq, (uintptr_t)t.grad};
+        const uintptr_t size = t.width > 0 ? (uintptr_t)d.n * t.width * sizeof(float) : 0;
+        for (int j = 0; j < d.n_tensors; ++j) {
+            const rg_adam_tensor& u = d.tensors[j];
+            const uintptr_t other[3] = {(uintptr_t)u.param, (uintptr_t)u.exp_avg, (uintptr_t)u.exp_avg_sq};
+            const uintptr_t u_size = u.width > 0 ? (uintptr_t)d.n * u.width * sizeof(float) : 0;
+            if (i == j) continue;
+            for (uintptr_t p : at)
+                for (uintptr_t q : other)
+                    if (p && q && p < q + u_size && q < p + size) return false;
+        }
+    }
+    return true;
+}
+
 }  // namespace
 
 extern "C" {
@@ -367,7 +390,7 @@ int rg_train_tail_step(const rg_train_tail* d, void* stream) {
         seg.block_end[seg.count++] = (unsigned)blocks;
     }
     if (n4 < d->n) blocks += seg.count;
-    if (blocks > 0x7fffffffll || !seg.count || l2_resident(*d)) n4 = 0;
+    if (blocks > 0x7fffffffll || !seg.count || l2_resident(*d) || !separate(*d)) n4 = 0;
     if (n4)
         k_tail_stream<<<(unsigned)blocks, kTailThreads, 0, st>>>(a, seg, n4);
     else
