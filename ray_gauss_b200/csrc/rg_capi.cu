@@ -124,13 +124,7 @@ int ensure_views(rg_engine* e, int views) {
 constexpr long long kRecordWordsPerRay = 24;
 constexpr long long kRecordBaseWords = 4096;
 
-// Tiles that a record sized for `tiles` whole ones covers: four times as many split ones, which only
-// small launches have.
-long long record_heads(long long tiles, int split) {
-    return split > 1 ? std::max(tiles, std::min(4 * tiles, 1ll << 22)) : tiles;
-}
-
-// Hit-list record storage for launches of up to n_rays rays (tiles <= rays).
+// Hit-list record storage for launches of up to n_rays rays (a tile of any layout holds a ray at least).
 int ensure_record(rg_engine* e, long long n_rays) {
     long long words = std::min(n_rays * kRecordWordsPerRay + kRecordBaseWords, (long long)0xfffffff0ll);
     long long tiles = std::min(n_rays, (long long)INT_MAX);
@@ -143,7 +137,7 @@ int ensure_record(rg_engine* e, long long n_rays) {
     }
     if (tiles > e->rec_tiles) {
         e->rec_tiles = 0;
-        if ((rc = grow(e, e->rec_tile, (size_t)record_heads(tiles, 4)))) return rc;
+        if ((rc = grow(e, e->rec_tile, (size_t)tiles))) return rc;
         e->rec_tiles = (int)tiles;
     }
     e->rec_valid = false;
@@ -462,7 +456,7 @@ int rg_launch_forward(rg_engine* e, const rg_camera* cams, int32_t n_cams, const
         a.rec_top = e->rec_top;
         a.rec_cap = e->rec_cap;
         a.rec_tile = e->rec_tile;
-        a.rec_tiles = (int)record_heads(e->rec_tiles, std::max(split.near, split.far));
+        a.rec_tiles = e->rec_tiles;
     }
     RG_CUDA(launch_splits(e, false, s, split, a, S(stream)), "render forward");
     e->launches += 1;
@@ -543,7 +537,7 @@ int rg_launch_backward(rg_engine* e, const rg_camera* cams, int32_t n_cams, cons
         a.rec_arena = e->rec_arena;
         a.rec_cap = e->rec_cap;
         a.rec_tile = e->rec_tile;
-        a.rec_tiles = (int)record_heads(e->rec_tiles, std::max(split.near, split.far));
+        a.rec_tiles = e->rec_tiles;
         a.replay = 1;
     }
     RG_CUDA(launch_splits(e, true, s, split, a, S(stream)), "render backward");
