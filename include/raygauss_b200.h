@@ -183,9 +183,12 @@ RG_API int rg_destroy(rg_engine* e);
 RG_API int rg_reserve(rg_engine* e, int64_t n, int32_t n_views, int64_t n_rays);
 /* The number of rays of the render launches that follow (the cameras are read on the device, so the
  * engine does not know it otherwise; 0, the default: unknown).  It chooses between the tile layouts of
- * the render kernels, not what they compute: a small launch ends with its slowest tile and runs on
- * smaller ones.  A backward that replays its forward's hit lists keeps the forward's layout. */
+ * the render kernels, not what they compute (images and Gaussians per ray are the same bit for bit): a
+ * small launch ends with its slowest tile and divides it.  A backward that replays its forward's hit lists keeps the forward's layout. */
 RG_API int rg_expect_rays(rg_engine* e, int64_t n_rays);
+/* The layout of the last render launch: 1 (whole tiles), or the 2 or 4 slabs of a ray that it took side by
+ * side.  Waits for the stream. */
+RG_API int rg_tile_layout(rg_engine* e, int32_t* slabs, void* stream);
 RG_API int rg_set_tuning(rg_engine* e, const rg_tuning* t);
 RG_API int rg_get_tuning(const rg_engine* e, rg_tuning* t);
 

@@ -132,6 +132,7 @@ SIGNATURES = {
     "rg_destroy": (ctypes.c_int, [_P]),
     "rg_reserve": (ctypes.c_int, [_P, ctypes.c_int64, ctypes.c_int32, ctypes.c_int64]),
     "rg_expect_rays": (ctypes.c_int, [_P, ctypes.c_int64]),
+    "rg_tile_layout": (ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int32), _P]),
     "rg_set_tuning": (ctypes.c_int, [_P, ctypes.POINTER(rg_tuning)]),
     "rg_get_tuning": (ctypes.c_int, [_P, ctypes.POINTER(rg_tuning)]),
     "rg_ellipsoids_bbox": (ctypes.c_int, [_P, ctypes.POINTER(rg_gaussians), _P, _P, _P]),

@@ -597,6 +597,17 @@ int rg_leaf_order(rg_engine* e, int32_t* leaf_gid_out, void* stream) {
     return RG_OK;
 }
 
+int rg_tile_layout(rg_engine* e, int32_t* slabs, void* stream) {
+    if (!e || !slabs) return RG_ERR_INVALID_ARG;
+    if (e->colors_views <= 0) return RG_ERR_STATE;
+    DeviceScope dev_scope;
+    int rc = dev_scope.enter(e);
+    if (rc) return rc;
+    RG_CUDA(cudaStreamSynchronize(S(stream)), "sync");
+    RG_CUDA(cudaMemcpy(slabs, &e->vt->split, sizeof(int32_t), cudaMemcpyDeviceToHost), "read layout");
+    return RG_OK;
+}
+
 int rg_get_status(rg_engine* e, rg_status* out, int32_t reset, void* stream) {
     if (!e || !out) return RG_ERR_INVALID_ARG;
     DeviceScope dev_scope;

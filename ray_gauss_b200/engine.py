@@ -187,6 +187,12 @@ class Engine:
         check(self.lib.rg_get_status(self.h, ctypes.byref(st), int(bool(reset)), _stream(self.device)), self.h, "rg_get_status")
         return {k: int(getattr(st, k)) for k, _ in _lib.rg_status._fields_}
 
+    def tile_layout(self) -> int:
+        """Slabs of a ray side by side in the last render launch: 1, 2 or 4."""
+        out = ctypes.c_int32(0)
+        check(self.lib.rg_tile_layout(self.h, ctypes.byref(out), _stream(self.device)), self.h, "rg_tile_layout")
+        return out.value
+
     def leaf_order(self, n):
         out = torch.empty((n,), dtype=torch.int32, device=self.device)
         check(self.lib.rg_leaf_order(self.h, _ptr(out), _stream(self.device)), self.h, "rg_leaf_order")
