@@ -2367,7 +2367,7 @@ int render_occupancy(bool backward, int mode, int cap, int split) {
 // Gaussians a tile sees; many share the traversal better when they are whole, above all where rays are
 // long (an unbounded scene's far field: chunk after chunk with few Gaussians).  The results are the same.
 // With T the launch's 8x4-pixel tiles and x = Gaussians * views / T / (T / 1000), the lines below are where
-// forward + backward cross: fast over 117 launches of 300 to 147,000 tiles, 1 to 8 views and 5k to 600k
+// forward + backward cross: fast over 122 launches of 300 to 147,000 tiles, 1 to 8 views and 5k to 600k
 // Gaussians in boxes, on shells (3 to 5 units across) and in a ball with a far field (200), where they lose
 // 1 to 2 % on the best choice for each; parity over 30 such launches of one view.  In ms with 4 / 2 / 1 slabs:
 //   fast, short    200k, 1500 tiles, 2 views  63.3 / 94.0 / 181    20k, 34187, 4 views    4.8 /  3.3 /  2.7
@@ -2381,7 +2381,7 @@ SplitPair render_split(int mode, int rnd_sample, int cap, long long n, int n_vie
     const double t = (double)std::max(1ll, n_rays / (kTileW * kTileH));
     const double x = 1000.0 * (double)n * n_views / (t * t);
     auto pick = [&](double four, double two) { return x >= four ? 4 : x >= two ? 2 : 1; };
-    return fast ? SplitPair{pick(2.5, 0.3), pick(45.0, 4.0)} : SplitPair{pick(1.5, 0.2), pick(32.0, 6.0)};
+    return fast ? SplitPair{pick(2.7, 0.6), pick(45.0, 4.0)} : SplitPair{pick(1.5, 0.2), pick(32.0, 6.0)};
 }
 
 cudaError_t launch_render(bool backward, int mode, int cap, int split, int grid, const RenderArgs& args, cudaStream_t s) {

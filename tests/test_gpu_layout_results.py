@@ -42,7 +42,7 @@ def test_layouts_agree(cuda, mode, kind, record):
     n = P["positions"].shape[0]
     dL = torch.randn((views.n_rays, 3), device=cuda, generator=torch.Generator(device=cuda).manual_seed(4)) * 1e-4
     # x = 1000 Gaussians views / tiles^2 decides (render_split): above every line, or between the two lines
-    line = 15.0 if kind == "far" else 0.33
+    line = 15.0 if kind == "far" else 1.0
     got = {}
     for split, rays in ((1, 0), (2, 32 * int(math.sqrt(2000.0 * n / line))), (4, 32)):
         eng = Engine()
