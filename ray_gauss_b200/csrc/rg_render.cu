@@ -11,10 +11,10 @@
 //   adjoint                   optix_raycasting/cuda_train/backward/gaussians_aabb.cu:505-775
 //
 // Design.  A warp owns an 8x4 pixel tile, or a part of one where it takes several slabs of a ray at a time
-// (TileShape; in the fast arithmetic the warps of a tile then share its list); tiles of all views are pulled from one atomic work counter.  Each ray marches with the
-// reference's slab sequence (tb += 0.02 in FP32); the warp advances in chunks of K slabs per ray (K adapts
-// between 1 and 255: it grows while hits are sparse and shrinks in place when the hit list overflows).  For a
-// chunk the warp traverses the wide BVH once for the packet of its rays' segments (one child slot per lane,
+// (TileShape; in the fast arithmetic the warps of a tile then share its list); tiles of all views are pulled
+// from one atomic work counter.  Each ray marches with the reference's slab sequence (tb += 0.02 in FP32);
+// the warp advances in chunks of K slabs per ray (K adapts between 1 and 255: it grows while hits are sparse
+// and shrinks in place when the hit list overflows).  For a chunk the warp traverses the wide BVH once for the packet of its rays' segments (one child slot per lane,
 // tested with interval arithmetic over the rays' directions) with a warp-uniform stack.  Leaves wait until
 // there are 32, are culled one per lane against the tile's ray cone, and the candidates take the exact
 // ellipsoid test, all rays at a time.  A leaf that any ray hits is appended to a shared hit list with, per
@@ -836,8 +836,8 @@ __device__ __forceinline__ unsigned march(float& tb, float texit, int n) {
 // keep the first slab that they can reach.  When the tree is through, the candidates get the exact
 // test per ray, and those that any ray hits are appended to the warp list, whose entry count is
 // returned.  A leaf costs a visit's warp 1/32 of may_hit instead of a whole exact test: on 1M
-// Gaussians x 16 views 214M exact tests instead of 581M (122M entries used), forward 214.7 -> 196.8
-// ms; 3M x 4 x 1080p: 118.4 -> 98.3 ms.
+// Gaussians x 16 views 364M exact tests instead of 633M (128M entries), forward 251 -> 225 ms; 3M x 4 x
+// 1080p: 243 -> 198 ms.
 //
 // A chunk with too many Gaussians is shortened in place (K, nv and seg_hi): when the list fills up, K is
 // halved, entries that start at slab K or later are dropped, those that stay get the exact test again,
